@@ -90,6 +90,10 @@ struct Level {
     int W = 0, H = 0, gw = 0, gh = 0, count = 0;
     bool roi = false;
     DeviceBuffer plane, meta, inv, links, selected;
+    // The banded solver loop's copies: f (where the intensity plane is not it),
+    // (gx, gy), and the window's pixel table.
+    DeviceBuffer plane_f, plane_grad, pixel_table;
+    const float *solver_f = nullptr;
     DeviceBuffer intensity, spline, scratch, valid;  // preparation scratch
     DeviceBuffer admissible;                         // u8 per subset, ROI ignored
     DeviceBuffer moments;                            // quadratic row path: moments per subset
@@ -155,6 +159,9 @@ class Runtime {
     void upload_frame(Level &level, LevelSlot &slot, const uint8_t *frame, int64_t row_stride,
                       HostBuffer &staging, cudaStream_t stream);
     int persistent_grid(int lanes);
+    const BandPlan &band_plan(int lanes) const { return band_plans_[lanes == 16 ? 0 : (lanes == 32 ? 1 : 2)]; }
+    bool banded() const { return band_plans_[0].rows > 0 || band_plans_[1].rows > 0; }
+    void split_plane(Level &level, bool gradients);
     // Switch the solver variant (lanes per subset, persistent queue).
     void set_variant(int lanes, bool persistent);
     // Switch the pixel loop (GBDIC_SOLVER_*).
@@ -178,6 +185,7 @@ class Runtime {
     int sm_count_ = 0;
     int device_ = 0;
     int persistent_grid_ = 0;
+    BandPlan band_plans_[3] = {};  // 16 lanes, 32 lanes, more (always the direct loop)
     int persistent_lanes_ = 0;
     int persistent_variant_ = 0;  // 0 exact, 1 fast, 2 / 3 staged tile 1 / 2
     bool profiling_ = false;

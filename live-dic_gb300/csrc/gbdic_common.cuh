@@ -134,11 +134,25 @@ __device__ __forceinline__ void displacement(const Warp &w, float lx, float ly, 
 
 __device__ __forceinline__ float length2(float a, float b) { return sqrtf(fmaf(a, a, b * b)); }
 
+// How the banded loop (solver_band.cuh) walks a window; rows == 0: the direct
+// loop.
+struct BandPlan {
+    int rows;             // window rows sampled into shared memory at a time
+    int run, segments;    // rows of a vertical run, runs on top of each other in a band
+    int run32, segments32;  // the same while all 32 lanes of a warp sample one subset
+    int pitch;            // floats of one subset's band buffer
+    unsigned magic;       // ceil(2^20 / S)
+    int solo_count;       // 16 lanes: launches of at most this many subsets give each a warp
+};
+
 // Arguments of one IC-GN launch over one level.
 struct SolveArgs {
     const float *coef;         // B-spline coefficient plane (bspline mode)
     const uint8_t *img;        // target bytes (direct modes)
     const float4 *plane;       // reference plane [f, gx, gy, 0]
+    const float *plane_f;      // banded loop: its f and its (gx, gy) as planes of their own,
+    const float2 *plane_grad;  // and per window pixel (lx, ly, weight, plane offset as bits)
+    const float4 *pixel_table;
     const float *meta;         // metadata rows
     const float *inv;          // inverse Hessians
     const float *weights;      // S*S integration weights (Gaussian mode)
@@ -166,6 +180,7 @@ struct SolveArgs {
     // Staged tiles (solver_staged.cu): 0 off, 1 compact (56 x 44 floats per
     // warp), 2 wide (72 x 56).
     int staged_tile;
+    BandPlan band;
     // List mode (exact loop, complete windows): group g solves subset
     // subset_list[g] for g < count, or g < min(count, *list_count) when
     // list_count is set (a device count written by an earlier kernel).

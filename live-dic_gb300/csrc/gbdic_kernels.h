@@ -19,8 +19,12 @@ cudaError_t launch_icgn_model(const SolveArgs &a, int interp, int lanes, bool ga
                               cudaStream_t stream, int *occupancy_only);
 // Grid for a non-persistent launch of `count` subsets with `lanes` lanes.
 int icgn_grid(int count, int lanes);
+int icgn_band_grid(const SolveArgs &a, int lanes);
+// The banded loop's plan for complete B-spline windows of side S, or rows 0
+// where the direct loop is the better one.
+BandPlan plan_bands(int S, int model, int interp, int lanes, int sm_count);
 // Resident CTAs per SM of the solver variant (for persistent grids).
-int icgn_occupancy(int model, int interp, int lanes, bool gauss);
+int icgn_occupancy(int model, int interp, int lanes, bool gauss, int S, const BandPlan &band);
 cudaError_t launch_icgn(const SolveArgs &a, int model, int interp, int lanes, bool gauss,
                         int persistent_grid, cudaStream_t stream);
 // Rows 0 .. total-1 of a.state as the seeded solver writes disabled subsets
@@ -91,6 +95,7 @@ struct PrepArgs {
     float *spline;          // H*W (B-spline coefficients) and transposes
     float *scratch;         // H*W
     float4 *plane;          // H*W
+    float2 *plane_grad;     // H*W copies of its (gx, gy), or nullptr
     float *meta;            // count * meta_stride
     float *inv;             // count * n * n
     unsigned *valid_count;
@@ -100,6 +105,8 @@ struct PrepArgs {
     float *moments;
 };
 cudaError_t launch_reference_prep(const PrepArgs &a, cudaStream_t stream);
+// f and (unless nullptr) (gx, gy) of a reference plane as planes of their own.
+cudaError_t launch_split_plane(const float4 *plane, size_t pixels, float *f, float2 *grad, cudaStream_t stream);
 // Quadratic preparation by window rows (column sums shared by the windows of
 // a grid row, one thread per 12x12 inverse): uniform or Gaussian weights (the
 // Gaussian as the outer product of axis_weights), overlapping windows

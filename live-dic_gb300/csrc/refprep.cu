@@ -140,7 +140,7 @@ __global__ void spline_columns_kernel(const float *__restrict__ in, int n, int c
 
 // ---------------------------------------------------------------- stage 3
 __global__ void gradient_kernel(const float *__restrict__ intensity, const float *__restrict__ src,
-                                int W, int H, int bspline, float4 *__restrict__ plane) {
+                                int W, int H, int bspline, float4 *__restrict__ plane, float2 *__restrict__ grad) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W || y >= H) return;
     const int xm = mirror_clamp(x - 1, W), xp = mirror_clamp(x + 1, W);
@@ -157,6 +157,16 @@ __global__ void gradient_kernel(const float *__restrict__ intensity, const float
         gy = gy / 6.0f;
     }
     plane[(size_t)y * W + x] = make_float4(intensity[(size_t)y * W + x], gx, gy, 0.0f);
+    if (grad) grad[(size_t)y * W + x] = make_float2(gx, gy);
+}
+
+__global__ void split_plane_kernel(const float4 *__restrict__ plane, size_t pixels, float *__restrict__ f,
+                                   float2 *__restrict__ grad) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= pixels) return;
+    const float4 v = plane[i];
+    f[i] = v.x;
+    if (grad) grad[i] = make_float2(v.y, v.z);
 }
 
 // ---------------------------------------------------------------- stage 4
@@ -567,6 +577,11 @@ __global__ void __launch_bounds__(128) subset_prep_kernel(PrepArgs a) {
 
 }  // namespace
 
+cudaError_t launch_split_plane(const float4 *plane, size_t pixels, float *f, float2 *grad, cudaStream_t stream) {
+    split_plane_kernel<<<(unsigned)((pixels + 255) / 256), 256, 0, stream>>>(plane, pixels, f, grad);
+    return cudaGetLastError();
+}
+
 cudaError_t set_gauss_taps(const float *taps7) { return cudaMemcpyToSymbol(c_gauss, taps7, 7 * sizeof(float)); }
 
 cudaError_t launch_reference_prep(const PrepArgs &a, cudaStream_t stream) {
@@ -589,7 +604,7 @@ cudaError_t launch_reference_prep(const PrepArgs &a, cudaStream_t stream) {
         grad_src = a.spline;
     }
     gradient_kernel<<<dim3((W + 127) / 128, H), 128, 0, stream>>>(a.intensity, grad_src, W, H,
-                                                                    bspline ? 1 : 0, a.plane);
+                                                                    bspline ? 1 : 0, a.plane, a.plane_grad);
     const int blocks = (a.count + 3) / 4;
     if (blocks > 0 && a.moments) {
         const cudaError_t err = launch_quadratic_row_prep(a, stream);

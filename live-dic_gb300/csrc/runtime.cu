@@ -166,6 +166,7 @@ Runtime::Runtime(const gbdic_options &options) {
     axis_weights_.ensure(axis.size() * sizeof(float));
     check_cuda(cudaMemcpy(axis_weights_.get(), axis.data(), axis.size() * sizeof(float), cudaMemcpyHostToDevice),
                "axis weights upload");
+    for (int k = 0; k < 2; ++k) band_plans_[k] = plan_bands(S, options.motion_model, options.interpolation, 16 << k, sm_count_);
     if (options.persistent) persistent_grid(opt_.lanes);
 }
 
@@ -215,7 +216,8 @@ int Runtime::persistent_grid(int lanes) {
         const bool gauss = opt_.o.spatial_weighting == 1;
         const int per_sm = fast   ? icgn_fast_occupancy(opt_.o.motion_model, lanes, gauss)
                            : tile ? icgn_staged_occupancy(opt_.o.motion_model, lanes, gauss, tile)
-                                  : icgn_occupancy(opt_.o.motion_model, opt_.o.interpolation, lanes, gauss);
+                                  : icgn_occupancy(opt_.o.motion_model, opt_.o.interpolation, lanes, gauss,
+                                                   opt_.o.subset_size, band_plan(lanes));
         persistent_grid_ = std::max(1, per_sm) * sm_count_;
         persistent_lanes_ = lanes;
         persistent_variant_ = variant;
@@ -240,7 +242,33 @@ void Runtime::configure_level(Level &level, int W, int H, int slots) {
     grid_of(W, H, opt_.o.subset_size, opt_.o.subset_stride, level.gw, level.gh);
     level.count = level.gw * level.gh;
     level.slots.clear();
+    if (banded()) {
+        const int S = opt_.o.subset_size;
+        std::vector<float4> table((size_t)S * S);
+        for (int r = 0; r < S; ++r)
+            for (int c = 0; c < S; ++c) {
+                float4 &t = table[(size_t)r * S + c];
+                const uint32_t offset = (uint32_t)r * (uint32_t)W + (uint32_t)c;
+                t = make_float4((float)c - 0.5f * (S - 1), (float)r - 0.5f * (S - 1), opt_.weights[(size_t)r * S + c], 0.0f);
+                std::memcpy(&t.w, &offset, sizeof(offset));
+            }
+        level.pixel_table.ensure(table.size() * sizeof(float4));
+        check_cuda(cudaMemcpyAsync(level.pixel_table.get(), table.data(), table.size() * sizeof(float4),
+                                   cudaMemcpyHostToDevice, stream_), "pixel table upload");
+        check_cuda(cudaStreamSynchronize(stream_), "pixel table upload");
+    }
     ensure_slots(level, slots);
+}
+
+// f of the plane for the banded loop: the intensity plane, or a copy where
+// the preparation centred the windows of a tiled grid in the plane.
+void Runtime::split_plane(Level &level, bool gradients) {
+    const size_t px = (size_t)level.W * level.H;
+    level.plane_f.ensure(px * sizeof(float));
+    if (gradients) level.plane_grad.ensure(px * sizeof(float2));
+    check_cuda(launch_split_plane(level.plane.as<float4>(), px, level.plane_f.as<float>(),
+                                  gradients ? level.plane_grad.as<float2>() : nullptr, stream_), "plane split");
+    level.solver_f = level.plane_f.as<float>();
 }
 
 void Runtime::ensure_slots(Level &level, int slots) {
@@ -304,6 +332,8 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
     a.spline = level.spline.as<float>();
     a.scratch = level.scratch.as<float>();
     a.plane = level.plane.as<float4>();
+    if (banded()) level.plane_grad.ensure(px * sizeof(float2));
+    a.plane_grad = banded() ? level.plane_grad.as<float2>() : nullptr;
     a.meta = level.meta.as<float>();
     a.inv = level.inv.as<float>();
     a.valid_count = level.valid.as<unsigned>();
@@ -318,6 +348,8 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
     check_cuda(cudaEventCreate(&e1), "event");
     cudaEventRecord(e0, stream_);
     check_cuda(launch_reference_prep(a, stream_), "reference preparation launch");
+    level.solver_f = level.intensity.as<float>();
+    if (banded() && a.stride == a.S) split_plane(level, false);
     cudaEventRecord(e1, stream_);
     unsigned valid = 0;
     check_cuda(cudaMemcpyAsync(&valid, level.valid.get(), sizeof(unsigned), cudaMemcpyDeviceToHost, stream_), "readback");
@@ -340,6 +372,10 @@ void Runtime::upload_reference_arrays(Level &level, const float *plane, const fl
     level.inv.ensure((size_t)level.count * n * n * sizeof(float));
     level.partial_count = 0;
     check_cuda(cudaMemcpy(level.plane.get(), plane, px * sizeof(float4), cudaMemcpyHostToDevice), "plane upload");
+    if (banded()) {
+        split_plane(level, true);
+        check_cuda(cudaStreamSynchronize(stream_), "plane split");
+    }
     check_cuda(cudaMemcpy(level.meta.get(), meta, (size_t)level.count * meta_stride(model) * sizeof(float),
                           cudaMemcpyHostToDevice), "metadata upload");
     check_cuda(cudaMemcpy(level.inv.get(), inverse, (size_t)level.count * n * n * sizeof(float),
@@ -424,6 +460,10 @@ SolveArgs Runtime::solve_args(Level &level, LevelSlot &slot, const gbdic_solver_
     a.coef = slot.coef.as<float>();
     a.img = frame ? frame : slot.frame.as<uint8_t>();
     a.plane = level.plane.as<float4>();
+    a.plane_f = level.solver_f;
+    a.plane_grad = level.plane_grad.as<float2>();
+    a.pixel_table = level.pixel_table.as<float4>();
+    a.band = band_plan(opt_.lanes);
     a.meta = level.meta.as<float>();
     a.inv = level.inv.as<float>();
     a.weights = opt_.o.spatial_weighting == 1 ? weights_.as<float>() : nullptr;
@@ -527,6 +567,7 @@ void Runtime::enqueue_solve_list(Level &level, LevelSlot &slot, const gbdic_solv
     SolveArgs a = solve_args(level, slot, cfg, true, false, frame, state);
     a.fast_segments = 0;
     a.staged_tile = 0;
+    a.band = band_plan(lanes);
     const int model = opt_.o.motion_model, interp = opt_.o.interpolation;
     check_cuda(launch_disabled_rows(a, model, level.count, s), "disabled rows");
     if (length <= 0) return;
@@ -538,7 +579,7 @@ void Runtime::enqueue_solve_list(Level &level, LevelSlot &slot, const gbdic_solv
     if (list_count != nullptr) {
         // a device-side length: a persistent grid over the list
         a.persistent = 1;
-        const int per_sm = icgn_occupancy(model, interp, lanes, gauss);
+        const int per_sm = icgn_occupancy(model, interp, lanes, gauss, a.S, a.band);
         grid = std::max(1, per_sm) * sm_count_;
         check_cuda(cudaMemsetAsync(slot.counter.get(), 0, sizeof(unsigned), s), "queue reset");
     } else {

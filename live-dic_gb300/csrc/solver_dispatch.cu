@@ -1,5 +1,6 @@
 // Launch geometry and dispatch of the IC-GN solver variants.
 #include "gbdic_kernels.h"
+#include "solver_band.cuh"
 
 namespace gbdic {
 
@@ -58,8 +59,64 @@ cudaError_t dispatch(const SolveArgs &a, int model, int interp, int lanes, bool 
 }
 }  // namespace
 
-int icgn_occupancy(int model, int interp, int lanes, bool gauss) {
+// Run length of one band of `rows` x S pixels walked by `samplers` lanes, and
+// its steps: runs are walked two to a lane, and each costs three quarters of
+// a step more for its first taps.
+static double band_steps(int S, int rows, int samplers, int &run, int &segments) {
+    double best = 1e30;
+    for (int r = 1; r <= rows; ++r) {
+        const int s = (rows + r - 1) / r, phases = (S * s + 2 * samplers - 1) / (2 * samplers);
+        const double cost = phases * (r + 0.75) + 0.5;
+        if (cost < best) {
+            best = cost;
+            run = r;
+            segments = s;
+        }
+    }
+    return best;
+}
+
+BandPlan plan_bands(int S, int model, int interp, int lanes, int sm_count) {
+    BandPlan best{};
+    if (interp != kInterpBspline || lanes > 32 || S > kMaxBandFloats) return best;
+    double steps = 1e30;
+    for (int bands = 1; bands <= S; ++bands) {
+        const int rows = (S + bands - 1) / bands;
+        if (rows * S > kMaxBandFloats) continue;
+        int run = 0, segments = 0;
+        const double cost = (S + rows - 1) / rows * band_steps(S, rows, lanes, run, segments);
+        if (cost < steps) {
+            steps = cost;
+            best.rows = rows;
+            best.run = run;
+            best.segments = segments;
+        }
+    }
+    // Against the direct loop's S^2 / (2 lanes) steps.  Measured at 2560 x
+    // 1440 (band / direct time): affine 16 lanes 0.89 at a ratio of 1.07
+    // (S 31), 0.94 at 1.20 (S 41), 1.00 at 1.26 (S 51), 1.03 at 1.34 (S 33),
+    // 1.08 at 1.49 (S 65); 32 lanes 0.95 at 1.31 (S 16), 1.02 at 1.35 (S 51);
+    // translation and quadratic 0.82 and 0.85 at 1.49, and with 32 lanes 1.11
+    // and 1.04 at 1.70.
+    const double limit = model != kModelAffine ? 1.6 : (lanes == 16 ? 1.25 : 1.34);
+    if (steps * 2 * lanes > limit * S * S) return BandPlan{};
+    band_steps(S, best.rows, 32, best.run32, best.segments32);
+    best.magic = ((1u << 20) + S - 1) / S;
+    best.pitch = (best.rows * S + 15) / 32 * 32 + 16;  // groups of one warp start 16 banks apart
+    if (lanes == 16) best.solo_count = sm_count * 4 * (model == kModelQuadratic ? kBandQuadBlocks : kBandBlocks);
+    return best;
+}
+
+// CTAs of a non-persistent launch of the banded loop.
+int icgn_band_grid(const SolveArgs &a, int lanes) {
+    const int per_warp = lanes == 16 && a.count > a.band.solo_count ? 2 : 1;
+    return ((a.count + per_warp - 1) / per_warp + 3) / 4;
+}
+
+int icgn_occupancy(int model, int interp, int lanes, bool gauss, int S, const BandPlan &band) {
     SolveArgs unused{};
+    unused.S = S;
+    unused.band = band;
     int blocks = 0;
     if (dispatch(unused, model, interp, lanes, gauss, 0, nullptr, &blocks) != cudaSuccess) return 0;
     return blocks;

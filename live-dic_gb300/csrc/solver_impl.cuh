@@ -258,13 +258,19 @@ __device__ __forceinline__ float divergence_status(const SolveArgs &a, float cha
     return (stalled >= (unsigned)a.div_patience) ? 3.0f : status;
 }
 
+template <bool SHARED>
+__device__ __forceinline__ float load_row(const float *p) {
+    return SHARED ? *p : __ldg(p);
+}
+
 // Gauss-Newton update from the reduced totals (icgn.wgsl:801-921).  Returns
 // the new status; modifies the warp on a successful composition.
 // Quadratic: `sl` / `mask` as for compose_quadratic; lane r of each 16-lane
-// segment forms row r of H^-1 r and the rows are exchanged by shuffles.
-template <int MODEL>
+// segment forms row r of H^-1 r and takes one control point, exchanged by
+// shuffles.  SHARED: the metadata and inverse rows are in shared memory.
+template <int MODEL, bool SHARED = false>
 __device__ __forceinline__ float gn_update(const SolveArgs &a, const float (&t)[SumCount<MODEL>::value],
-                                           const float *__restrict__ md, const float *__restrict__ hi,
+                                           const float *md, const float *hi,
                                            float wsum, float half, unsigned it1, Warp &w,
                                            float &prev_change, unsigned &stalled, int sl, unsigned mask) {
     constexpr int n = parameter_count(MODEL);
@@ -279,7 +285,7 @@ __device__ __forceinline__ float gn_update(const SolveArgs &a, const float (&t)[
     }
     const float mean_g = t[0] / wsum;
     const float norm_g = sqrtf(fmaxf(0.0f, fmaf(-t[0], mean_g, t[1])));
-    const float norm_f = __ldg(md + 0);
+    const float norm_f = load_row<SHARED>(md + 0);
     if (norm_g < 1e-9f || norm_f < 1e-9f) return -2.0f;
     const float ratio = norm_f / norm_g;
     const int sum_off = 2 + n;
@@ -287,24 +293,24 @@ __device__ __forceinline__ float gn_update(const SolveArgs &a, const float (&t)[
 #pragma unroll
     for (int k = 0; k < 12; ++k) delta[k] = 0.0f;
     if (MODEL == kModelTranslation) {
-        float r0 = fmaf(-ratio, fmaf(-mean_g, __ldg(md + sum_off + 0), jg[0]), __ldg(md + 2));
-        float r3 = fmaf(-ratio, fmaf(-mean_g, __ldg(md + sum_off + 3), jg[3]), __ldg(md + 5));
-        float a0 = __ldg(hi + 0) * r0;
-        a0 = fmaf(__ldg(hi + 3), r3, a0);
-        float a3 = __ldg(hi + 18) * r0;
-        a3 = fmaf(__ldg(hi + 21), r3, a3);
+        float r0 = fmaf(-ratio, fmaf(-mean_g, load_row<SHARED>(md + sum_off + 0), jg[0]), load_row<SHARED>(md + 2));
+        float r3 = fmaf(-ratio, fmaf(-mean_g, load_row<SHARED>(md + sum_off + 3), jg[3]), load_row<SHARED>(md + 5));
+        float a0 = load_row<SHARED>(hi + 0) * r0;
+        a0 = fmaf(load_row<SHARED>(hi + 3), r3, a0);
+        float a3 = load_row<SHARED>(hi + 18) * r0;
+        a3 = fmaf(load_row<SHARED>(hi + 21), r3, a3);
         delta[0] = -a0;
         delta[3] = -a3;
     } else {
         float res[n];
 #pragma unroll
         for (int k = 0; k < n; ++k)
-            res[k] = fmaf(-ratio, fmaf(-mean_g, __ldg(md + sum_off + k), jg[k]), __ldg(md + 2 + k));
+            res[k] = fmaf(-ratio, fmaf(-mean_g, load_row<SHARED>(md + sum_off + k), jg[k]), load_row<SHARED>(md + 2 + k));
         if (MODEL == kModelQuadratic) {
             const int row = sl < n ? sl : 0;
             float acc = 0.0f;
 #pragma unroll
-            for (int k = 0; k < n; ++k) acc = fmaf(__ldg(hi + row * n + k), res[k], acc);
+            for (int k = 0; k < n; ++k) acc = fmaf(load_row<SHARED>(hi + row * n + k), res[k], acc);
 #pragma unroll
             for (int r = 0; r < n; ++r) delta[r] = -__shfl_sync(mask, acc, r, 16);
         } else {
@@ -312,7 +318,7 @@ __device__ __forceinline__ float gn_update(const SolveArgs &a, const float (&t)[
             for (int r = 0; r < n; ++r) {
                 float acc = 0.0f;
 #pragma unroll
-                for (int k = 0; k < n; ++k) acc = fmaf(__ldg(hi + r * n + k), res[k], acc);
+                for (int k = 0; k < n; ++k) acc = fmaf(load_row<SHARED>(hi + r * n + k), res[k], acc);
                 delta[r] = -acc;
             }
         }
@@ -320,17 +326,18 @@ __device__ __forceinline__ float gn_update(const SolveArgs &a, const float (&t)[
     float change;
     if (MODEL == kModelQuadratic) {
         if (!compose_quadratic(w, delta, sl, mask)) return -1.0f;
-        change = 0.0f;
+        // control point `sl` on each lane of the segment (0 again beyond the ninth)
+        const int p = sl < 9 ? sl : 0;
+        const float x = (float)(p % 3 - 1) * half, y = (float)(p / 3 - 1) * half;
+        const float hx2 = 0.5f * x * x, xy = x * y, hy2 = 0.5f * y * y;
+        float ca = fmaf(delta[2], y, fmaf(delta[1], x, delta[0]));
+        ca = ca + fmaf(delta[6], hx2, fmaf(delta[7], xy, delta[8] * hy2));
+        float cb = fmaf(delta[5], y, fmaf(delta[4], x, delta[3]));
+        cb = cb + fmaf(delta[9], hx2, fmaf(delta[10], xy, delta[11] * hy2));
+        change = length2(ca, cb);
 #pragma unroll
-        for (int p = 0; p < 9; ++p) {
-            float x = (float)(p % 3 - 1) * half, y = (float)(p / 3 - 1) * half;
-            float hx2 = 0.5f * x * x, xy = x * y, hy2 = 0.5f * y * y;
-            float ca = fmaf(delta[2], y, fmaf(delta[1], x, delta[0]));
-            ca = ca + fmaf(delta[6], hx2, fmaf(delta[7], xy, delta[8] * hy2));
-            float cb = fmaf(delta[5], y, fmaf(delta[4], x, delta[3]));
-            cb = cb + fmaf(delta[9], hx2, fmaf(delta[10], xy, delta[11] * hy2));
-            change = fmaxf(change, length2(ca, cb));
-        }
+        for (int off = 8; off >= 1; off >>= 1) change = fmaxf(change, __shfl_xor_sync(mask, change, off));
+        change = fmaxf(0.0f, change);
     } else if (MODEL == kModelTranslation) {
         w.t0 = w.t0 - delta[0];
         w.t1 = w.t1 - delta[3];
@@ -366,18 +373,14 @@ __device__ __forceinline__ float gn_update(const SolveArgs &a, const float (&t)[
 // One pixel's contribution to the lane's sums (icgn.wgsl:712-780), in the
 // reference's order: sum w g, w g^2, w f g, then the Jacobian-weighted terms.
 template <int MODEL, bool GAUSS, int N>
-__device__ __forceinline__ void accumulate_pixel(float (&s)[N], const SolveArgs &a, float g, unsigned ridx, int p,
-                                                 float lx, float ly, float ref_mean, float hx2, float xy,
-                                                 float hy2) {
-    const float4 rv = __ldg(a.plane + ridx);
-    const float f = rv.x - ref_mean;
+__device__ __forceinline__ void accumulate_values(float (&s)[N], float g, float f, float gx, float gy, float wt,
+                                                  float lx, float ly, float hx2, float xy, float hy2) {
     float wc = g, wf = f;
     if (GAUSS) {
-        const float wt = __ldg(a.weights + p);
         wc = wt * g;
         wf = wt * f;
     }
-    const float gxg = rv.y * wc, gyg = rv.z * wc;
+    const float gxg = gx * wc, gyg = gy * wc;
     s[0] = s[0] + wc;
     s[1] = fmaf(wc, g, s[1]);
     s[2] = fmaf(wf, g, s[2]);
@@ -400,6 +403,15 @@ __device__ __forceinline__ void accumulate_pixel(float (&s)[N], const SolveArgs 
             s[14] = fmaf(gyg, hy2, s[14]);
         }
     }
+}
+
+template <int MODEL, bool GAUSS, int N>
+__device__ __forceinline__ void accumulate_pixel(float (&s)[N], const SolveArgs &a, float g, unsigned ridx, int p,
+                                                 float lx, float ly, float ref_mean, float hx2, float xy,
+                                                 float hy2) {
+    const float4 rv = __ldg(a.plane + ridx);
+    accumulate_values<MODEL, GAUSS, N>(s, g, rv.x - ref_mean, rv.y, rv.z, GAUSS ? __ldg(a.weights + p) : 1.0f, lx, ly,
+                                       hx2, xy, hy2);
 }
 
 // Packed FP32 pairs (sm_100 FADD2 / FMUL2 / FFMA2): component k of every
@@ -860,6 +872,27 @@ __global__ void __launch_bounds__(128, MODEL == kModelQuadratic ? GBDIC_QUAD_MIN
     }
 }
 
+// Banded loop (solver_band.cuh) of B-spline windows with 16 or 32 lanes.
+template <int MODEL, int LANES, bool GAUSS>
+__global__ void icgn_band_kernel(SolveArgs a);
+
+#define GBDIC_BAND_CASE(MODEL, LANES)                                                             \
+    if (interp == kInterpBspline && a.band.rows > 0 && lanes == LANES) {                          \
+        const size_t smem = 4 * band_warp_floats(a, MODEL, LANES) * sizeof(float);                \
+        const int ctas = a.persistent ? grid : icgn_band_grid(a, LANES);                           \
+        if (occupancy_only) {                                                                      \
+            return gauss ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(                          \
+                               occupancy_only, icgn_band_kernel<MODEL, LANES, true>, 128, smem)    \
+                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(                          \
+                               occupancy_only, icgn_band_kernel<MODEL, LANES, false>, 128, smem);  \
+        }                                                                                          \
+        if (gauss)                                                                                 \
+            icgn_band_kernel<MODEL, LANES, true><<<ctas, 128, smem, stream>>>(a);                  \
+        else                                                                                       \
+            icgn_band_kernel<MODEL, LANES, false><<<ctas, 128, smem, stream>>>(a);                 \
+        return cudaGetLastError();                                                                 \
+    }
+
 #define GBDIC_SOLVER_CASE(MODEL, INTERP, LANES)                                                   \
     if (interp == INTERP && lanes == LANES) {                                                     \
         if (occupancy_only) {                                                                      \
@@ -887,6 +920,8 @@ __global__ void __launch_bounds__(128, MODEL == kModelQuadratic ? GBDIC_QUAD_MIN
     template <>                                                                                    \
     cudaError_t launch_icgn_model<MODEL>(const SolveArgs &a, int interp, int lanes, bool gauss,    \
                                          int grid, cudaStream_t stream, int *occupancy_only) {     \
+        GBDIC_BAND_CASE(MODEL, 16)                                                                 \
+        GBDIC_BAND_CASE(MODEL, 32)                                                                 \
         GBDIC_SOLVER_CASE(MODEL, kInterpBspline, 16)                                               \
         GBDIC_SOLVER_CASE(MODEL, kInterpBspline, 32)                                               \
         GBDIC_SOLVER_CASE(MODEL, kInterpBspline, 64)                                               \

@@ -1,0 +1,97 @@
+"""The banded IC-GN loop (solver_band.cuh) against the CPU oracle, bit for bit.
+
+Complete B-spline windows with 16 or 32 lanes are sampled by vertical runs
+into shared memory and accumulated from there in the reference's order.  The
+sizes below are where that can go wrong: runs of every length modulo the
+ring's four rows, one to five bands (the last one overlapping the band above
+it), windows narrower than the lanes, one more column than the lanes walk at
+once, tiled grids (whose plane is centred per window), Gaussian weights, and
+warps that leave the frame, cross tap rows and columns, bulge over the border
+(quadratic) and stop after different iteration counts within a warp."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from live_dic_gb300 import ICGNWGPU, synthetic
+from oracle import oracle as oracle_c
+from oracle import reference_prep as rp
+
+pytestmark = pytest.mark.gpu
+
+W, H = 203, 171
+
+
+@pytest.fixture(scope="module")
+def pairs():
+    ref, sp = synthetic.reference_image(W, H, seed=301, device="cpu")
+    strong = synthetic.affine_field(0.6, 2e-2, -3e-2, 1.1, 2.5e-2, -1.5e-2)
+
+    def bulge(X, Y):
+        u, v = strong(X - W / 2, Y - H / 2)
+        return u + 3e-4 * (X - W / 2) ** 2, v - 2e-4 * (Y - H / 2) ** 2
+
+    shift = synthetic.affine_field(1.37, 0.0, 0.0, -2.21, 0.0, 0.0)
+    return ref, {name: synthetic.deformed_image(sp, field, noise_seed=302, device="cpu")
+                 for name, field in (("affine", strong), ("quadratic", bulge), ("translation", shift))}
+
+
+CASES = [("affine", 31, 8, 16, "uniform"), ("affine", 29, 14, 16, "uniform"), ("affine", 27, 9, 16, "gaussian"),
+         ("affine", 21, 7, 16, "uniform"), ("affine", 41, 13, 16, "uniform"), ("affine", 16, 16, 16, "uniform"),
+         ("affine", 61, 20, 16, "gaussian"), ("affine", 32, 11, 32, "uniform"), ("affine", 41, 41, 32, "gaussian"),
+         ("affine", 25, 12, 32, "uniform"), ("quadratic", 41, 10, 16, "uniform"), ("quadratic", 13, 6, 16, "uniform"),
+         ("quadratic", 33, 11, 16, "gaussian"), ("quadratic", 65, 21, 16, "uniform"),
+         ("quadratic", 21, 21, 32, "uniform"), ("translation", 15, 5, 16, "uniform"),
+         ("translation", 17, 17, 16, "gaussian"), ("translation", 49, 24, 16, "uniform"),
+         ("translation", 16, 8, 32, "uniform"), ("translation", 81, 30, 32, "uniform")]
+
+
+@pytest.mark.parametrize("model,size,stride,lanes,weighting", CASES)
+def test_banded_loop_bit_exact(pairs, model, size, stride, lanes, weighting):
+    ref, targets = pairs
+    tgt = targets[model]
+    plane, inverse, metadata = rp.reference_arrays(ref, motion_model=model, subset_size=size, subset_stride=stride,
+                                                   spatial_weighting=weighting)
+    gw, gh = 1 + (W - size) // stride, 1 + (H - size) // stride
+    width = 16 if model == "quadratic" else 8
+    n = 12 if model == "quadratic" else 6
+    rng = np.random.default_rng(size)
+    # seeds near and far from the field: unequal iteration counts, some windows pushed off the frame
+    seeds = np.zeros((gh * gw, width), np.float32)
+    seeds[:, 0], seeds[:, 3] = rng.normal(0.0, 1.5, (2, gh * gw))
+    coef = oracle_c.prefilter(tgt, rp.runtime_fir_taps())
+    kw = dict(subset_size=size, subset_stride=stride, model=model, lanes=lanes, tolerance=1e-4)
+    with ICGNWGPU(subset_size=size, subset_stride=stride, motion_model=model, outlier_policy="disabled",
+                  solver_workgroup_size=lanes, spatial_weighting=weighting) as engine:
+        engine.set_reference_arrays(W, H, plane, metadata, inverse, tolerance=1e-4)
+        weights = engine.export_weights() if weighting == "gaussian" else None
+        result = engine.register(tgt)
+        got = np.concatenate([result.parameters, result.status[..., None], result.iterations[..., None]], -1)
+        seeded = engine._register_seeded_states(tgt, seeds.reshape(gh, gw, width), np.ones((gh, gw), np.uint32))
+    expected = oracle_c.solve(tgt, coef, plane, metadata, inverse, weights=weights, **kw)
+    np.testing.assert_array_equal(got, expected.reshape(gh, gw, -1)[..., :n + 2])
+    expected = oracle_c.solve(tgt, coef, plane, metadata, inverse, weights=weights, seed_state=seeds,
+                              active=np.ones(gh * gw, np.uint32), **kw)
+    np.testing.assert_array_equal(seeded[..., :n + 2], expected.reshape(gh, gw, -1)[..., :n + 2])
+    assert (got[..., n] > 0.5).any() and len(np.unique(got[..., n + 1])) > 1
+
+
+@pytest.mark.parametrize("lanes", [16, 32])
+def test_prepared_plane_copies(pairs, lanes):
+    """A reference prepared on the GPU (overlapping and tiled windows) gives the oracle's field on its exported
+    arrays, also after another reference of the same size replaced it."""
+    ref, targets = pairs
+    tgt = targets["affine"]
+    coef = oracle_c.prefilter(tgt, rp.runtime_fir_taps())
+    for size, stride in ((31, 10), (21, 21)):
+        with ICGNWGPU(subset_size=size, subset_stride=stride, outlier_policy="disabled",
+                      solver_workgroup_size=lanes) as engine:
+            for image in (np.ascontiguousarray(ref[::-1]), ref):
+                engine.set_reference(image)
+            result = engine.register(tgt)
+            plane, inverse, metadata = engine.export_reference()
+        got = np.concatenate([result.parameters, result.status[..., None], result.iterations[..., None]], -1)
+        expected = oracle_c.solve(tgt, coef, plane, metadata, inverse, subset_size=size, subset_stride=stride,
+                                  lanes=lanes)
+        np.testing.assert_array_equal(got, expected.reshape(got.shape))
