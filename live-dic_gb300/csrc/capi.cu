@@ -78,6 +78,7 @@ int guarded(Handle *h, F &&f) {
 struct gbdic_engine {
     std::unique_ptr<gbdic::Runtime> rt;
     gbdic::Level level;
+    gbdic::DeviceBuffer zncc;  // final ZNCC per subset
     std::vector<SlotHost> host;
     std::vector<gbdic_solver_cfg> slot_cfg;
     bool ready = false;
@@ -382,12 +383,14 @@ int gbdic_final_zncc(gbdic_engine *e, float *out_zncc) {
             fail(GBDIC_EINVAL, "include_zncc requires affine motion and uniform full windows");
         auto &lvl = e->level;
         auto &slot = *lvl.slots[0];
-        gbdic::DeviceBuffer out;
+        gbdic::DeviceBuffer &out = e->zncc;
         out.ensure((size_t)lvl.count * sizeof(float));
         gbdic::ZnccArgs z{};
         z.coef = slot.coef.as<float>();
         z.img = slot.frame.as<uint8_t>();
         z.plane = lvl.plane.as<float4>();
+        z.plane_f = lvl.solver_f;
+        z.band = gbdic::zncc_bands(e->rt->opts().o.subset_size, e->rt->opts().o.interpolation);
         z.state = e->rt->output_state(slot);
         z.out = out.as<float>();
         z.W = lvl.W; z.H = lvl.H; z.grid_w = lvl.gw; z.count = lvl.count;

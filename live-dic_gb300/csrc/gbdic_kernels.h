@@ -121,10 +121,13 @@ struct ZnccArgs {
     const float *coef;
     const uint8_t *img;
     const float4 *plane;
+    const float *plane_f;  // its f as a plane of its own, or nullptr
     const float *state;
     float *out;
     int W, H, grid_w, count, S, stride, interp;
+    BandPlan band;         // B-spline windows: how a warp samples one (zncc_bands), else rows 0
 };
+BandPlan zncc_bands(int S, int interp);
 cudaError_t launch_final_zncc(const ZnccArgs &a, cudaStream_t stream);
 
 // ------------------------------------------------------------ pyramid

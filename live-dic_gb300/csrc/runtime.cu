@@ -348,7 +348,7 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
     check_cuda(cudaEventCreate(&e1), "event");
     cudaEventRecord(e0, stream_);
     check_cuda(launch_reference_prep(a, stream_), "reference preparation launch");
-    level.solver_f = level.intensity.as<float>();
+    level.solver_f = banded() ? level.intensity.as<float>() : nullptr;
     if (banded() && a.stride == a.S) split_plane(level, false);
     cudaEventRecord(e1, stream_);
     unsigned valid = 0;
@@ -372,6 +372,7 @@ void Runtime::upload_reference_arrays(Level &level, const float *plane, const fl
     level.inv.ensure((size_t)level.count * n * n * sizeof(float));
     level.partial_count = 0;
     check_cuda(cudaMemcpy(level.plane.get(), plane, px * sizeof(float4), cudaMemcpyHostToDevice), "plane upload");
+    level.solver_f = nullptr;
     if (banded()) {
         split_plane(level, true);
         check_cuda(cudaStreamSynchronize(stream_), "plane split");

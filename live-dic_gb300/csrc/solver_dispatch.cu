@@ -107,6 +107,29 @@ BandPlan plan_bands(int S, int model, int interp, int lanes, int sm_count) {
     return best;
 }
 
+// The final ZNCC samples a window once, with all lanes of a warp; its direct
+// kernel is slower at every size (no limit on the steps).
+BandPlan zncc_bands(int S, int interp) {
+    BandPlan best{};
+    if (interp != kInterpBspline || S > kMaxBandFloats) return best;
+    double steps = 1e30;
+    for (int bands = 1; bands <= S; ++bands) {
+        const int rows = (S + bands - 1) / bands;
+        if (rows * S > kMaxBandFloats) continue;
+        int run = 0, segments = 0;
+        const double cost = (S + rows - 1) / rows * band_steps(S, rows, 32, run, segments);
+        if (cost < steps) {
+            steps = cost;
+            best.rows = rows;
+            best.run = best.run32 = run;
+            best.segments = best.segments32 = segments;
+        }
+    }
+    best.magic = ((1u << 20) + S - 1) / S;
+    best.pitch = (best.rows * S + 31) / 32 * 32;
+    return best;
+}
+
 // CTAs of a non-persistent launch of the banded loop.
 int icgn_band_grid(const SolveArgs &a, int lanes) {
     const int per_warp = lanes == 16 && a.count > a.band.solo_count ? 2 : 1;

@@ -2,6 +2,7 @@
 // temporal kernels (reference: shaders/full_pyramid.wgsl).
 #include "gbdic_common.cuh"
 #include "gbdic_kernels.h"
+#include "solver_band.cuh"
 
 namespace gbdic {
 
@@ -69,6 +70,117 @@ __global__ void __launch_bounds__(128) final_zncc_kernel(ZnccArgs a) {
     } else {
         a.out[index] = -2.0f;
     }
+}
+
+// final_zncc_kernel of B-spline windows, a warp to a subset: the window is
+// sampled as by the banded solver loop (sample_band: tap rows in a register
+// ring, two runs to a lane), then every lane adds the pixels of the two of
+// the 64 lanes it stands for, in their order.  The value is defined only if
+// every pixel lands in [2, W-3] x [2, H-3], so the check is made on the four
+// corner pixels; pixels between corners that lie inside by a margin lie
+// inside too (an affine map, rounded far below the margin), and a window
+// closer to the bound is checked pixel by pixel.
+// FMA-bound as the solver's sampling.  UHD S 31 / s 8 (127,359 subsets): 1,011
+// us with sixteen clamped taps gathered and two integer divisions per pixel
+// (final_zncc_kernel), 517 us here.
+__global__ void __launch_bounds__(128, kBandBlocks) final_zncc_band_kernel(SolveArgs a, const float *f_plane, int f_pitch,
+                                                                           float *out) {
+    extern __shared__ float band_smem[];
+    const int lane = threadIdx.x & 31, index = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (index >= a.count) return;  // warp-uniform
+    float *buf = band_smem + (threadIdx.x >> 5) * a.band.pitch;
+    const float4 *st = reinterpret_cast<const float4 *>(a.state + (size_t)index * 8);
+    const float4 p = __ldg(st), q = __ldg(st + 1);
+    const Warp w = {p.x, p.w, p.y, p.z, q.x, q.y, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    const int S = a.S, W = a.W, H = a.H;
+    const int px0 = (index % a.grid_w) * a.stride, py0 = (index / a.grid_w) * a.stride;
+    const float half = ((float)S - 1.0f) * 0.5f;
+    auto position = [&](int col, int row, float &tx, float &ty) {
+        const float lx = (float)col - half, ly = (float)row - half;
+        float dx, dy;
+        displacement<kModelAffine>(w, lx, ly, 0.0f, 0.0f, 0.0f, dx, dy);
+        tx = (float)(px0 + col) + dx;
+        ty = (float)(py0 + row) + dy;
+    };
+    auto inside = [&](float tx, float ty, float m) {
+        return tx >= 2.0f + m && ty >= 2.0f + m && tx <= (float)(W - 3) - m && ty <= (float)(H - 3) - m;
+    };
+    float tx, ty;
+    position((lane & 1) * (S - 1), ((lane >> 1) & 1) * (S - 1), tx, ty);
+    bool valid = q.z == 1.0f && __all_sync(kFullMask, inside(tx, ty, 0.0f));
+    if (valid && !__all_sync(kFullMask, inside(tx, ty, 0.0625f + 1e-6f * (float)(W + H)))) {
+        bool all = true;
+        for (int k = lane; k < S * S; k += 32) {
+            position(k % S, k / S, tx, ty);
+            all = all && inside(tx, ty, 0.0f);
+        }
+        valid = __all_sync(kFullMask, all);
+    }
+    if (!valid) {
+        if (lane == 0) out[index] = -2.0f;
+        return;
+    }
+    float s[2][5];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int k = 0; k < 5; ++k) s[h][k] = 0.0f;
+    const int rows = a.band.rows;
+    const float *f_window = f_plane + ((size_t)py0 * W + px0) * f_pitch;
+    for (int first = 0; first < S; first += rows) {
+        const int top = min(first, S - rows), last = min(first + rows, S);
+        __syncwarp();
+        sample_band<kModelAffine>(a, w, buf, top, lane, 32, px0, py0, half);
+        __syncwarp();
+        const float *g = buf - top * S;
+        // pixel 32 m + lane belongs to lane 32 (m & 1) + lane of the 64
+        const int end = last * S;
+        int m = first * S / 32;
+        int k = 32 * m + lane;
+        int row = k / S, col = k - row * S;
+        const int sdiv = div_subset(a, 32), smod = 32 - sdiv * S;
+        auto add = [&](float (&t)[5]) {
+            if (k >= first * S && k < end) {
+                const float fv = __ldg(f_window + (size_t)(row * W + col) * f_pitch), gv = g[k];
+                t[0] = t[0] + fv;
+                t[1] = t[1] + gv;
+                t[2] = fmaf(fv, fv, t[2]);
+                t[3] = fmaf(gv, gv, t[3]);
+                t[4] = fmaf(fv, gv, t[4]);
+            }
+            k += 32;
+            row += sdiv;
+            col += smod;
+            if (col >= S) { col -= S; ++row; }
+        };
+        if (m & 1) {
+            add(s[1]);
+            ++m;
+        }
+#pragma unroll 4
+        for (; 32 * m < end; m += 2) {
+            add(s[0]);
+            add(s[1]);
+        }
+    }
+    float t[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        float v = s[0][k] + s[1][k];
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) v = v + __shfl_down_sync(kFullMask, v, off);
+        t[k] = v;
+    }
+    if (lane != 0) return;
+    const float n = (float)(S * S), nn = fmaxf(n, 1.0f);
+    const float vf = t[2] - t[0] * t[0] / nn;
+    const float vg = t[3] - t[1] * t[1] / nn;
+    float value = -2.0f;
+    if (vf > 1e-9f && vg > 1e-9f) {
+        const float r = (t[4] - t[0] * t[1] / n) / sqrtf(vf * vg);
+        value = fminf(fmaxf(r, -1.0f), 1.0f);
+    }
+    out[index] = value;
 }
 
 // ------------------------------------------------------------ reduction
@@ -326,6 +438,16 @@ __global__ void temporal_merge_kernel(TemporalArgs a) {
 }  // namespace
 
 cudaError_t launch_final_zncc(const ZnccArgs &a, cudaStream_t stream) {
+    if (a.band.rows > 0) {
+        SolveArgs b{};
+        b.coef = a.coef;
+        b.state = const_cast<float *>(a.state);
+        b.W = a.W; b.H = a.H; b.grid_w = a.grid_w; b.count = a.count; b.S = a.S; b.stride = a.stride;
+        b.band = a.band;
+        final_zncc_band_kernel<<<(a.count + 3) / 4, 128, 4 * (size_t)a.band.pitch * sizeof(float), stream>>>(
+            b, a.plane_f ? a.plane_f : reinterpret_cast<const float *>(a.plane), a.plane_f ? 1 : 4, a.out);
+        return cudaGetLastError();
+    }
     if (a.count <= 0) return cudaSuccess;
     const int grid = (a.count + 1) / 2;
     switch (a.interp) {

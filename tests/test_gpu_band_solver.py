@@ -95,3 +95,24 @@ def test_prepared_plane_copies(pairs, lanes):
         expected = oracle_c.solve(tgt, coef, plane, metadata, inverse, subset_size=size, subset_stride=stride,
                                   lanes=lanes)
         np.testing.assert_array_equal(got, expected.reshape(got.shape))
+
+
+@pytest.mark.parametrize("size,stride", [(16, 16), (21, 10), (31, 8), (33, 11), (41, 13), (63, 20)])
+def test_final_zncc_by_bands(size, stride):
+    """The final ZNCC's band sampling against the oracle: a shift of about 2 px puts the first windows' corners
+    within a sixteenth of a pixel of the bound, on either side of it."""
+    ref, sp = synthetic.reference_image(W, H, seed=303, device="cpu")
+    tgt = synthetic.deformed_image(sp, synthetic.affine_field(2.0, 4e-4, -3e-4, 2.0, 2e-4, 5e-4), noise_seed=304,
+                                   device="cpu")
+    with ICGNWGPU(subset_size=size, subset_stride=stride) as engine:
+        engine.set_reference(ref)
+        result = engine.register_seeded(tgt, np.tile(np.array([2, 0, 0, 2, 0, 0], np.float32),
+                                                     (engine.grid_height, engine.grid_width, 1)),
+                                        np.ones((engine.grid_height, engine.grid_width), bool), include_zncc=True)
+        plane, _, _ = engine.export_reference()
+    state = np.concatenate([result.parameters, result.status[..., None], result.iterations[..., None]], -1)
+    coef = oracle_c.prefilter(tgt, rp.runtime_fir_taps())
+    expected = oracle_c.final_zncc(tgt, coef, plane, state.reshape(-1, 8), subset_size=size, subset_stride=stride)
+    expected[expected < -1.0] = np.nan
+    np.testing.assert_array_equal(result.zncc.ravel(), expected)
+    assert np.isfinite(expected).any()
