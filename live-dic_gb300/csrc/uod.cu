@@ -157,13 +157,15 @@ __device__ void median_motion(const UodArgs &a, int index) {
     store_state(a.out + (size_t)index * ss, ss, out);
 }
 
-__global__ void uod_kernel(UodArgs a) {
+__global__ void median_motion_kernel(UodArgs a) {
     const int index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= a.count) return;
-    if (a.policy == 3) {
-        median_motion(a, index);
-        return;
-    }
+    if (index < a.count) median_motion(a, index);
+}
+
+// 3x3 UOD of one quadratic subset by the reference's bubble sort of the valid
+// neighbours' values.  uod3_kernel comes here when a value is NaN: only then
+// does the order of the comparisons show in a median.
+__device__ __noinline__ void quadratic_uod_unordered(const UodArgs &a, int index) {
     const int ss = state_stride(a.model);
     const int sat = status_slot(a.model);
     float own[16];
@@ -181,7 +183,6 @@ __global__ void uod_kernel(UodArgs a) {
                 if (dx == 0 && dy == 0) continue;
                 const int nx = px + dx, ny = py + dy;
                 if (nx < 0 || ny < 0 || nx >= a.grid_w || ny >= a.grid_h) continue;
-                if (a.model != kModelQuadratic && !allowed(a, index, dx, dy, false)) continue;
                 const float *ns = a.state + ((size_t)ny * a.grid_w + nx) * ss;
                 if (ns[sat] < 0.5f) continue;
                 load_state(ns, ss, nbr);
@@ -249,10 +250,32 @@ __device__ __forceinline__ float median_sorted8(const float (&v)[8], int count) 
     }
 }
 
-// 3x3 UOD (replace / flag) of translation and affine states with every
-// neighbour in registers: the neighbour slots keep the scan order of the
-// generic kernel, missing ones read +inf, and the order statistics come
-// from sort8, so the result equals uod_kernel's bit for bit.
+// Component `comp` of the neighbours in the slots set in `valid`, recentred on
+// this subset; +inf in the others.
+template <int MODEL>
+__device__ __forceinline__ void neighbour_values(const UodArgs &a, int index, unsigned valid, int comp, float (&v)[8]) {
+    constexpr int ss = state_stride(MODEL);
+#pragma unroll
+    for (int slot = 0; slot < 8; ++slot) {
+        const int cell = slot < 4 ? slot : slot + 1;  // 3x3 scan order without the centre
+        const int dx = cell % 3 - 1, dy = cell / 3 - 1;
+        v[slot] = __int_as_float(0x7f800000);
+        if (valid >> slot & 1u) {
+            float nbr[ss];
+            load_state(a.state + ((size_t)index + dy * a.grid_w + dx) * ss, ss, nbr);
+            v[slot] = recentered(MODEL, nbr, comp, -(float)a.subset_stride * (float)dx, -(float)a.subset_stride * (float)dy);
+        }
+    }
+}
+
+// 3x3 UOD (replace / flag) with the neighbours' values in registers: the slots
+// keep the scan order of the reference, missing ones read +inf, and the
+// order statistics come from sort8, so the result equals its bubble sort's
+// bit for bit.  Only the translations decide whether a subset is an outlier;
+// the other components' medians are taken for the few that are.  Bound by
+// HBM / L2 reads of the states: UHD S 41 / s 10 quadratic (80,560 subsets)
+// 112 us with every component's values in local memory, 16.5 us here; UHD
+// S 31 / s 8 affine (127,359 subsets) 10.8 us with every median taken, 7.5.
 template <int MODEL>
 __global__ void __launch_bounds__(128) uod3_kernel(UodArgs a) {
     constexpr int ss = state_stride(MODEL), sat = status_slot(MODEL), nc = parameter_count(MODEL);
@@ -260,76 +283,84 @@ __global__ void __launch_bounds__(128) uod3_kernel(UodArgs a) {
     if (index >= a.count) return;
     float own[ss];
     load_state(a.state + (size_t)index * ss, ss, own);
-    float out[ss];
-#pragma unroll
-    for (int k = 0; k < ss; ++k) out[k] = own[k];
     if (own[sat] >= 0.5f) {
         const int px = index % a.grid_w, py = index / a.grid_w;
         const float kInf = __int_as_float(0x7f800000);
-        float nb[8][nc];
-        bool valid[8];
-        int count = 0;
+        float nb[2][8];  // tx, ty
+        unsigned valid = 0u;
 #pragma unroll
         for (int slot = 0; slot < 8; ++slot) {
-            const int cell = slot < 4 ? slot : slot + 1;  // 3x3 scan order without the centre
+            const int cell = slot < 4 ? slot : slot + 1;
             const int dx = cell % 3 - 1, dy = cell / 3 - 1;
             const int nx = px + dx, ny = py + dy;
-            bool ok = nx >= 0 && ny >= 0 && nx < a.grid_w && ny < a.grid_h && allowed(a, index, dx, dy, false);
-            float nbr[ss];
+            bool ok = nx >= 0 && ny >= 0 && nx < a.grid_w && ny < a.grid_h &&
+                      (MODEL == kModelQuadratic || allowed(a, index, dx, dy, false));
+            nb[0][slot] = nb[1][slot] = kInf;
             if (ok) {
+                float nbr[ss];
                 load_state(a.state + ((size_t)ny * a.grid_w + nx) * ss, ss, nbr);
-                ok = nbr[sat] >= 0.5f;
+                if (nbr[sat] >= 0.5f) {
+                    const float ox = -(float)a.subset_stride * (float)dx, oy = -(float)a.subset_stride * (float)dy;
+                    valid |= 1u << slot;
+                    nb[0][slot] = recentered(MODEL, nbr, 0, ox, oy);
+                    nb[1][slot] = recentered(MODEL, nbr, 3, ox, oy);
+                }
             }
-            valid[slot] = ok;
-            count += ok ? 1 : 0;
-            const float ox = -(float)a.subset_stride * (float)dx, oy = -(float)a.subset_stride * (float)dy;
-#pragma unroll
-            for (int k = 0; k < nc; ++k) nb[slot][k] = ok ? recentered(MODEL, nbr, k, ox, oy) : kInf;
         }
+        const int count = __popc(valid);
         if (count >= 4) {
-            float filtered[nc], medians[nc];
-#pragma unroll
-            for (int k = 0; k < nc; ++k) filtered[k] = medians[k] = own[k];
-            constexpr int model_components = MODEL == kModelTranslation ? 2 : nc;
-            const int median_count = a.policy == 1 ? model_components : 2;
-#pragma unroll
-            for (int ai = 0; ai < model_components; ++ai) {
-                if (ai >= median_count) break;
-                const int comp = ai == 0 ? 0 : (ai == 1 ? 3 : (ai == 2 ? 1 : (ai == 3 ? 2 : ai)));
-                float v[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = nb[i][comp];
-                sort8(v);
-                medians[comp] = median_sorted8(v, count);
-            }
+            bool unordered = false;
+            float medians[2];
             bool flagged = false;
 #pragma unroll
             for (int ai = 0; ai < 2; ++ai) {
-                const int comp = ai == 0 ? 0 : 3;
                 float v[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = valid[i] ? fabsf(nb[i][comp] - medians[comp]) : kInf;
+                for (int i = 0; i < 8; ++i) v[i] = nb[ai][i];
+                sort8(v);
+                medians[ai] = median_sorted8(v, count);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    v[i] = valid >> i & 1u ? fabsf(nb[ai][i] - medians[ai]) : kInf;
+                    unordered = unordered || !(v[i] >= 0.0f);
+                }
                 sort8(v);
                 const float spread = median_sorted8(v, count);
-                const float score = fabsf(filtered[comp] - medians[comp]) / (spread + 0.1f);
-                if (score > 2.0f) flagged = true;
+                if (fabsf(own[ai * 3] - medians[ai]) / (spread + 0.1f) > 2.0f) flagged = true;
+            }
+            if (MODEL == kModelQuadratic && unordered) {
+                quadratic_uod_unordered(a, index);
+                return;
             }
             if (flagged) {
                 if (a.policy == 1) {
+                    own[0] = medians[0];
+                    own[3] = medians[1];
+                    if (MODEL != kModelTranslation) {
 #pragma unroll
-                    for (int k = 0; k < model_components; ++k) {
-                        const int comp = k == 0 ? 0 : (k == 1 ? 3 : (k == 2 ? 1 : (k == 3 ? 2 : k)));
-                        filtered[comp] = medians[comp];
+                        for (int comp = 1; comp < nc; ++comp) {
+                            if (comp == 3) continue;
+                            float v[8];
+                            neighbour_values<MODEL>(a, index, valid, comp, v);
+                            if (MODEL == kModelQuadratic) {
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) unordered = unordered || isnan(v[i]);
+                            }
+                            sort8(v);
+                            own[comp] = median_sorted8(v, count);
+                        }
+                        if (MODEL == kModelQuadratic && unordered) {
+                            quadratic_uod_unordered(a, index);
+                            return;
+                        }
                     }
                 }
-#pragma unroll
-                for (int k = 0; k < nc; ++k) out[k] = filtered[k];
-                out[6] = 2.0f;
-                out[7] = own[7];
+                own[sat] = 2.0f;
+                if (MODEL == kModelQuadratic) own[14] = own[15] = 0.0f;
             }
         }
     }
-    store_state(a.out + (size_t)index * ss, ss, out);
+    store_state(a.out + (size_t)index * ss, ss, own);
 }
 
 }  // namespace
@@ -337,9 +368,10 @@ __global__ void __launch_bounds__(128) uod3_kernel(UodArgs a) {
 cudaError_t launch_uod(const UodArgs &a, cudaStream_t stream) {
     if (a.count <= 0) return cudaSuccess;
     const int grid = (a.count + 127) / 128;
-    if (a.policy != 3 && a.model == kModelAffine) uod3_kernel<kModelAffine><<<grid, 128, 0, stream>>>(a);
-    else if (a.policy != 3 && a.model == kModelTranslation) uod3_kernel<kModelTranslation><<<grid, 128, 0, stream>>>(a);
-    else uod_kernel<<<grid, 128, 0, stream>>>(a);
+    if (a.policy == 3) median_motion_kernel<<<grid, 128, 0, stream>>>(a);
+    else if (a.model == kModelAffine) uod3_kernel<kModelAffine><<<grid, 128, 0, stream>>>(a);
+    else if (a.model == kModelTranslation) uod3_kernel<kModelTranslation><<<grid, 128, 0, stream>>>(a);
+    else uod3_kernel<kModelQuadratic><<<grid, 128, 0, stream>>>(a);
     return cudaGetLastError();
 }
 

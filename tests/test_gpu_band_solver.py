@@ -116,3 +116,29 @@ def test_final_zncc_by_bands(size, stride):
     expected[expected < -1.0] = np.nan
     np.testing.assert_array_equal(result.zncc.ravel(), expected)
     assert np.isfinite(expected).any()
+
+
+@pytest.mark.parametrize("policy", ["replace", "flag"])
+def test_quadratic_outliers_bit_exact(pairs, policy):
+    """Planted outliers, rejected neighbours, infinities and NaNs in quadratic states."""
+    ref, _ = pairs
+    plane, inverse, metadata = rp.reference_arrays(ref, motion_model="quadratic", subset_size=21, subset_stride=10)
+    gw, gh = 1 + (W - 21) // 10, 1 + (H - 21) // 10
+    rng = np.random.default_rng(12)
+    state = np.zeros((gh, gw, 16), np.float32)
+    state[..., :12] = rng.normal(0, 1e-3, (gh, gw, 12))
+    state[..., 0] += 0.3 + rng.normal(0, 0.05, (gh, gw))
+    state[..., 3] += rng.normal(0, 0.05, (gh, gw))
+    state[..., 12] = rng.choice(np.array([1.0] * 12 + [0.0, -1.0], np.float32), (gh, gw))
+    state[..., 13] = 3.0
+    state[rng.random((gh, gw)) < 0.1, 0] += 2.5
+    state[2, 3, 0] = np.inf
+    state[9, 11, 4] = np.nan
+    state[12, 4, 3] = np.nan
+    with ICGNWGPU(subset_size=21, subset_stride=10, motion_model="quadratic", outlier_policy=policy) as engine:
+        engine.set_reference_arrays(W, H, plane, metadata, inverse)
+        got = engine.apply_outlier_filter(state)
+    expected = oracle_c.uod(state.reshape(-1, 16), metadata, grid=(gw, gh), subset_stride=10, model="quadratic",
+                            policy=policy)
+    np.testing.assert_array_equal(got.reshape(-1, 16), expected)
+    assert (got[..., 12] == 2.0).sum() > 5
