@@ -105,3 +105,29 @@ def test_device_shift_rows_match_host_estimate(shift):
     again = init.estimate(tgt)
     assert (again["dx"], again["dy"], again["peakScore"]) == (est["dx"], est["dy"], est["peakScore"])
     init.close()
+
+
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("size", [32, 64, 128, 256, 512, 1024])
+def test_every_window_size_matches_oracle(size, masked):
+    """The packed half-spectrum transforms of each window size: figures of the
+    oracle's float64 FFTs to 1e-9 (rounding of 2 log2(1024) levels and of the
+    normalisation stays below 1e-11 of them)."""
+    rng = np.random.default_rng(size + masked)
+    big = rng.integers(0, 256, (size + 40, size + 48)).astype(np.uint8)
+    shift = (6, -4)
+    ref = np.ascontiguousarray(big[16:16 + size + 3, 16:16 + size + 5])
+    tgt = np.ascontiguousarray(big[16 - shift[1]:16 - shift[1] + size + 3, 16 - shift[0]:16 - shift[0] + size + 5])
+    mask = None
+    if masked:
+        mask = np.ones(ref.shape, bool)
+        mask[: size // 3, size // 4:] = False
+    init = FourierInitializer(ref, mask)
+    expected = fourier_oracle.estimate(ref, tgt, mask)
+    raw = init._raw(tgt)
+    init.close()
+    assert init.size == size
+    np.testing.assert_array_equal(raw[:2], [expected["dx"], expected["dy"]])
+    np.testing.assert_allclose(raw[2:5], [expected["peakScore"], expected["overlap"], expected["correlation"]],
+                               rtol=1e-9, atol=1e-12)
+    np.testing.assert_allclose(raw[6], expected["std"], rtol=1e-12)
