@@ -397,6 +397,10 @@ int gbdic_fp32_peak_probe(int32_t device, double *tflops);
  * RegistrationResult (engine.py:106-327; wgpu_backend.py:2595-2668). */
 int gbdic_field_summary(const float *packed, int64_t count, int32_t stride, int32_t n, float *accepted_tx,
                         float *accepted_ty, float *accepted_iterations, int64_t *accepted, int64_t *replaced);
+/* The same counts with the FP64 means themselves: `means` receives the means of
+ * the accepted subsets' floats 0, 3 and n + 1 (zeros when none is accepted). */
+int gbdic_field_means(const float *packed, int64_t count, int32_t stride, int32_t n, double *means, int64_t *accepted,
+                      int64_t *replaced);
 
 /* Switch the IC-GN solver variant (lanes per subset 16/32/64/128, persistent
  * work queue on/off) of a prepared handle without re-preparing the reference;

@@ -363,15 +363,17 @@ int gbdic_batch_register(gbdic_batch *b, const uint8_t *const *frames, const int
         if (!frames || !out_states) fail(GBDIC_EINVAL, "frames and out_states are required");
         const auto t0 = std::chrono::steady_clock::now();
         b->rebuild();
+        std::vector<gbdic::HostRows> copies;
+        copies.reserve(b->jobs.size());
         for (size_t j = 0; j < b->jobs.size(); ++j) {
             auto &job = *b->jobs[j];
             if (!frames[j] || !out_states[j]) fail(GBDIC_EINVAL, "every job needs a frame and an output");
             const size_t W = (size_t)job.level.W, H = (size_t)job.level.H;
             const int64_t stride = row_strides ? row_strides[j] : (int64_t)W;
             if (stride < (int64_t)W) fail(GBDIC_EINVAL, "row_stride must be at least the width");
-            uint8_t *dst = b->in.as<uint8_t>() + job.in_offset;
-            gbdic::host_copy_rows(dst, frames[j], W, H, stride);
+            copies.push_back({b->in.as<uint8_t>() + job.in_offset, frames[j], W, H, stride});
         }
+        gbdic::host_copy_many(copies.data(), copies.size());
         const double upload_ms = gbdic::ms_since(t0);
         if (!b->host_graph) b->host_graph = b->capture(true);
         const auto t1 = std::chrono::steady_clock::now();
@@ -381,10 +383,14 @@ int gbdic_batch_register(gbdic_batch *b, const uint8_t *const *frames, const int
         gbdic::wait_event(b->end, gbdic::kWaitMs);
         const double execute_ms = gbdic::ms_since(t1);
         const auto t2 = std::chrono::steady_clock::now();
+        copies.clear();
         for (size_t j = 0; j < b->jobs.size(); ++j) {
             auto &job = *b->jobs[j];
-            gbdic::host_copy(out_states[j], b->out.as<uint8_t>() + job.out_offset, job.state_bytes);
+            const size_t rows = (size_t)job.level.gh, width = job.state_bytes / rows;
+            copies.push_back({reinterpret_cast<uint8_t *>(out_states[j]), b->out.as<uint8_t>() + job.out_offset, width,
+                              rows, (int64_t)width});
         }
+        gbdic::host_copy_many(copies.data(), copies.size());
         if (timing) {
             float dev = 0.0f;
             cudaEventElapsedTime(&dev, b->begin, b->end);

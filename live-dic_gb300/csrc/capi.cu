@@ -491,6 +491,21 @@ int gbdic_field_summary(const float *packed, int64_t count, int32_t stride, int3
     return GBDIC_OK;
 }
 
+int gbdic_field_means(const float *packed, int64_t count, int32_t stride, int32_t n, double *means, int64_t *accepted,
+                      int64_t *replaced) {
+    if (!packed || count < 0 || n < 4 || stride < n + 2 || !means || !accepted || !replaced) {
+        gbdic::set_thread_error("field summary arguments are invalid");
+        return GBDIC_EINVAL;
+    }
+    try {
+        gbdic::field_means(packed, count, stride, n, means, accepted, replaced);
+    } catch (const std::exception &x) {
+        gbdic::set_thread_error(x.what());
+        return GBDIC_ECUDA;
+    }
+    return GBDIC_OK;
+}
+
 int gbdic_set_partial_support(gbdic_engine *e, int32_t count, const int32_t *indices, const uint32_t *words,
                               int32_t words_per_window, const float *boxes, const float *metadata_rows,
                               const float *inverse_rows) {

@@ -38,6 +38,18 @@ void set_thread_error(const std::string &message);
 // bytes, source rows `stride` bytes apart.
 void host_copy(void *dst, const void *src, size_t bytes);
 void host_copy_rows(uint8_t *dst, const uint8_t *src, size_t width, size_t height, int64_t stride);
+// Several row copies as one pass (a batch's frames or fields): rows of `width`
+// bytes, `stride` apart at the source, dense at the destination.
+struct HostRows {
+    uint8_t *dst;
+    const uint8_t *src;
+    size_t width, height;
+    int64_t stride;
+};
+void host_copy_many(const HostRows *jobs, size_t count);
+// Counts and FP64 means of one packed field (see gbdic_field_means).
+void field_means(const float *packed, int64_t count, int32_t stride, int32_t n, double *means, int64_t *accepted,
+                 int64_t *replaced);
 constexpr double kWaitMs = 120000.0;
 
 // Owning device allocation.

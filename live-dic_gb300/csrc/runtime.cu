@@ -708,23 +708,103 @@ void host_copy(void *dst, const void *src, size_t bytes) {
     });
 }
 
-void host_copy_rows(uint8_t *dst, const uint8_t *src, size_t width, size_t height, int64_t stride) {
-    if (stride == (int64_t)width) {
-        host_copy(dst, src, width * height);
+namespace {
+
+// Rows [height k / parts, height (k + 1) / parts) of a copy.
+void copy_part(const HostRows &job, size_t k, size_t parts) {
+    const size_t begin = job.height * k / parts, end = job.height * (k + 1) / parts;
+    if (begin >= end) return;
+    if (job.stride == (int64_t)job.width) {
+        std::memcpy(job.dst + begin * job.width, job.src + begin * job.width, (end - begin) * job.width);
         return;
     }
-    if (width * height < kParallelCopyBytes) {
-        for (size_t r = 0; r < height; ++r) std::memcpy(dst + r * width, src + (size_t)r * stride, width);
+    for (size_t r = begin; r < end; ++r) std::memcpy(job.dst + r * job.width, job.src + (int64_t)r * job.stride, job.width);
+}
+
+// Subsets per partial sum of a field's means.
+constexpr int64_t kMeanBlock = 1024;
+// A field from which the means are worth waking the workers (about 15 us): a
+// megabyte is 33,000 affine subsets, some 35 us on one core.
+constexpr size_t kParallelMeanBytes = 1u << 20;
+
+struct FieldBlock {
+    double sum[3];
+    int64_t accepted, replaced;
+};
+
+// Four interleaved partial sums, so that the additions of a block overlap.
+FieldBlock block_means(const float *s, int64_t count, int32_t stride, int32_t n) {
+    double sum[3][4] = {};
+    FieldBlock b{};
+    const auto add = [&](const float *q, int lane) {
+        const float status = q[n];
+        const bool ok = status > 0.5f;
+        sum[0][lane] += ok ? (double)q[0] : 0.0;
+        sum[1][lane] += ok ? (double)q[3] : 0.0;
+        sum[2][lane] += ok ? (double)q[n + 1] : 0.0;
+        b.accepted += ok;
+        b.replaced += status > 1.5f;
+    };
+    const float *q = s;
+    int64_t i = 0;
+    for (; i + 4 <= count; i += 4, q += 4 * (int64_t)stride) {
+        add(q, 0);
+        add(q + stride, 1);
+        add(q + 2 * (int64_t)stride, 2);
+        add(q + 3 * (int64_t)stride, 3);
+    }
+    for (int lane = 0; i < count; ++i, ++lane, q += stride) add(q, lane);
+    for (int k = 0; k < 3; ++k) b.sum[k] = (sum[k][0] + sum[k][1]) + (sum[k][2] + sum[k][3]);
+    return b;
+}
+
+}  // namespace
+
+void host_copy_many(const HostRows *jobs, size_t count) {
+    size_t bytes = 0;
+    for (size_t j = 0; j < count; ++j) bytes += jobs[j].width * jobs[j].height;
+    if (bytes < kParallelCopyBytes) {
+        for (size_t j = 0; j < count; ++j) copy_part(jobs[j], 0, 1);
         return;
     }
     CopyPool &pool = CopyPool::get();
     const int parts = pool.width();
-    const size_t rows = (height + parts - 1) / parts;
     pool.run(parts, [&](int k) {
-        const size_t begin = (size_t)k * rows, end = std::min(height, begin + rows);
-        for (size_t r = begin; r < end; ++r) std::memcpy(dst + r * width, src + (size_t)r * stride, width);
+        for (size_t j = 0; j < count; ++j) copy_part(jobs[j], (size_t)k, (size_t)parts);
     });
 }
 
-}  // namespace gbdic
+void host_copy_rows(uint8_t *dst, const uint8_t *src, size_t width, size_t height, int64_t stride) {
+    const HostRows job{dst, src, width, height, stride};
+    host_copy_many(&job, 1);
+}
 
+// The sums are taken per block of 1,024 subsets and the blocks added in order,
+// so the result does not depend on how many workers shared them.
+void field_means(const float *packed, int64_t count, int32_t stride, int32_t n, double *means, int64_t *accepted,
+                 int64_t *replaced) {
+    const int64_t blocks = (count + kMeanBlock - 1) / kMeanBlock;
+    std::vector<FieldBlock> part((size_t)blocks);
+    const auto run = [&](int k, int parts) {
+        for (int64_t b = blocks * k / parts; b < blocks * (k + 1) / parts; ++b)
+            part[(size_t)b] = block_means(packed + b * kMeanBlock * stride, std::min(kMeanBlock, count - b * kMeanBlock),
+                                          stride, n);
+    };
+    if ((size_t)count * (size_t)stride * sizeof(float) < kParallelMeanBytes) {
+        run(0, 1);
+    } else {
+        CopyPool &pool = CopyPool::get();
+        const int parts = pool.width();
+        pool.run(parts, [&](int k) { run(k, parts); });
+    }
+    double sum[3] = {};
+    *accepted = *replaced = 0;
+    for (const FieldBlock &b : part) {
+        for (int k = 0; k < 3; ++k) sum[k] += b.sum[k];
+        *accepted += b.accepted;
+        *replaced += b.replaced;
+    }
+    for (int k = 0; k < 3; ++k) means[k] = *accepted ? sum[k] / (double)*accepted : 0.0;
+}
+
+}  // namespace gbdic

@@ -295,6 +295,33 @@ def test_result_summary_matches_numpy_selection(model):
     assert np.shares_memory(r.parameters, packed)
 
 
+@pytest.mark.parametrize("count,stride,accepted", [(1, 8, 1.0), (1, 8, 0.0), (1023, 8, 0.9), (1025, 16, 0.9),
+                                                  (32767, 8, 0.5), (40001, 8, 0.9), (40001, 16, 0.0)])
+def test_field_means_blocks_and_workers(count, stride, accepted):
+    """Counts exact; means against exact sums over one block, a ragged last
+    block and fields shared by the copy workers (each sum has fewer than
+    2,000 additions in a chain: below 2000 * 2^-53 of the magnitudes' mean)."""
+    import math
+
+    from live_dic_gb300.engine import result_from_packed
+
+    rng = np.random.default_rng(count + stride)
+    n = 12 if stride == 16 else 6
+    packed = (rng.normal(size=(1, count, stride)) * 10.0 ** rng.integers(-6, 6, (1, count, stride))).astype(np.float32)
+    packed[..., n] = np.where(rng.random((1, count)) < accepted, rng.choice([1.0, 2.0], size=(1, count)), -1.0)
+    r = result_from_packed(packed, motion_model="quadratic" if stride == 16 else "affine", timing={}, config={},
+                           width=64, height=64, subset_size=21, subset_stride=10)
+    mask = packed[..., n] > 0.5
+    assert r.accepted == int(mask.sum()) and r.replaced == int((packed[..., n] > 1.5).sum())
+    if not mask.any():
+        assert r.mean_translation is None and r.mean_iterations is None
+        return
+    for got, k in zip((*r.mean_translation, r.mean_iterations), (0, 3, n + 1)):
+        values = packed[..., k][mask].astype(np.float64)
+        tolerance = 2000 * 2.0 ** -53 * float(np.mean(np.abs(values)))
+        assert abs(got - math.fsum(values) / values.size) <= tolerance
+
+
 def test_package_exports_cover_the_reference_api():
     """live_dic.__all__ (__init__.py:21-41) without the headless-browser engine."""
     import live_dic_gb300
