@@ -102,9 +102,12 @@ struct Level {
     int W = 0, H = 0, gw = 0, gh = 0, count = 0;
     bool roi = false;
     DeviceBuffer plane, meta, inv, links, selected;
-    // The banded solver loop's copies: f (where the intensity plane is not it),
-    // (gx, gy), and the window's pixel table.
-    DeviceBuffer plane_f, plane_grad, pixel_table;
+    // For the banded solver loop: f where the intensity plane is not it, and,
+    // behind the plane in its allocation, (gx, gy) and the window's pixel table.
+    DeviceBuffer plane_f;
+    float2 *plane_grad = nullptr;
+    float4 *pixel_table = nullptr;
+    std::vector<float4> host_table;
     const float *solver_f = nullptr;
     DeviceBuffer intensity, spline, scratch, valid;  // preparation scratch
     DeviceBuffer admissible;                         // u8 per subset, ROI ignored
@@ -173,6 +176,7 @@ class Runtime {
     int persistent_grid(int lanes);
     const BandPlan &band_plan(int lanes) const { return band_plans_[lanes == 16 ? 0 : (lanes == 32 ? 1 : 2)]; }
     bool banded() const { return band_plans_[0].rows > 0 || band_plans_[1].rows > 0; }
+    void ensure_plane(Level &level);
     void split_plane(Level &level, bool gradients);
     // Switch the solver variant (lanes per subset, persistent queue).
     void set_variant(int lanes, bool persistent);

@@ -242,22 +242,31 @@ void Runtime::configure_level(Level &level, int W, int H, int slots) {
     grid_of(W, H, opt_.o.subset_size, opt_.o.subset_stride, level.gw, level.gh);
     level.count = level.gw * level.gh;
     level.slots.clear();
-    if (banded()) {
-        const int S = opt_.o.subset_size;
-        std::vector<float4> table((size_t)S * S);
-        for (int r = 0; r < S; ++r)
-            for (int c = 0; c < S; ++c) {
-                float4 &t = table[(size_t)r * S + c];
-                const uint32_t offset = (uint32_t)r * (uint32_t)W + (uint32_t)c;
-                t = make_float4((float)c - 0.5f * (S - 1), (float)r - 0.5f * (S - 1), opt_.weights[(size_t)r * S + c], 0.0f);
-                std::memcpy(&t.w, &offset, sizeof(offset));
-            }
-        level.pixel_table.ensure(table.size() * sizeof(float4));
-        check_cuda(cudaMemcpyAsync(level.pixel_table.get(), table.data(), table.size() * sizeof(float4),
-                                   cudaMemcpyHostToDevice, stream_), "pixel table upload");
-        check_cuda(cudaStreamSynchronize(stream_), "pixel table upload");
-    }
+    level.host_table.clear();
     ensure_slots(level, slots);
+}
+
+// The reference plane, and behind it what the banded loop reads: its pixel
+// table and the gradients on their own (one allocation: a prepared engine
+// costs its user three fewer).
+void Runtime::ensure_plane(Level &level) {
+    const size_t px = (size_t)level.W * level.H;
+    const int S = opt_.o.subset_size;
+    const size_t table = banded() ? (size_t)S * S : 0;
+    level.plane.ensure((px + table) * sizeof(float4) + (banded() ? px * sizeof(float2) : 0));
+    level.pixel_table = banded() ? level.plane.as<float4>() + px : nullptr;
+    level.plane_grad = banded() ? reinterpret_cast<float2 *>(level.plane.as<float4>() + px + table) : nullptr;
+    if (!banded() || !level.host_table.empty()) return;
+    level.host_table.resize(table);
+    for (int r = 0; r < S; ++r)
+        for (int c = 0; c < S; ++c) {
+            float4 &t = level.host_table[(size_t)r * S + c];
+            const uint32_t offset = (uint32_t)r * (uint32_t)level.W + (uint32_t)c;
+            t = make_float4((float)c - 0.5f * (S - 1), (float)r - 0.5f * (S - 1), opt_.weights[(size_t)r * S + c], 0.0f);
+            std::memcpy(&t.w, &offset, sizeof(offset));
+        }
+    check_cuda(cudaMemcpyAsync(level.pixel_table, level.host_table.data(), table * sizeof(float4),
+                               cudaMemcpyHostToDevice, stream_), "pixel table upload");
 }
 
 // f of the plane for the banded loop: the intensity plane, or a copy where
@@ -265,9 +274,8 @@ void Runtime::configure_level(Level &level, int W, int H, int slots) {
 void Runtime::split_plane(Level &level, bool gradients) {
     const size_t px = (size_t)level.W * level.H;
     level.plane_f.ensure(px * sizeof(float));
-    if (gradients) level.plane_grad.ensure(px * sizeof(float2));
     check_cuda(launch_split_plane(level.plane.as<float4>(), px, level.plane_f.as<float>(),
-                                  gradients ? level.plane_grad.as<float2>() : nullptr, stream_), "plane split");
+                                  gradients ? level.plane_grad : nullptr, stream_), "plane split");
     level.solver_f = level.plane_f.as<float>();
 }
 
@@ -293,7 +301,7 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
                                   const float *roi_links) {
     const int model = opt_.o.motion_model, n = parameter_count(model);
     const size_t px = (size_t)level.W * level.H;
-    level.plane.ensure(px * sizeof(float4));
+    ensure_plane(level);
     level.meta.ensure((size_t)level.count * meta_stride(model) * sizeof(float));
     level.inv.ensure((size_t)level.count * n * n * sizeof(float));
     level.intensity.ensure(px * sizeof(float));
@@ -332,8 +340,7 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
     a.spline = level.spline.as<float>();
     a.scratch = level.scratch.as<float>();
     a.plane = level.plane.as<float4>();
-    if (banded()) level.plane_grad.ensure(px * sizeof(float2));
-    a.plane_grad = banded() ? level.plane_grad.as<float2>() : nullptr;
+    a.plane_grad = level.plane_grad;
     a.meta = level.meta.as<float>();
     a.inv = level.inv.as<float>();
     a.valid_count = level.valid.as<unsigned>();
@@ -367,7 +374,7 @@ void Runtime::upload_reference_arrays(Level &level, const float *plane, const fl
                                       const float *links) {
     const int model = opt_.o.motion_model, n = parameter_count(model);
     const size_t px = (size_t)level.W * level.H;
-    level.plane.ensure(px * sizeof(float4));
+    ensure_plane(level);
     level.meta.ensure((size_t)level.count * meta_stride(model) * sizeof(float));
     level.inv.ensure((size_t)level.count * n * n * sizeof(float));
     level.partial_count = 0;
@@ -462,8 +469,8 @@ SolveArgs Runtime::solve_args(Level &level, LevelSlot &slot, const gbdic_solver_
     a.img = frame ? frame : slot.frame.as<uint8_t>();
     a.plane = level.plane.as<float4>();
     a.plane_f = level.solver_f;
-    a.plane_grad = level.plane_grad.as<float2>();
-    a.pixel_table = level.pixel_table.as<float4>();
+    a.plane_grad = level.plane_grad;
+    a.pixel_table = level.pixel_table;
     a.band = band_plan(opt_.lanes);
     a.meta = level.meta.as<float>();
     a.inv = level.inv.as<float>();
