@@ -60,6 +60,32 @@ def test_partial_solver_bit_exact(pair, model, interp, lanes):
     assert (flat[plan.partial_indices[admitted], 6] == 1).mean() > 0.8
 
 
+@pytest.mark.parametrize("lanes", [16, 32, 64, 128])
+@pytest.mark.parametrize("model,weighting,subset", [("affine", "gaussian", 21), ("translation", "uniform", 11),
+                                                    ("affine", "uniform", 47), ("translation", "gaussian", 61)])
+def test_partial_window_blocks_bit_exact(model, weighting, subset, lanes):
+    """A block to a partial window: every lane count's split of the sums, the
+    weights, and windows of more than one sampled chunk of 1,024 pixels."""
+    ref, sp = synthetic.reference_image(W, H, seed=303, device="cpu")
+    tgt = synthetic.deformed_image(sp, synthetic.affine_field(*FIELD), noise_seed=304, device="cpu")
+    mask = synthetic.hole_mask(W, H, 41.0)
+    with ICGNWGPU(subset_size=subset, subset_stride=9, motion_model=model, spatial_weighting=weighting,
+                  outlier_policy="disabled", solver_workgroup_size=lanes) as engine:
+        info = engine.set_reference(ref, roi_mask=mask, roi_policy="partial")
+        result = engine.register(tgt)
+        plane, inverse, metadata = engine.export_reference()
+        coef = engine.export_coefficients()
+        weights = engine.export_weights() if weighting == "gaussian" else None
+    plan = info.roi
+    assert plan.partial_indices.size > 0
+    common = dict(subset_size=subset, subset_stride=9, model=model, lanes=lanes, roi_enabled=True, weights=weights)
+    state = oracle_c.solve(tgt, coef, plane, metadata, inverse, **common)
+    state = oracle_c.solve(tgt, coef, plane, metadata, inverse, **common, state=state,
+                           partial=(plan.partial_indices, plan.support_words, plan.support_boxes))
+    got = _packed(result)
+    np.testing.assert_array_equal(got, state.reshape(got.shape[0], got.shape[1], -1)[..., : got.shape[-1]])
+
+
 def test_partial_windows_recover_field_under_hole(pair):
     ref, tgt = pair
     mask = synthetic.hole_mask(W, H, 45.0)
