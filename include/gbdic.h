@@ -577,6 +577,21 @@ typedef struct {
  * gbdic_nn_gemm on the materialised matrix, which is never written. */
 int gbdic_nn_conv_gemm(const gbdic_nn_gemm_desc *desc, int32_t mode, const gbdic_nn_conv_shape *shape,
                        int32_t *device_error, void *stream);
+/* Mode 2 with the ReLU backward and bias gradient of the layer below in its
+ * epilogue: desc->d_bf16 (BF16, M x N, row stride ldd; d_f32 and bias NULL)
+ * receives dY where y (its activations, BF16, the same rows and stride) is
+ * positive and 0 elsewhere; db[n] its column sums before rounding, in a fixed
+ * order.  partial: device scratch of N * M / 128 floats. */
+int gbdic_nn_conv_dgrad_relu(const gbdic_nn_gemm_desc *desc, const gbdic_nn_conv_shape *shape, const void *y,
+                             float *partial, float *db, int32_t *device_error, void *stream);
+/* Weight gradient dw[Cout][Kp] = sum over output pixels of the im2col row of x
+ * (NHWC BF16, C % 8 == 0) times dz (B*OH*OW x Cout BF16, Cout % 64 == 0), with
+ * neither operand transposed nor the im2col matrix written.  With fewer than
+ * eight channels (Kp 64, Cout 32) x is the matrix gbdic_nn_im2col wrote.
+ * Pixels are split over `splits` partial sums (B*OH*OW % (64 splits) == 0) in
+ * `partial` (splits * Kp * Cout floats), added in split order. */
+int gbdic_nn_conv_wgrad(const gbdic_nn_conv_shape *shape, const void *x, const void *dz, int32_t splits,
+                        float *partial, float *dw, int32_t *device_error, void *stream);
 /* Forward GEMM operand A[(b, oy, ox)][(ky, kx, ci)] (zero beyond 9 C). */
 int gbdic_nn_im2col(const gbdic_nn_conv_shape *shape, const void *x, void *a, void *stream);
 /* Inference form of the 2-channel input layer (Cout 32): the 3x3 stride-2

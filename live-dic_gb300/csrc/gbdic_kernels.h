@@ -235,9 +235,27 @@ struct TcGemmArgs {
     // gradient `a` (rows B*H*W, K = 9 Cout).  k_split 1.
     int gather;
     NnConvShape conv;
+    // ReLU backward in the epilogue: D is zeroed where `mask` (BF16, D's rows and
+    // stride) is not positive, and column_partial[n][M / 128] receives its FP32
+    // column sums per tile of 128 rows.
+    const void *mask;
+    float *column_partial;
+    int ring;  // stages, set by the launcher
 };
 int tc_gemm_tile_n(int N);
 cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t stream);
+// Weight gradient partials [split][Kp][Cout] of a convolution from its input x
+// (NHWC BF16, C % 8 == 0; for fewer channels the im2col matrix of Kp = 64
+// columns) and dz (B*OH*OW x Cout BF16).
+struct TcWgradArgs {
+    NnConvShape conv;
+    const void *x, *dz;
+    float *partial;
+    int splits, k_rows;  // k_rows = Kp
+    int *error;
+};
+cudaError_t launch_tc_wgrad(const TcWgradArgs &a, cudaStream_t stream);
+cudaError_t launch_nn_bias_reduce(const float *partial, int tiles, int C, float *db, cudaStream_t s);
 
 struct NnPatchArgs {
     const uint8_t *const *refs;   // device array of device image pointers

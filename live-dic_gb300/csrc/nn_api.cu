@@ -61,6 +61,37 @@ int gbdic_nn_conv_gemm(const gbdic_nn_gemm_desc *d, int32_t mode, const gbdic_nn
               "implicit convolution GEMM (rows and K of the convolution, C or Cout % 8, k_split 1 for mode 2)");
 }
 
+int gbdic_nn_conv_dgrad_relu(const gbdic_nn_gemm_desc *d, const gbdic_nn_conv_shape *s, const void *y, float *partial,
+                             float *db, int32_t *device_error, void *stream) {
+    if (!d || !valid_shape(s) || !y || !partial || !db) return invalid("data-gradient arguments are incomplete");
+    if (!d->d_bf16 || d->d_f32 || d->bias || d->relu || d->accumulate)
+        return invalid("the ReLU-masked data gradient is written as BF16 only");
+    gbdic::TcGemmArgs a{};
+    a.a = d->a; a.b = d->b;
+    a.M = d->M; a.N = d->N; a.K = d->K; a.k_split = d->k_split;
+    a.d_bf16 = d->d_bf16; a.ldd = d->ldd;
+    a.error = device_error;
+    a.gather = gbdic::kGatherDgrad;
+    a.conv = shape_of(s);
+    a.mask = y;
+    a.column_partial = partial;
+    const int code = rc(gbdic::launch_tc_gemm(a, as_stream(stream)),
+                        "ReLU-masked data gradient (rows and K of the convolution, Cout % 8, ldd % 8, k_split 1)");
+    if (code != GBDIC_OK) return code;
+    return rc(gbdic::launch_nn_bias_reduce(partial, d->M / 128, d->N, db, as_stream(stream)), "bias gradient");
+}
+
+int gbdic_nn_conv_wgrad(const gbdic_nn_conv_shape *s, const void *x, const void *dz, int32_t splits, float *partial,
+                        float *dw, int32_t *device_error, void *stream) {
+    if (!valid_shape(s) || !x || !dz || !partial || !dw) return invalid("weight-gradient arguments are incomplete");
+    gbdic::TcWgradArgs a{shape_of(s), x, dz, partial, splits, s->Kp, device_error};
+    const int code = rc(gbdic::launch_tc_wgrad(a, as_stream(stream)),
+                        "weight gradient (C % 8 and Cout % 64, or Kp 64 and Cout 32; B*OH*OW % (64 splits), aligned)");
+    if (code != GBDIC_OK) return code;
+    return rc(gbdic::launch_nn_splitk_reduce(partial, splits, s->Kp, s->Cout, s->Kp, dw, as_stream(stream)),
+              "split-K reduction");
+}
+
 int gbdic_nn_patches(const uint8_t *const *refs, const uint8_t *const *tgts, const int32_t *image_index,
                      const float *centres, int32_t count, int32_t width, int32_t height, void *out,
                      const float *shift, int32_t shift_ld, float shift_scale, void *stream) {

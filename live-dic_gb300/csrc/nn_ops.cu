@@ -397,14 +397,14 @@ __global__ void splitk_reduce_kernel(const float *partial, int splits, int Kp_ro
     const float *p = partial + (size_t)k * N + n;
     float acc = 0.0f;
     int s = 0;
-    for (; s + 4 <= splits; s += 4) {
-        const float v0 = __ldg(p + s * stride), v1 = __ldg(p + (s + 1) * stride);
-        const float v2 = __ldg(p + (s + 2) * stride), v3 = __ldg(p + (s + 3) * stride);
-        acc += v0;
-        acc += v1;
-        acc += v2;
-        acc += v3;
+    for (; s + 32 <= splits; s += 32) {  // loads in flight together, added in split order
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = __ldg(p + (s + j) * stride);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc += v[j];
     }
+#pragma unroll 4
     for (; s < splits; ++s) acc += __ldg(p + s * stride);
     out[(size_t)n * Kp + k] = acc;
 }
@@ -455,21 +455,23 @@ __global__ void pack_weights_kernel(const float *w, int Cout, int Cin, int Kp, _
 }
 
 // Loss 0.5 / B sum (pred - target)^2 over the first `outputs` columns and
-// its gradient (pred - target) / B as BF16 [B][ldg] (zero elsewhere); one CTA.
+// its gradient (pred - target) / B as BF16 [B][ldg] (zero elsewhere); the first CTA takes the
+// loss (batch 512: 23 us with one CTA for both).
 __global__ void __launch_bounds__(1024) regression_loss_kernel(const float *pred, int ldp, const float *target,
                                                                int outputs, int B, __nv_bfloat16 *grad,
                                                                float *grad_f32, int ldg, float *loss) {
-    float acc = 0.0f;
-    for (int i = threadIdx.x; i < B * ldg; i += 1024) {
+    const int i = blockIdx.x * 1024 + threadIdx.x;
+    if (i < B * ldg) {
         const int b = i / ldg, j = i % ldg;
-        float g = 0.0f;
-        if (j < outputs) {
-            const float d = pred[(size_t)b * ldp + j] - target[(size_t)b * outputs + j];
-            acc += 0.5f * d * d;
-            g = d / (float)B;
-        }
+        const float g = j < outputs ? (pred[(size_t)b * ldp + j] - target[(size_t)b * outputs + j]) / (float)B : 0.0f;
         grad[i] = __float2bfloat16(g);
         if (grad_f32) grad_f32[i] = g;
+    }
+    if (blockIdx.x != 0) return;
+    float acc = 0.0f;
+    for (int k = threadIdx.x; k < B * outputs; k += 1024) {
+        const float d = pred[(size_t)(k / outputs) * ldp + k % outputs] - target[k];
+        acc += 0.5f * d * d;
     }
     __shared__ float red[1024];
     red[threadIdx.x] = acc;
@@ -904,6 +906,11 @@ cudaError_t launch_nn_relu_bias_backward(const float *dy, int ld, const void *y,
     return cudaGetLastError();
 }
 
+cudaError_t launch_nn_bias_reduce(const float *partial, int tiles, int C, float *db, cudaStream_t s) {
+    bias_reduce_kernel<<<C, 256, 0, s>>>(partial, tiles, db);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_nn_splitk_bias_relu(const float *partial, int splits, long long rows, int N, long long split_stride,
                                       const float *bias, int relu, void *y, cudaStream_t s) {
     if (!partial || !y || splits < 1 || rows <= 0 || N <= 0 || N % 4 || split_stride < rows * N ||
@@ -957,7 +964,7 @@ cudaError_t launch_nn_pack_weights(const float *w, int Cout, int Cin, int Kp, vo
 
 cudaError_t launch_nn_regression_loss(const float *pred, int ldp, const float *target, int outputs, int B, void *grad,
                                       float *grad_f32, int ldg, float *loss, cudaStream_t s) {
-    regression_loss_kernel<<<1, 1024, 0, s>>>(pred, ldp, target, outputs, B, static_cast<__nv_bfloat16 *>(grad),
+    regression_loss_kernel<<<blocks((long long)B * ldg, 1024), 1024, 0, s>>>(pred, ldp, target, outputs, B, static_cast<__nv_bfloat16 *>(grad),
                                              grad_f32, ldg, loss);
     return cudaGetLastError();
 }

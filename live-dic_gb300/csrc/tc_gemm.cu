@@ -21,16 +21,15 @@
 // straight from the NHWC tensor (an im2col row of the forward, or the
 // data-gradient gather of the output gradient; zero-filled outside the
 // image), at the positions the 128-byte swizzle gives them, from a table of
-// the tile's 128 row origins built once per CTA; each warp arrives on a
-// stage's full barrier once that stage's copies landed and were fenced to
-// the async proxy that tcgen05.mma reads through, while its next stage's
-// copies are in flight; TMA still loads B.  The 9x-expanded im2col matrix is never
+// the tile's 128 row origins built once per CTA; each thread's arrival on the
+// stage's full barrier follows its copies, and the MMA issuer fences them to
+// the async proxy that tcgen05.mma reads through; TMA still loads B.  The 9x-expanded im2col matrix is never
 // written or read.  The data-gradient GEMM orders its rows by the input
 // pixel's stride-2 parity class and skips the K blocks of the taps that are
 // zero for the tile's class (9 of the 36 class-tap pairs remain).  The
-// ring has min(4, K blocks) stages (2 in gather mode, where the copies, not
-// the ring, set the pace), so short K loops and gathering CTAs need little
-// shared memory and more CTAs stay resident.
+// ring has min(4, K blocks) stages (2 to 4 in gather mode, as many as leave
+// every CTA of the launch resident), so short K loops and launches of many
+// gathering CTAs need little shared memory.
 // Every mbarrier wait is bounded: on expiry the CTA records an error code and
 // carries on, so a fault of the pipeline ends the kernel instead of hanging.
 // Before a failed CTA frees its tensor memory and exits, it waits (bounded
@@ -50,25 +49,17 @@ namespace {
 #ifndef GBDIC_GEMM_STAGES
 #define GBDIC_GEMM_STAGES 4
 #endif
-#ifndef GBDIC_GATHER_AHEAD
-#define GBDIC_GATHER_AHEAD 1
-#endif
 #ifndef GBDIC_GATHER_WARPS
 #define GBDIC_GATHER_WARPS 8
 #endif
-#ifndef GBDIC_GATHER_STAGES
-#define GBDIC_GATHER_STAGES 2
-#endif
 constexpr int kStages = GBDIC_GEMM_STAGES;
-// Ring depth in gather mode (<= kStages): the gathers keep only a few
-// stages in flight, so a shallower ring leaves room for more resident CTAs.
-constexpr int kGatherStages = GBDIC_GATHER_STAGES;
-static_assert(kGatherStages >= 2 && kGatherStages <= kStages, "gather ring depth");
 // Gather mode: warps 2 .. 2 + kGatherWarps - 1 fill operand A.
 constexpr int kGatherWarps = GBDIC_GATHER_WARPS;
 constexpr int kGatherThreads = 32 * kGatherWarps;
 constexpr int kMaxThreads = 64 + kGatherThreads;
 static_assert(kGatherWarps == 2 || kGatherWarps == 4 || kGatherWarps == 8, "1024 chunks per stage split evenly");
+// Weight gradient: stages of 64 pixels.
+constexpr int kWgradStages = 3;
 constexpr int kBM = 128;
 constexpr int kBK = 64;
 constexpr uint32_t kSpinLimit = 1u << 22;
@@ -103,8 +94,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     return false;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+// Arrives (one of the barrier's expected count) once this thread's cp.async
+// copies so far have landed; the thread goes on.
+__device__ __forceinline__ void mbar_arrive_copies(uint64_t *bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // 16 bytes from global to shared memory; src_bytes 0 writes zeros.
@@ -113,13 +106,16 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, uint3
 }
 
 // Row descriptor of the gathered operand, built once per CTA: the chunk
-// (8-element) offset of the row's pixel origin in the NHWC source and the
-// origin's coordinates.  im2col row m = (b, oy, ox): origin (2 oy - 1,
-// 2 ox - 1) of input image b, tap (ky, kx) reads pixel (y + ky, x + kx).
-// Data-gradient row m = (b, iy, ix): origin (iy + 1, ix + 1), tap (ky, kx)
-// reads output-gradient pixel ((y - ky) / 2, (x - kx) / 2) when both are
-// even and inside the OH x OW grid.  Same mapping as im2col_vec_kernel /
-// dgrad_gather_vec_kernel (nn_ops.cu).
+// (8-element) offset of the row's origin in the NHWC source, and a bit per tap
+// 3 ky + kx whose pixel lies in the tensor (and, for the data gradient, exists).
+// Every tap's pixel is then the origin plus an offset of the tap alone
+// (gather_tap), so a copy costs a bit test and an addition.
+// im2col row m = (b, oy, ox): origin (2 oy - 1, 2 ox - 1) of input image b, tap
+// (ky, kx) reads pixel (y + ky, x + kx).
+// Data-gradient row m = (b, iy, ix): tap (ky, kx) reads output-gradient pixel
+// ((iy + 1 - ky) / 2, (ix + 1 - kx) / 2) when both are whole and inside the
+// OH x OW grid; with whole quotients that is ((iy + 1) >> 1) - (ky >> 1), likewise
+// in x.  Same mapping as im2col_vec_kernel / dgrad_gather_vec_kernel (nn_ops.cu).
 //
 // Parity classes (kGatherDgradClasses, even H and W): the rows are ordered
 // by class c = 2 py + px of the input pixel (iy, ix) = (2u + py, 2v + px),
@@ -129,20 +125,45 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void *src, uint3
 // output-gradient pixel (u + dy, v + dx), dy = 1 for (py, ky) = (1, 0), else
 // 0.  The other taps' K blocks are zero for every row of the tile and are
 // skipped: they would add exact zeros to the accumulator.
-__device__ __forceinline__ int4 gather_row(const TcGemmArgs &a, int m) {
+__device__ __forceinline__ int2 gather_row(const TcGemmArgs &a, int m, int cls) {
     const NnConvShape &s = a.conv;
+    int base, mask = 0;
     if (a.gather == kGatherIm2col) {
         const int ox = m % s.OW, t = m / s.OW, oy = t % s.OH, b = t / s.OH;
         const int y = 2 * oy - 1, x = 2 * ox - 1;
-        return make_int4(((b * s.H + y) * s.W + x) * (s.C / 8), y, x, 0);
+        base = ((b * s.H + y) * s.W + x) * (s.C / 8);
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap)
+            mask |= ((unsigned)(y + tap / 3) < (unsigned)s.H && (unsigned)(x + tap % 3) < (unsigned)s.W) << tap;
+        return make_int2(base, mask);
     }
     if (a.gather == kGatherDgradClasses) {
         const int local = m % (s.B * s.OH * s.OW);
         const int v = local % s.OW, t = local / s.OW, u = t % s.OH, b = t / s.OH;
-        return make_int4(((b * s.OH + u) * s.OW + v) * (s.Cout / 8), u, v, 0);
+        base = ((b * s.OH + u) * s.OW + v) * (s.Cout / 8);
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap)
+            mask |= (u + ((cls >> 1) && tap / 3 == 0) < s.OH && v + ((cls & 1) && tap % 3 == 0) < s.OW) << tap;
+        return make_int2(base, mask);
     }
     const int ix = m % s.W, t = m / s.W, iy = t % s.H, b = t / s.H;
-    return make_int4(b * s.OH * s.OW * (s.Cout / 8), iy + 1, ix + 1, 0);
+    base = ((b * s.OH + ((iy + 1) >> 1)) * s.OW + ((ix + 1) >> 1)) * (s.Cout / 8);
+#pragma unroll
+    for (int tap = 0; tap < 9; ++tap) {
+        const int ty = iy + 1 - tap / 3, tx = ix + 1 - tap % 3;
+        mask |= (!((ty | tx) & 1) && (unsigned)ty < (unsigned)(2 * s.OH) && (unsigned)tx < (unsigned)(2 * s.OW)) << tap;
+    }
+    return make_int2(base, mask);
+}
+
+// Chunk offset of tap (ky, kx) from a row's origin.
+__device__ __forceinline__ int gather_tap(const TcGemmArgs &a, int ky, int kx, int cls) {
+    const NnConvShape &s = a.conv;
+    if (a.gather == kGatherIm2col) return (ky * s.W + kx) * (s.C / 8);
+    const int cell = a.gather == kGatherDgradClasses
+                         ? ((cls >> 1) && ky == 0 ? s.OW : 0) + ((cls & 1) && kx == 0 ? 1 : 0)
+                         : -((ky >> 1) * s.OW + (kx >> 1));
+    return cell * (s.Cout / 8);
 }
 
 // Parity class of the tile starting at row m0 (class mode), else 0.
@@ -164,40 +185,6 @@ __device__ __forceinline__ int kblock_offset(const TcGemmArgs &a, int kb, int k_
     const int nx = (cls & 1) ? 2 : 1, ty = t / nx, tx = t - ty * nx;
     const int ky = (cls >> 1) ? 2 * ty : 1, kx = (cls & 1) ? 2 * tx : 1;
     return (ky * 3 + kx) * a.conv.Cout + within * kBK;
-}
-
-// Tap of the chunk starting at K element k0: C (Cout) % 8 == 0, so a chunk
-// never straddles two taps.  im2col: (ky, kx, the tap's chunk offset, 0 for
-// the K padding beyond 9 C); data gradient: (ky, kx, channel chunk, 1);
-// class mode: (dy, dx, chunk offset of pixel (dy, dx) and channel, 1).
-__device__ __forceinline__ int4 gather_tap(const TcGemmArgs &a, int k0, int cls) {
-    const NnConvShape &s = a.conv;
-    const int per_tap = (a.gather == kGatherIm2col ? s.C : s.Cout) / 8;
-    const int q = k0 / 8, tap = q / per_tap, c8 = q - tap * per_tap, ky = tap / 3, kx = tap - 3 * ky;
-    if (a.gather == kGatherIm2col) return make_int4(ky, kx, (ky * s.W + kx) * per_tap + c8, tap < 9 ? 1 : 0);
-    if (a.gather == kGatherDgradClasses) {
-        const int dy = ((cls >> 1) && ky == 0) ? 1 : 0, dx = ((cls & 1) && kx == 0) ? 1 : 0;
-        return make_int4(dy, dx, (dy * s.OW + dx) * per_tap + c8, 1);
-    }
-    return make_int4(ky, kx, c8, 1);
-}
-
-// Source chunk of (row, tap), or nullptr where the operand is zero.
-__device__ __forceinline__ const uint4 *gather_src(const TcGemmArgs &a, int4 row, int4 tap) {
-    const NnConvShape &s = a.conv;
-    const uint4 *src = static_cast<const uint4 *>(a.a);
-    if (a.gather == kGatherIm2col) {
-        const int yy = row.y + tap.x, xx = row.z + tap.y;
-        if (!tap.w || (unsigned)yy >= (unsigned)s.H || (unsigned)xx >= (unsigned)s.W) return nullptr;
-        return src + (row.x + tap.z);
-    }
-    if (a.gather == kGatherDgradClasses) {
-        if (row.y + tap.x >= s.OH || row.z + tap.y >= s.OW) return nullptr;
-        return src + (row.x + tap.z);
-    }
-    const int ty = row.y - tap.x, tx = row.z - tap.y;
-    if (((ty | tx) & 1) || (unsigned)ty >= (unsigned)(2 * s.OH) || (unsigned)tx >= (unsigned)(2 * s.OW)) return nullptr;
-    return src + (row.x + ((ty >> 1) * s.OW + (tx >> 1)) * (s.Cout / 8) + tap.z);
 }
 
 // Output row of accumulator row m (class mode: back to (b, iy, ix) order).
@@ -235,8 +222,10 @@ __host__ __device__ constexpr uint32_t instr_desc(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// The bound on registers lets as many CTAs be resident as a ring of two stages
+// leaves room for.
 template <int BN>
-__global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
+__global__ void __launch_bounds__(kMaxThreads, BN <= 64 ? 4 : 3) tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
                                                          const __grid_constant__ CUtensorMap map_b,
                                                          TcGemmArgs args) {
     constexpr uint32_t kBytesA = kBM * kBK * 2;
@@ -248,7 +237,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
     __shared__ int issued_kb, consumed_kb;  // K blocks whose loads were issued / consumed
-    __shared__ int4 row_tab[kBM];           // gather mode: descriptors of the tile's rows
+    __shared__ int2 row_tab[kBM];           // gather mode: descriptors of the tile's rows
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -260,14 +249,13 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
     // The ring holds min(4, K blocks) stages (launch_bn sizes the dynamic
     // shared memory the same way), so short K loops leave room for more
     // resident CTAs.
-    const int ring = args.gather ? kGatherStages : kStages;
-    const int nst = num_kb < ring ? num_kb : ring;
+    const int nst = num_kb < args.ring ? num_kb : args.ring;
 
-    if (args.gather && tid < kBM) row_tab[tid] = gather_row(args, m0 + tid);
+    if (args.gather && tid < kBM) row_tab[tid] = gather_row(args, m0 + tid, cls);
     if (tid == 0) {
         // Full barriers: the TMA producer's arrive (with the stage's bytes),
-        // plus one arrive per gathering warp in gather mode.
-        const uint32_t full_count = args.gather ? 1u + (uint32_t)kGatherWarps : 1u;
+        // plus one arrive per gathering thread in gather mode.
+        const uint32_t full_count = args.gather ? 1u + (uint32_t)kGatherThreads : 1u;
         for (int s = 0; s < nst; ++s) {
             mbar_init(&full_bar[s], full_count);
             mbar_init(&empty_bar[s], 1);
@@ -315,6 +303,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
                 atomicExch(&failed, 1);
                 break;
             }
+            // gathered bytes (generic proxy) before the MMA's reads (async proxy)
+            if (args.gather) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
             const uint32_t b_addr = a_addr + kBytesA;
@@ -345,29 +335,34 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
         // tap, or two for C = 32).
         // Row r, chunk j lands at byte r * 128 + ((j ^ (r % 8)) * 16) of the
         // 1024-byte-aligned stage, the 128-byte swizzle of the TMA loads it
-        // replaces.  Each stage's copies form one cp.async group; a warp
-        // keeps up to kAhead groups in flight.  At the top of each iteration
-        // the oldest group is waited for, fenced to the async proxy that
-        // tcgen05.mma reads through and arrived on its full barrier, before
-        // the warp waits for the next ring slot, so the slot's release (by
-        // the MMAs of a stage arrived kAhead iterations earlier) is never
-        // held up by the warp's own arrivals.
-        // kAhead <= ring depth: the slot waited for at iteration kb belongs to
-        // stage kb - nst, arrived at the top of iteration kb - nst + kAhead <= kb.
-        constexpr int kAhead = GBDIC_GATHER_AHEAD;
-        static_assert(kAhead >= 1 && kAhead <= kGatherStages, "gather look-ahead must stay within the ring");
+        // replaces.  Each thread's arrival on the stage's full barrier is left
+        // to its copies, so the ring alone limits how far the gathering runs
+        // ahead.  (Waiting for each stage's copies and fencing them here, warp
+        // by warp, cost 1 us a K block whatever the ring's depth: the fence
+        // waits for the later stages' copies too.)
         constexpr int kRowStep = kGatherThreads / 8, kRowsPerThread = kBM / kRowStep;
         const int g = tid - 64, j = g & 7, r0 = g >> 3;
-        int kb = 0, arrived = 0;
-        for (; kb < num_kb; ++kb) {
+        const uint4 *src = static_cast<const uint4 *>(args.a);
+        int base[kRowsPerThread], mask[kRowsPerThread];
+#pragma unroll
+        for (int i = 0; i < kRowsPerThread; ++i) {
+            const int2 row = row_tab[r0 + kRowStep * i];
+            base[i] = row.x;
+            mask[i] = row.y;
+        }
+        const uint32_t place = (uint32_t)(r0 * 128 + ((j ^ (r0 & 7)) << 4));  // rows step by multiples of 8
+        static_assert(kRowStep % 8 == 0, "a thread's rows share their swizzle phase");
+        // The chunk's tap and its chunk within the tap, advanced by 8 chunks a K
+        // block (class mode: over the class's taps).
+        const bool classes = args.gather == kGatherDgradClasses;
+        const int per_tap = (args.gather == kGatherIm2col ? args.conv.C : args.conv.Cout) / 8;
+        const int q = kblock_offset(args, 0, k_begin, cls) / 8 + j;
+        const int kx_first = classes && !(cls & 1) ? 1 : 0, kx_step = classes ? 2 : 1;
+        const int ky_step = classes && (cls >> 1) ? 2 : 1;
+        int tap = q / per_tap, c8 = q - tap * per_tap, ky = tap / 3, kx = tap - 3 * ky;
+        int delta = gather_tap(args, ky, kx, cls);
+        for (int kb = 0; kb < num_kb; ++kb) {
             const int s = kb % nst;
-            if (kb - arrived == kAhead) {
-                asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&full_bar[arrived % nst]);
-                ++arrived;
-            }
             if (kb >= nst) {
                 int ok = 1;
                 if (lane == 0) ok = mbar_wait(&empty_bar[s], ((kb / nst) - 1) & 1) ? 1 : 0;
@@ -377,31 +372,46 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
                     break;
                 }
             }
-            const uint32_t sa = smem_u32(smem + s * kStageBytes);
-            const int4 tap = gather_tap(args, kblock_offset(args, kb, k_begin, cls) + 8 * j, cls);
+            const uint32_t dst = smem_u32(smem + s * kStageBytes) + place;
+            const int offset = delta + c8, bit = 3 * ky + kx;  // beyond the ninth tap (K padding): no bit is set
 #pragma unroll
             for (int i = 0; i < kRowsPerThread; ++i) {
-                const int r = r0 + kRowStep * i;
-                const uint4 *src = gather_src(args, row_tab[r], tap);
-                cp_async_16(sa + (uint32_t)(r * 128 + ((j ^ (r & 7)) << 4)), src ? src : args.a, src ? 16u : 0u);
+                const bool in = (mask[i] >> bit) & 1;
+                cp_async_16(dst + (uint32_t)(kRowStep * i * 128), src + (in ? base[i] + offset : 0), in ? 16u : 0u);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
+            mbar_arrive_copies(&full_bar[s]);
+            c8 += 8;
+            if (c8 >= per_tap) {
+                do {
+                    c8 -= per_tap;
+                    kx += kx_step;
+                    if (kx > 2) {
+                        kx = kx_first;
+                        ky += ky_step;
+                    }
+                } while (c8 >= per_tap);
+                delta = gather_tap(args, ky, kx, cls);
+            }
         }
         // Drain: every issued copy lands before the warp moves on (also after
         // a failed wait, so no copy is left writing into shared memory).
         asm volatile("cp.async.wait_all;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        for (; arrived < kb; ++arrived)
-            if (lane == 0) mbar_arrive(&full_bar[arrived % nst]);
     }
     __syncwarp();
+    // Epilogue: warp w < 4 owns accumulator lanes (rows) 32w .. 32w + 31.
+    __shared__ float column_sum[4][BN];
+    const int row = output_row(args, m0 + warp * 32 + lane, cls);
+    if (args.mask != nullptr && warp < 4) {
+        // the row's activations, on their way while the last MMAs finish
+        const char *m = reinterpret_cast<const char *>(static_cast<const __nv_bfloat16 *>(args.mask) +
+                                                       (size_t)row * args.ldd + n0);
+#pragma unroll
+        for (int b = 0; b < 2 * BN; b += 64) asm volatile("prefetch.global.L1 [%0];" ::"l"(m + b));
+    }
     if (!mbar_wait(&done_bar, 0)) atomicExch(&failed, 1);
     __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
-    // Epilogue: warp w < 4 owns accumulator lanes (rows) 32w .. 32w + 31.
-    const int row = output_row(args, m0 + warp * 32 + lane, cls);
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
 #pragma unroll 1
     for (int c = 0; c < (warp < 4 ? BN : 0); c += 16) {
@@ -419,6 +429,35 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
             v[j] = __uint_as_float(r[j]);
             if (args.bias) v[j] = v[j] + args.bias[n0 + c + j];
             if (args.relu) v[j] = fmaxf(v[j], 0.0f);
+        }
+        if (args.mask != nullptr) {
+            // ReLU backward where the row's activation is zero, and the sums
+            // over the warp's 32 rows: halves of the columns go to halves of
+            // the lanes, until lane pair l holds column l / 2.
+            const uint4 *m = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(args.mask) +
+                                                             (size_t)row * args.ldd + n0 + c);
+            const uint4 m0 = __ldg(m), m1 = __ldg(m + 1);
+            const uint32_t words[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __nv_bfloat162 y = *reinterpret_cast<const __nv_bfloat162 *>(&words[j]);
+                if (!(__bfloat162float(y.x) > 0.0f)) v[2 * j] = 0.0f;
+                if (!(__bfloat162float(y.y) > 0.0f)) v[2 * j + 1] = 0.0f;
+            }
+            float t[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) t[j] = v[j];
+#pragma unroll
+            for (int half = 8; half >= 1; half >>= 1) {
+                const bool upper = lane & (2 * half);
+#pragma unroll
+                for (int j = 0; j < half; ++j) {
+                    const float keep = upper ? t[j + half] : t[j], send = upper ? t[j] : t[j + half];
+                    t[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
+                }
+            }
+            t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
+            if ((lane & 1) == 0) column_sum[warp][c + (lane >> 1)] = t[0];
         }
         const size_t base = (size_t)blockIdx.z * (size_t)args.split_stride + (size_t)row * args.ldd + n0 + c;
         if (args.d_f32) {
@@ -441,6 +480,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (args.mask != nullptr)
+        for (int c = tid; c < BN; c += blockDim.x)
+            args.column_partial[(size_t)(n0 + c) * gridDim.y + blockIdx.y] =
+                (column_sum[0][c] + column_sum[1][c]) + (column_sum[2][c] + column_sum[3][c]);
     if (warp == 0) {
         if (lane == 0 && failed) {
             // The producer runs at most kStages K blocks ahead of the issuer,
@@ -451,6 +494,207 @@ __global__ void __launch_bounds__(kMaxThreads, 1) tc_gemm_kernel(const __grid_co
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+    }
+    if (tid == 0 && failed && args.error) atomicExch(args.error, 1);
+}
+
+// ------------------------------------------------------- weight gradient
+// dW^T[k][co] = sum_m A[m][k] dZ[m][co] over the output pixels m, A the im2col
+// rows of the layer's input.  The reduction runs over the rows of both
+// operands, so both are taken MN-major (a pixel's channels contiguous, as they
+// lie in memory): neither A^T nor dZ^T is ever written.  What it replaced, the
+// transposed im2col matrix of every layer and a K-major GEMM over it, moved 9 x
+// the activations twice: batch 512, five layers, 109 us + 97 us, where this takes
+// 84.
+//
+// One CTA per 128 k x BN co tile and split of m, 64 pixels to a stage: dZ by TMA
+// (64-channel boxes, 128-byte swizzle; one 32-channel box, 64-byte swizzle, for
+// the first layer), A gathered by eight warps with 16-byte copies to the places
+// the 128-byte swizzle gives them (row r of a 64-channel group at 128 r, chunk j
+// at (j ^ r % 8) 16), or, where a pixel's channels are fewer than a chunk (the
+// two-channel input layer), by TMA from the forward's im2col matrix of 64
+// columns.  Then the accumulator's rows 64 and up repeat the first 64 (both
+// groups of the descriptor are the one tile) and are not written.
+// Shared-memory matrix descriptor, MN-major: groups of 64 (32) channels `lead`
+// bytes apart, groups of 8 pixels `stride` bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t lead, uint32_t stride, uint64_t swizzle) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | (uint64_t)((lead >> 4) & 0x3FFFu) << 16 |
+           (uint64_t)((stride >> 4) & 0x3FFFu) << 32 | (uint64_t)1u << 46 | swizzle << 61;
+}
+
+template <int BN, bool GATHER>
+__global__ void __launch_bounds__(GATHER ? kMaxThreads : 128, 1)
+    tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    TcWgradArgs args) {
+    constexpr int kPixels = 64;
+    constexpr uint32_t kBytesA = (GATHER ? 2 : 1) * kPixels * 128;
+    constexpr uint32_t kBytesB = BN * kPixels * 2;
+    constexpr uint32_t kStageBytes = kBytesA + kBytesB;
+    constexpr int kRing = kWgradStages;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t full_bar[kRing], empty_bar[kRing], done_bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int failed;
+    __shared__ int issued_kb, consumed_kb;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const NnConvShape &s = args.conv;
+    const int n0 = blockIdx.x * BN, k0 = blockIdx.y * kBM;
+    const int pixels = s.B * s.OH * s.OW / args.splits, m_begin = blockIdx.z * pixels, num_kb = pixels / kPixels;
+
+    if (tid == 0) {
+        for (int i = 0; i < kRing; ++i) {
+            mbar_init(&full_bar[i], GATHER ? 1u + (uint32_t)kGatherThreads : 1u);
+            mbar_init(&empty_bar[i], 1);
+        }
+        mbar_init(&done_bar, 1);
+        failed = 0;
+        issued_kb = 0;
+        consumed_kb = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"((uint32_t)BN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 0 && lane == 0) {
+        int kb = 0;
+        for (; kb < num_kb; ++kb) {
+            const int st = kb % kRing;
+            if (kb >= kRing && !mbar_wait(&empty_bar[st], ((kb / kRing) - 1) & 1)) {
+                atomicExch(&failed, 1);
+                break;
+            }
+            uint8_t *sa = smem + st * kStageBytes, *sb = sa + kBytesA;
+            mbar_expect_tx(&full_bar[st], GATHER ? kBytesB : kStageBytes);
+            const int m = m_begin + kb * kPixels;
+            if (!GATHER) tma_load_2d(sa, &map_a, &full_bar[st], 0, m);
+#pragma unroll
+            for (int g = 0; g < (BN + 63) / 64; ++g)
+                tma_load_2d(sb + g * kPixels * 128, &map_b, &full_bar[st], n0 + 64 * g, m);
+        }
+        issued_kb = kb;
+    } else if (warp == 1 && lane == 0) {
+        // kind::f16, FP32 accumulator, BF16 operands, both MN-major (bits 15, 16).
+        constexpr uint32_t idesc = instr_desc(kBM, BN) | (1u << 15) | (1u << 16);
+        constexpr uint32_t kRowB = BN < 64 ? 2 * BN : 128;  // bytes of a pixel in a group of B
+        int kb = 0;
+        for (; kb < num_kb; ++kb) {
+            const int st = kb % kRing;
+            if (!mbar_wait(&full_bar[st], (kb / kRing) & 1)) {
+                atomicExch(&failed, 1);
+                break;
+            }
+            if (GATHER) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_addr = smem_u32(smem + st * kStageBytes), b_addr = a_addr + kBytesA;
+#pragma unroll
+            for (int kk = 0; kk < kPixels / 16; ++kk) {
+                const uint64_t da = smem_desc_mn(a_addr + kk * 16 * 128, GATHER ? kPixels * 128 : 0, 1024, 2);
+                const uint64_t db = smem_desc_mn(b_addr + kk * 16 * kRowB, kPixels * kRowB, 8 * kRowB, BN < 64 ? 4 : 2);
+                const uint32_t accumulate = (kb > 0 || kk > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+                    "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             smem_u32(&empty_bar[st]))
+                         : "memory");
+        }
+        consumed_kb = kb;
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                         smem_u32(&done_bar))
+                     : "memory");
+    }
+    if (GATHER && warp >= 2) {
+        // Thread g copies chunk g % 16 (one tap's eight channels, the same for
+        // every pixel) of pixels g / 16 + 16 i; the pixels advance by 64 a stage.
+        constexpr int kRows = kPixels * 16 / kGatherThreads, kStep = kGatherThreads / 16;
+        const int g = tid - 64, chunk = g & 15, r0 = g >> 4, j = chunk & 7;
+        const int per_tap = s.C / 8, q = k0 / 8 + chunk, tap = q / per_tap, c8 = q - tap * per_tap;
+        const int ky = tap / 3, kx = tap - 3 * ky;
+        const bool used = tap < 9;
+        const uint4 *x = static_cast<const uint4 *>(args.x);
+        int ox[kRows], oy[kRows], b[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const int m = m_begin + r0 + kStep * i, t = m / s.OW;
+            ox[i] = m - t * s.OW;
+            b[i] = t / s.OH;
+            oy[i] = t - b[i] * s.OH;
+        }
+        const int dx = kPixels % s.OW, dt = kPixels / s.OW, dy = dt % s.OH, dbatch = dt / s.OH;
+        for (int kb = 0; kb < num_kb; ++kb) {
+            const int st = kb % kRing;
+            if (kb >= kRing) {
+                int ok = 1;
+                if (lane == 0) ok = mbar_wait(&empty_bar[st], ((kb / kRing) - 1) & 1) ? 1 : 0;
+                ok = __shfl_sync(0xffffffffu, ok, 0);
+                if (!ok) {
+                    if (lane == 0) atomicExch(&failed, 1);
+                    break;
+                }
+            }
+            const uint32_t sa = smem_u32(smem + st * kStageBytes) + (uint32_t)((chunk >> 3) * kPixels * 128);
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const int r = r0 + kStep * i, yy = 2 * oy[i] - 1 + ky, xx = 2 * ox[i] - 1 + kx;
+                const bool in = used && (unsigned)yy < (unsigned)s.H && (unsigned)xx < (unsigned)s.W;
+                const uint4 *src = in ? x + ((b[i] * s.H + yy) * s.W + xx) * per_tap + c8 : x;
+                cp_async_16(sa + (uint32_t)(r * 128 + ((j ^ (r & 7)) << 4)), src, in ? 16u : 0u);
+                ox[i] += dx;
+                oy[i] += dy;
+                b[i] += dbatch;
+                if (ox[i] >= s.OW) { ox[i] -= s.OW; ++oy[i]; }
+                if (oy[i] >= s.OH) { oy[i] -= s.OH; ++b[i]; }
+            }
+            mbar_arrive_copies(&full_bar[st]);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    __syncwarp();
+    if (!mbar_wait(&done_bar, 0)) atomicExch(&failed, 1);
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+    const int row = warp * 32 + lane;
+#pragma unroll 1
+    for (int c = 0; c < (warp < 4 ? BN : 0); c += 16) {
+        uint32_t r[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (k0 + row >= args.k_rows) continue;
+        float4 *o = reinterpret_cast<float4 *>(args.partial + ((size_t)blockIdx.z * args.k_rows + k0 + row) * s.Cout +
+                                               n0 + c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            o[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                               __uint_as_float(r[4 * j + 3]));
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        if (lane == 0 && failed) {
+            for (int kb = consumed_kb; kb < issued_kb; ++kb) mbar_wait(&full_bar[kb % kRing], (kb / kRing) & 1);
+            mbar_wait(&done_bar, 0);
+        }
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)BN));
     }
     if (tid == 0 && failed && args.error) atomicExch(args.error, 1);
 }
@@ -472,24 +716,42 @@ EncodeTiled encode_fn() {
     return fn;
 }
 
-// 2-D BF16 row-major matrix rows x cols (cols contiguous), box box_rows x 64.
-bool make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int box_rows) {
+// 2-D BF16 row-major matrix rows x cols (cols contiguous), box box_rows x 64
+// (128-byte swizzle), or x 32 (64-byte swizzle).
+bool make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int box_rows, int box_cols = kBK) {
     EncodeTiled fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t estride[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(ptr), dims, strides, box, estride,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Stages of the gathering ring.  A launch with more CTAs than fit at once hides
+// the copies' latency behind other CTAs, and a ring of two stages lets the most
+// of them be resident; one with fewer takes the deepest ring that still leaves
+// every CTA resident.  Batch 512, 16 CTAs of 18 K blocks (128 -> 64 channels at
+// 2 x 2): 26 us with two stages and a wait per stage, 20 with four and the
+// arrivals left to the copies, 15 with the taps stepped instead of divided out;
+// 64 CTAs of 18 (128 -> 128 at 4 x 4): 29 -> 24 -> 18.
+int gather_ring(long long ctas, size_t stage_bytes) {
+    const long long per_sm = (ctas + 151) / 152;
+    for (int ring = kStages; ring > 2; --ring)
+        if (per_sm * (long long)(ring * stage_bytes + 8192) <= 224 * 1024) return ring;
+    return 2;
+}
+
 template <int BN>
-cudaError_t launch_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemmArgs &a, cudaStream_t stream) {
+cudaError_t launch_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemmArgs &args, cudaStream_t stream) {
+    TcGemmArgs a = args;
+    const long long ctas = (long long)(a.N / BN) * (a.M / kBM) * a.k_split;
+    a.ring = a.gather ? gather_ring(ctas, kBM * kBK * 2 + BN * kBK * 2) : kStages;
     const int num_kb = a.K / a.k_split / kBK;
-    const int ring = a.gather ? kGatherStages : kStages;
-    const int nst = num_kb < ring ? num_kb : ring;
+    const int nst = num_kb < a.ring ? num_kb : a.ring;
     const size_t smem = (size_t)nst * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
     const size_t smem_max = (size_t)kStages * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
     // The attribute is per device; set it once per device and tile width.
@@ -507,7 +769,51 @@ cudaError_t launch_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemm
     return cudaGetLastError();
 }
 
+template <int BN, bool GATHER>
+cudaError_t launch_wgrad(const CUtensorMap &ma, const CUtensorMap &mb, const TcWgradArgs &a, cudaStream_t stream) {
+    const size_t smem = (size_t)kWgradStages * ((GATHER ? 2 : 1) * 64 * 128 + BN * 128) + 1024;
+    static thread_local int configured_device = -1;
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    if (configured_device != device) {
+        err = cudaFuncSetAttribute(tc_wgrad_kernel<BN, GATHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (err != cudaSuccess) return err;
+        configured_device = device;
+    }
+    const dim3 grid(a.conv.Cout / BN, (a.k_rows + kBM - 1) / kBM, a.splits);
+    tc_wgrad_kernel<BN, GATHER><<<grid, GATHER ? kMaxThreads : 128, smem, stream>>>(ma, mb, a);
+    return cudaGetLastError();
+}
+
 }  // namespace
+
+cudaError_t launch_tc_wgrad(const TcWgradArgs &a, cudaStream_t stream) {
+    const NnConvShape &s = a.conv;
+    const long long pixels = (long long)s.B * s.OH * s.OW;
+    const bool gather = s.C % 8 == 0;
+    if (s.B < 1 || s.H < 1 || s.W < 1 || s.OH != (s.H + 1) / 2 || s.OW != (s.W + 1) / 2 || !a.x || !a.dz ||
+        !a.partial || a.splits < 1 || pixels >= (1ll << 31) || pixels % (64ll * a.splits) || s.Kp < 9 * s.C ||
+        a.k_rows != s.Kp)
+        return cudaErrorInvalidValue;
+    if (gather) {
+        // chunk offsets are 32-bit in the kernel
+        if (s.Cout % 64 || (long long)s.B * s.H * s.W * (s.C / 8) >= (1ll << 31)) return cudaErrorInvalidValue;
+    } else if (s.Kp != 64 || s.Cout != 32) {
+        return cudaErrorInvalidValue;
+    }
+    if ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.dz) | reinterpret_cast<uintptr_t>(a.partial)) &
+        15u)
+        return cudaErrorMisalignedAddress;
+    CUtensorMap ma, mb;
+    if (!make_map(&mb, a.dz, (int)pixels, s.Cout, 64, gather ? 64 : 32)) return cudaErrorInvalidValue;
+    if (!gather) {
+        if (!make_map(&ma, a.x, (int)pixels, s.Kp, 64)) return cudaErrorInvalidValue;
+        return launch_wgrad<32, false>(ma, mb, a, stream);
+    }
+    ma = mb;  // not read: A is gathered
+    return s.Cout % 128 == 0 ? launch_wgrad<128, true>(ma, mb, a, stream) : launch_wgrad<64, true>(ma, mb, a, stream);
+}
 
 int tc_gemm_tile_n(int N) {
     if (N % 128 == 0) return 128;
@@ -521,7 +827,8 @@ cudaError_t launch_tc_gemm(const TcGemmArgs &a, cudaStream_t stream) {
     const int bn = tc_gemm_tile_n(a.N);
     if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.k_split < 1 || a.M % kBM != 0 || bn == 0 ||
         a.K % (kBK * a.k_split) != 0 || a.ldd < a.N || a.ldd % 4 != 0 || !a.a || !a.b ||
-        (!a.d_f32 && !a.d_bf16) || (a.accumulate && !a.d_f32) || (a.k_split > 1 && a.bias))
+        (!a.d_f32 && !a.d_bf16) || (a.mask && (!a.column_partial || a.k_split != 1 || a.ldd % 8)) ||
+        (reinterpret_cast<uintptr_t>(a.mask) & 15u) || (a.accumulate && !a.d_f32) || (a.k_split > 1 && a.bias))
         return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(a.a) | reinterpret_cast<uintptr_t>(a.b)) & 15u) return cudaErrorMisalignedAddress;
     if (a.gather != kGatherNone) {

@@ -241,14 +241,12 @@ class SeedNet:
             "doutT": torch.zeros(OUT_PAD, B, dtype=bf16, device=dev),
             "y5T": torch.zeros(self.features, B, dtype=bf16, device=dev),
             "dw6T": torch.zeros(self.features, OUT_PAD, dtype=f32, device=dev),
-            "dy": [torch.zeros(c.M, c.cout, dtype=f32, device=dev) for c in self.convs],
+            "dy": torch.zeros(B, self.features, dtype=f32, device=dev),
             "dz": [torch.zeros(c.M, c.cout, dtype=bf16, device=dev) for c in self.convs],
             "db_partial": [torch.zeros(c.cout * ((c.M + 63) // 64), dtype=f32, device=dev) for c in self.convs],
-            "dzT": [torch.zeros(c.cout, c.M, dtype=bf16, device=dev) for c in self.convs],
-            "aT": [torch.zeros(c.kp_rows, c.M, dtype=bf16, device=dev) for c in self.convs],
         }
         bufs["splits"] = [self._splits(c) for c in self.convs]
-        bufs["partial"] = [torch.zeros(s, c.kp_rows, c.cout, dtype=f32, device=dev)
+        bufs["partial"] = [torch.zeros(s, c.kp, c.cout, dtype=f32, device=dev)
                            for s, c in zip(bufs["splits"], self.convs, strict=True)]
         return bufs
 
@@ -295,27 +293,25 @@ class SeedNet:
         _call(lib, "gbdic_nn_splitk_reduce", _ptr(b["dw6T"]), 1, F, OUT_PAD, F, _ptr(self.grads[2 * nconv]), stream)
         _call(lib, "gbdic_nn_bias_grad", _ptr(b["dout_f32"]), LOSS_PAD, None, B, OUT_PAD,
               _ptr(self.grads[2 * nconv + 1]), stream)
-        self._gemm(b["dout"], self.w6t, B, F, LOSS_PAD, d_f32=b["dy"][-1].view(B, F), stream=stream)
+        self._gemm(b["dout"], self.w6t, B, F, LOSS_PAD, d_f32=b["dy"], stream=stream)
+        last = self.convs[-1]
+        _call(lib, "gbdic_nn_relu_bias_backward", _ptr(b["dy"]), last.cout, _ptr(self.y[-1]), last.M, last.cout,
+              _ptr(b["dz"][-1]), None, _ptr(b["db_partial"][-1]), _ptr(self.grads[2 * nconv - 1]), stream)
         for i in range(nconv - 1, -1, -1):
             c = self.convs[i]
-            dy, dz = b["dy"][i], b["dz"][i]
-            # dZ, its transpose and the bias gradient in one pass over dY
-            _call(lib, "gbdic_nn_relu_bias_backward", _ptr(dy), c.cout, _ptr(self.y[i]), c.M, c.cout, _ptr(dz),
-                  _ptr(b["dzT"][i]), _ptr(b["db_partial"][i]), _ptr(self.grads[nconv + i]), stream)
-            # weight gradient: dW^T[k][co] = sum_m A[m][k] dZ[m][co], with A^T
-            # written straight from the layer input (A is never materialised)
-            x = self.x0 if i == 0 else self.y[i - 1]
-            _call(lib, "gbdic_nn_im2col_t", C.byref(self._shape(i)), _ptr(x), _ptr(b["aT"][i]), c.kp_rows, stream)
-            splits = b["splits"][i]
-            self._gemm(b["aT"][i], b["dzT"][i], c.kp_rows, c.cout, c.M, d_f32=b["partial"][i], k_split=splits,
-                       split_stride=c.kp_rows * c.cout, stream=stream)
-            _call(lib, "gbdic_nn_splitk_reduce", _ptr(b["partial"][i]), splits, c.kp_rows, c.cout, c.kp,
-                  _ptr(self.grads[i]), stream)
+            dz = b["dz"][i]
+            # weight gradient from the layer input and dZ as they lie in memory
+            # (the 2-channel input layer: from the forward's im2col matrix)
+            x = self.a[0] if i == 0 else self.y[i - 1]
+            _call(lib, "gbdic_nn_conv_wgrad", C.byref(self._shape(i)), _ptr(x), _ptr(dz), b["splits"][i],
+                  _ptr(b["partial"][i]), _ptr(self.grads[i]), _ptr(self.err), stream)
             if i > 0:
-                # data gradient: dY_{i-1}[m][ci] = sum_(ky,kx,co) G[m][.] Wt[ci][.],
-                # G gathered from dZ in the kernel (implicit GEMM)
-                self._gemm(dz, self.wt[i], c.Min, c.cin, c.kt, d_f32=b["dy"][i - 1], stream=stream, gather=2,
-                           shape=self._shape(i))
+                # data gradient, gathered from dZ in the kernel (implicit GEMM),
+                # with the layer below's ReLU backward and bias gradient
+                desc = _native.NnGemmDesc(dz.data_ptr(), self.wt[i].data_ptr(), c.Min, c.cin, c.kt, 1, None,
+                                          b["dz"][i - 1].data_ptr(), c.cin, 0, None, 0, 0)
+                _call(lib, "gbdic_nn_conv_dgrad_relu", C.byref(desc), C.byref(self._shape(i)), _ptr(self.y[i - 1]),
+                      _ptr(b["db_partial"][i - 1]), _ptr(self.grads[nconv + i - 1]), _ptr(self.err), stream)
 
     def adam_step(self, lr: float = 1e-3, *, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8,
                   weight_decay: float = 0.0, stream=None) -> None:

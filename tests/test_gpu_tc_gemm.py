@@ -190,3 +190,64 @@ def test_implicit_conv_gemm_rejects_mismatched_shapes():
     shape = _native.NnConvShape(2, 16, 16, 32, 8, 8, 64, 320)
     with pytest.raises(ValueError, match="implicit convolution GEMM"):
         _conv_gemm(x, w, 1, shape, 256, 320, out)   # rows are 2 * 8 * 8 = 128
+
+
+@pytest.mark.parametrize("B,H,Cin,Cout,splits", [(8, 32, 32, 64, 4), (4, 16, 64, 128, 1), (16, 8, 128, 64, 2),
+                                               (2, 32, 16, 192, 8), (128, 7, 8, 64, 8), (64, 5, 24, 128, 3),
+                                               (4, 64, 2, 32, 16), (1, 16, 2, 32, 1)])
+def test_weight_gradient_of_untransposed_operands(B, H, Cin, Cout, splits):
+    """dW from the layer input and dZ as they lie in memory against FP32 products
+    of the im2col matrix: 64-, 128- and 192-channel tiles, ragged last K tile,
+    pixel counts that wrap rows and images within a stage, the two-channel
+    layer's materialised matrix.  BF16 products are exact in FP32; a sum of M
+    of them errs by at most M 2^-24 of the magnitudes' sum."""
+    lib = _native.load()
+    shape, g = _conv_case(B, H, Cin, Cout, B * H + Cin + splits)
+    M = B * shape.OH * shape.OW
+    if M % (64 * splits):
+        pytest.skip("pixels must fill the splits' stages")
+    x = torch.randn(B, H, H, Cin, generator=g, device="cuda").to(torch.bfloat16)
+    dz = torch.randn(M, Cout, generator=g, device="cuda").to(torch.bfloat16)
+    a = torch.empty(M, shape.Kp, dtype=torch.bfloat16, device="cuda")
+    _native.check(lib.gbdic_nn_im2col(C.byref(shape), C.c_void_p(x.data_ptr()), C.c_void_p(a.data_ptr()), None),
+                  lib.gbdic_last_error(None))
+    dw = torch.full((Cout, shape.Kp), 7.0, device="cuda")
+    partial = torch.empty(splits, shape.Kp, Cout, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    source = x if Cin % 8 == 0 else a
+    _native.check(lib.gbdic_nn_conv_wgrad(C.byref(shape), C.c_void_p(source.data_ptr()), C.c_void_p(dz.data_ptr()),
+                                          splits, C.c_void_p(partial.data_ptr()), C.c_void_p(dw.data_ptr()),
+                                          C.c_void_p(err.data_ptr()), None), lib.gbdic_last_error(None))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    want = dz.double().T @ a.double()
+    bound = M * 2.0 ** -24 * (dz.double().abs().T @ a.double().abs())
+    assert bool(((dw.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("B,H,Cin,Cout", [(8, 32, 32, 64), (4, 16, 64, 128), (16, 8, 128, 64), (128, 15, 16, 64)])
+def test_masked_data_gradient_epilogue(B, H, Cin, Cout):
+    """ReLU backward in the data gradient's epilogue: the masked, rounded FP32
+    data gradient bit for bit, and its column sums (M additions in FP32)."""
+    lib = _native.load()
+    shape, g = _conv_case(B, H, Cin, Cout, B * H + Cout + 1)
+    OH, Min = shape.OH, B * H * H
+    dz = torch.randn(B, OH, OH, Cout, generator=g, device="cuda").to(torch.bfloat16)
+    wt = torch.randn(Cin, 9 * Cout, generator=g, device="cuda").to(torch.bfloat16)
+    y = torch.relu(torch.randn(Min, Cin, generator=g, device="cuda")).to(torch.bfloat16)
+    dy = torch.empty(Min, Cin, device="cuda")
+    _conv_gemm(dz, wt, 2, shape, Min, 9 * Cout, dy)
+    out = torch.full((Min, Cin), 7.0, dtype=torch.bfloat16, device="cuda")
+    partial, db = torch.empty(Cin * (Min // 128), device="cuda"), torch.empty(Cin, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    desc = _native.NnGemmDesc(dz.data_ptr(), wt.data_ptr(), Min, Cin, 9 * Cout, 1, None, out.data_ptr(), Cin, 0, None,
+                              0, 0)
+    _native.check(lib.gbdic_nn_conv_dgrad_relu(C.byref(desc), C.byref(shape), C.c_void_p(y.data_ptr()),
+                                               C.c_void_p(partial.data_ptr()), C.c_void_p(db.data_ptr()),
+                                               C.c_void_p(err.data_ptr()), None), lib.gbdic_last_error(None))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    masked = torch.where(y > 0, dy, torch.zeros_like(dy))
+    assert torch.equal(out, masked.to(torch.bfloat16))
+    bound = Min * 2.0 ** -24 * masked.double().abs().sum(0)
+    assert bool(((db.double() - masked.double().sum(0)).abs() <= bound).all())
