@@ -142,3 +142,31 @@ def test_quadratic_outliers_bit_exact(pairs, policy):
                             policy=policy)
     np.testing.assert_array_equal(got.reshape(-1, 16), expected)
     assert (got[..., 12] == 2.0).sum() > 5
+
+
+@pytest.mark.parametrize("scope", ["rejected", "all"])
+@pytest.mark.parametrize("size", [3, 5])
+@pytest.mark.parametrize("model", ["translation", "affine", "quadratic"])
+def test_median_fields_in_registers_bit_exact(pairs, model, size, scope):
+    """3x3 and 5x5 medians: rejected neighbours, grid edges, infinities, and NaNs
+    (whose subsets take the general selection)."""
+    ref, _ = pairs
+    plane, inverse, metadata = rp.reference_arrays(ref, motion_model=model, subset_size=21, subset_stride=10)
+    gw, gh = 1 + (W - 21) // 10, 1 + (H - 21) // 10
+    rng = np.random.default_rng(size)
+    stride, n = (16, 12) if model == "quadratic" else (8, 6)
+    state = np.zeros((gh, gw, stride), np.float32)
+    state[..., :n] = rng.normal(0, 1e-2, (gh, gw, n))
+    if model == "translation":
+        state[..., [1, 2, 4, 5]] = 0.0
+    state[..., n] = rng.choice(np.array([1.0, 2.0, 1.0, 0.0, -1.0], np.float32), (gh, gw))
+    state[2, 3, 0] = np.inf
+    state[gh - 2, 4, 3] = -np.inf
+    state[9, 11, 0] = np.nan
+    with ICGNWGPU(subset_size=21, subset_stride=10, motion_model=model, outlier_policy="median",
+                  median_filter_size=size, median_filter_scope=scope) as engine:
+        engine.set_reference_arrays(W, H, plane, metadata, inverse)
+        got = engine.apply_outlier_filter(state)
+    expected = oracle_c.uod(state.reshape(-1, stride), metadata, grid=(gw, gh), subset_stride=10, model=model,
+                            policy="median", median_size=size, scope_all=scope == "all")
+    np.testing.assert_array_equal(got.reshape(-1, stride), expected)
