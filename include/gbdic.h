@@ -457,7 +457,10 @@ typedef struct {
 
 /* Step modes: PERSISTENT, one persistent launch per shape-function class
  * (affine + translation, quadratic) on two graph branches; PER_JOB, one
- * grid launch per job; SINGLE, one persistent launch over every job. */
+ * grid launch per job; SINGLE, one persistent launch over every job, or, with
+ * ctas_per_sm 0 and 16 or 32 lanes where windows over 16 x 16, or of the banded
+ * loop, hold a quarter or more of the pixels, every job as a branch of its own (upload to readback), the
+ * solves concurrent launches.  A job's result is the same in every mode. */
 enum { GBDIC_BATCH_PERSISTENT = 0, GBDIC_BATCH_PER_JOB = 1, GBDIC_BATCH_SINGLE = 2 };
 
 int gbdic_batch_create(int32_t device, gbdic_batch **out);

@@ -30,6 +30,18 @@ struct ClassQueue {
     int grid = 0;
 };
 
+// Streams that a step's jobs are dealt out to.
+constexpr int kBranches = 8;
+// Share of a step's pixels from which its jobs run as concurrent launches, in
+// windows that gain by it: those of the banded loop and those over 16 x 16 (a
+// launch of their own kind runs the direct loop faster than the one for jobs of
+// every kind).  Measured (16 lanes, host call, single launch -> branches): 8 jobs of
+// S 21, 80 to 11,408 subsets each, 463 -> 326 us to 2,229 -> 1,805; 128 jobs of 9
+// subsets 2,968 -> 2,352; 32 jobs of affine S 33 (direct loop) 3,545 -> 2,848; eight
+// uneven jobs 3,090 -> 2,820.  Affine S 15 (direct loop, 11,844 subsets): 8 jobs
+// 2,358 -> 2,395, 32 jobs 8,825 -> 8,844.  64 lanes, 8 jobs of S 21: 2,420 -> 2,637.
+constexpr double kBranchShare = 0.25;
+
 bool is_quadratic(const BatchJobHost &j) { return j.desc.motion_model == GBDIC_MODEL_QUADRATIC; }
 
 }  // namespace
@@ -44,6 +56,15 @@ struct gbdic_batch {
     std::vector<std::unique_ptr<BatchJobHost>> jobs;
     int lanes = 16, mode = GBDIC_BATCH_SINGLE, ctas_per_sm = 0;
     ClassQueue light, heavy, all;  // per-class queues, and the single queue
+    // GBDIC_BATCH_SINGLE with as many CTAs as are resident, where enough of the
+    // windows gain: the jobs run concurrently, each as its own launch (the one launch over jobs of every kind has the direct loop only; a
+    // banded loop in it lost more to its size than it gave).  Every job's upload,
+    // prefilter, solve, outlier pass and readback are a branch of the step, so
+    // the copies and short passes of one job run beside the solves of others.
+    bool branched = false;
+    std::vector<int> branch_order;
+    cudaStream_t branches[kBranches] = {};
+    cudaEvent_t branch_join[kBranches] = {};
     gbdic::HostBuffer in, out;
     size_t in_bytes = 0, out_bytes = 0;
     cudaGraphExec_t host_graph = nullptr, device_graph = nullptr;
@@ -54,9 +75,15 @@ struct gbdic_batch {
         if (stream) cudaStreamSynchronize(stream);
         if (side) cudaStreamSynchronize(side);
         drop_graphs();
+        for (cudaStream_t b : branches)
+            if (b) cudaStreamSynchronize(b);
         for (cudaEvent_t ev : {fork, join, begin, end, solve_begin, solve_end})
             if (ev) cudaEventDestroy(ev);
+        for (cudaEvent_t ev : branch_join)
+            if (ev) cudaEventDestroy(ev);
         jobs.clear();
+        for (cudaStream_t b : branches)
+            if (b) cudaStreamDestroy(b);
         if (side) cudaStreamDestroy(side);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -77,11 +104,36 @@ struct gbdic_batch {
     void rebuild() {
         if (!dirty) return;
         const int units = gbdic::batch_units(lanes);
+        double pixels = 0.0, gaining = 0.0;
+        for (auto &job : jobs) {
+            job->rt->set_variant(lanes, false);
+            const double work = (double)job->level.count * job->desc.subset_size * job->desc.subset_size;
+            const gbdic::SolveArgs a = job->rt->solve_args(job->level, *job->level.slots[0], job->desc.cfg, false,
+                                                           false, nullptr, nullptr);
+            pixels += work;
+            if (a.band.rows > 0 || (lanes <= 32 && job->desc.subset_size > 16)) gaining += work;
+        }
+        branched = mode == GBDIC_BATCH_SINGLE && ctas_per_sm == 0 && jobs.size() > 1 && gaining >= kBranchShare * pixels;
+        if (branched) {
+            branch_order.resize(jobs.size());
+            for (int j = 0; j < (int)jobs.size(); ++j) branch_order[j] = j;
+            const auto cost = [&](int j) {
+                return (is_quadratic(*jobs[j]) ? 1.5 : 1.0) * jobs[j]->desc.subset_size * jobs[j]->desc.subset_size *
+                       jobs[j]->level.count;
+            };
+            std::stable_sort(branch_order.begin(), branch_order.end(), [&](int a, int b) { return cost(a) > cost(b); });
+            for (int b = 0; b < std::min(kBranches, (int)jobs.size()); ++b) {
+                if (!branches[b])
+                    check_cuda(cudaStreamCreateWithFlags(&branches[b], cudaStreamNonBlocking), "stream");
+                if (!branch_join[b])
+                    check_cuda(cudaEventCreateWithFlags(&branch_join[b], cudaEventDisableTiming), "event");
+            }
+        }
         // Queue 0: light class, 1: quadratic class, 2: every job (SINGLE).
         for (int cls = 0; cls < 3; ++cls) {
             ClassQueue &q = cls == 0 ? light : cls == 1 ? heavy : all;
             q.order.clear();
-            if ((cls == 2) != (mode == GBDIC_BATCH_SINGLE)) {
+            if (branched || (cls == 2) != (mode == GBDIC_BATCH_SINGLE)) {
                 q.grid = 0;
                 continue;
             }
@@ -135,7 +187,6 @@ struct gbdic_batch {
             in_bytes += ((size_t)job.level.W * job.level.H + 255) / 256 * 256;
             job.out_offset = out_bytes;
             out_bytes += (job.state_bytes + 255) / 256 * 256;
-            job.rt->set_variant(lanes, false);
         }
         in.ensure(in_bytes);
         out.ensure(out_bytes);
@@ -157,14 +208,42 @@ struct gbdic_batch {
                    "batch solver launch");
     }
 
+    // fn(job, stream) for every job on the branches, costliest first; `s` before
+    // and after.
+    template <typename F>
+    void on_branches(cudaStream_t s, F &&fn) {
+        const int used = std::min(kBranches, (int)jobs.size());
+        check_cuda(cudaEventRecord(fork, s), "fork");
+        for (int b = 0; b < used; ++b) check_cuda(cudaStreamWaitEvent(branches[b], fork, 0), "fork");
+        for (size_t k = 0; k < branch_order.size(); ++k)
+            fn(*jobs[(size_t)branch_order[k]], branches[k % (size_t)used]);
+        for (int b = 0; b < used; ++b) {
+            check_cuda(cudaEventRecord(branch_join[b], branches[b]), "join");
+            check_cuda(cudaStreamWaitEvent(s, branch_join[b], 0), "join");
+        }
+    }
+
+    void solve_job(BatchJobHost &job, cudaStream_t s) {
+        job.rt->enqueue_solve(job.level, *job.level.slots[0], job.desc.cfg, false, false, nullptr, nullptr, s);
+    }
+    void upload_job(BatchJobHost &job, cudaStream_t s) {
+        check_cuda(cudaMemcpyAsync(job.level.slots[0]->frame.get(), in.as<uint8_t>() + job.in_offset,
+                                   (size_t)job.level.W * job.level.H, cudaMemcpyHostToDevice, s), "frame upload");
+    }
+    void readback_job(BatchJobHost &job, cudaStream_t s) {
+        check_cuda(cudaMemcpyAsync(out.as<uint8_t>() + job.out_offset, job.rt->output_state(*job.level.slots[0]),
+                                   job.state_bytes, cudaMemcpyDeviceToHost, s), "state readback");
+    }
+
     // Prefilter -> solver launches -> outlier passes on `s`; with `timed`,
     // events bracket the solver section.
     void enqueue_compute(cudaStream_t s, bool timed) {
         for (auto &jp : jobs) jp->rt->enqueue_prefilter(jp->level, *jp->level.slots[0], nullptr, s);
         if (timed) check_cuda(cudaEventRecord(solve_begin, s), "event");
-        if (mode == GBDIC_BATCH_PER_JOB) {
-            for (auto &jp : jobs)
-                jp->rt->enqueue_solve(jp->level, *jp->level.slots[0], jp->desc.cfg, false, false, nullptr, nullptr, s);
+        if (branched) {
+            on_branches(s, [&](BatchJobHost &job, cudaStream_t b) { solve_job(job, b); });
+        } else if (mode == GBDIC_BATCH_PER_JOB) {
+            for (auto &jp : jobs) solve_job(*jp, s);
         } else if (mode == GBDIC_BATCH_SINGLE) {
             launch_class(all, 2, s);
         } else {
@@ -189,18 +268,22 @@ struct gbdic_batch {
         cudaGraph_t graph = nullptr;
         check_cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "capture");
         try {
-            if (with_copies)
-                for (auto &jp : jobs)
-                    check_cuda(cudaMemcpyAsync(jp->level.slots[0]->frame.get(), in.as<uint8_t>() + jp->in_offset,
-                                               (size_t)jp->level.W * jp->level.H, cudaMemcpyHostToDevice, stream),
-                               "frame upload");
-            enqueue_compute(stream, false);
-            if (with_copies)
-                for (auto &jp : jobs)
-                    check_cuda(cudaMemcpyAsync(out.as<uint8_t>() + jp->out_offset,
-                                               jp->rt->output_state(*jp->level.slots[0]), jp->state_bytes,
-                                               cudaMemcpyDeviceToHost, stream),
-                               "state readback");
+            if (branched) {
+                on_branches(stream, [&](BatchJobHost &job, cudaStream_t b) {
+                    auto &slot = *job.level.slots[0];
+                    if (with_copies) upload_job(job, b);
+                    job.rt->enqueue_prefilter(job.level, slot, nullptr, b);
+                    solve_job(job, b);
+                    job.rt->enqueue_uod(job.level, slot, false, nullptr, b);
+                    if (with_copies) readback_job(job, b);
+                });
+            } else {
+                if (with_copies)
+                    for (auto &jp : jobs) upload_job(*jp, stream);
+                enqueue_compute(stream, false);
+                if (with_copies)
+                    for (auto &jp : jobs) readback_job(*jp, stream);
+            }
         } catch (...) {
             cudaStreamEndCapture(stream, &graph);
             if (graph) cudaGraphDestroy(graph);

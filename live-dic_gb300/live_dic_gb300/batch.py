@@ -8,7 +8,9 @@ weighting, zero seed, the job's outlier pass) and a step runs all jobs as one
 CUDA graph: every target's prefilter, one persistent IC-GN launch per
 shape-function class over a device work queue ("persistent"), or one
 persistent launch over every job with the shape function dispatched per job
-("single"), then the outlier passes.
+("single"), then the outlier passes.  Unless most of the pixels are in
+windows up to 16 x 16, "single" without a limit on CTAs runs the jobs as
+concurrent branches of the graph instead, upload to readback.
 A job's result is bit-identical to ICGNWGPU.register with the same lanes per
 subset.
 

@@ -132,3 +132,31 @@ def test_batch_argument_errors(pairs):
             batch.register([])
         with pytest.raises(ValueError, match="does not match"):
             batch.register([np.zeros((32, 32), np.uint8)])
+
+
+@pytest.mark.parametrize("lanes", [16, 32])
+def test_batch_branches_equal_the_single_launch(pairs, lanes):
+    """More jobs than branches, banded and direct loops, host frames and device
+    frames on the caller's stream: fields of the one persistent launch."""
+    torch = pytest.importorskip("torch")
+    jobs = [pairs[k % len(pairs)] for k in range(11)]
+    targets = [j["target"] for j in jobs]
+    with _batch(jobs, solver_workgroup_size=lanes) as batch:
+        batch.set_variant(lanes, "single", 32)
+        expected = [_packed(r) for r in batch.register(targets)]
+        batch.set_variant(lanes, "single")
+        for _ in range(2):
+            for got, want in zip(batch.register(targets), expected, strict=True):
+                np.testing.assert_array_equal(_packed(got), want)
+        # other frames, then the first again, on a stream of the caller
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            for frames in ([np.roll(t, 3, 1) for t in targets], targets):
+                device = [torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in frames]
+                for j, f in enumerate(device):
+                    batch.load_device(j, f.data_ptr(), f.stride(0), stream.cuda_stream)
+                batch.run_device(stream.cuda_stream)
+        stream.synchronize()
+        for j, want in enumerate(expected):
+            got = batch.export_state(j)
+            np.testing.assert_array_equal(got[..., : want.shape[-1]], want)
