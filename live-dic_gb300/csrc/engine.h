@@ -111,7 +111,7 @@ struct Level {
     const float *solver_f = nullptr;
     DeviceBuffer intensity, spline, scratch, valid;  // preparation scratch
     DeviceBuffer admissible;                         // u8 per subset, ROI ignored
-    DeviceBuffer moments;                            // quadratic row path: moments per subset
+    DeviceBuffer moments;                            // affine, quadratic row path: moments per subset
     DeviceBuffer ref_image;                          // reference bytes (seed search)
     DeviceBuffer partial_index, partial_words, partial_boxes;  // partial-support windows
     int partial_count = 0, support_words = 0;

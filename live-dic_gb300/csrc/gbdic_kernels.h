@@ -103,7 +103,9 @@ struct PrepArgs {
     // quadratic row path: [71][count] binary32 moments and means, or nullptr
     // (per-window path)
     float *moments;
+    float *window_moments;  // affine: affine_prep_moment_floats(count) floats
 };
+size_t affine_prep_moment_floats(int count);
 cudaError_t launch_reference_prep(const PrepArgs &a, cudaStream_t stream);
 // f and (unless nullptr) (gx, gy) of a reference plane as planes of their own.
 cudaError_t launch_split_plane(const float4 *plane, size_t pixels, float *f, float2 *grad, cudaStream_t stream);

@@ -118,9 +118,15 @@ __global__ void spline_columns_kernel(const float *__restrict__ in, int n, int c
         prev = 0.0f;
         k = s;
     }
+    // Unrolled so that the loads of several rows are in flight: the chain is
+    // four cycles a row, a load alone hundreds (1280 x 720: 14.7 us a pass with
+    // a row at a time, 9.0 so).
+#pragma unroll 8
+    for (; k < a0; ++k) prev = fmaf(z, prev, gain * in[(size_t)k * cols + c]);
+#pragma unroll 8
     for (; k < e; ++k) {
         prev = fmaf(z, prev, gain * in[(size_t)k * cols + c]);
-        if (k >= a0) cp[k - a0] = prev;
+        cp[k - a0] = prev;
     }
     float next;
     int j;
@@ -132,9 +138,13 @@ __global__ void spline_columns_kernel(const float *__restrict__ in, int n, int c
         next = 0.0f;
         j = e - 1;
     }
+    // (the product rounded by itself: not contracted into the next row's difference)
+#pragma unroll 8
+    for (; j >= b; --j) next = __fmul_rn(z, next - cp[j - a0]);
+#pragma unroll 8
     for (; j >= a; --j) {
-        next = z * (next - cp[j - a0]);
-        if (j < b) out[(size_t)j * cols + c] = next;
+        next = __fmul_rn(z, next - cp[j - a0]);
+        out[(size_t)j * cols + c] = next;
     }
 }
 
@@ -285,72 +295,9 @@ __device__ __forceinline__ void warp_compensated_sum(float &s, float &c) {
     }
 }
 
-// Warp-cooperative Cholesky inverse of an SPD n x n matrix held in shared
-// memory (row-major A), with Jacobi scaling d_i = 1/sqrt(A_ii).  On return
-// X holds A^-1; returns false if A is not numerically positive definite.
-// Used for the FP32 6x6 Hessians; the FP64 12x12 quadratic ones go through
-// cholesky_inverse_split.
-template <typename T>
-__device__ bool cholesky_inverse(T *A, T *X, T *d, int n, int lane) {
-    bool ok = true;
-    if (lane < n) {
-        const T aii = A[lane * n + lane];
-        ok = aii > T(0);
-        d[lane] = ok ? T(1) / sqrt(aii) : T(0);
-    }
-    ok = __all_sync(kFullMask, ok);
-    if (!ok) return false;
-    __syncwarp();
-    if (lane < n)
-        for (int j = 0; j < n; ++j) A[lane * n + j] = A[lane * n + j] * d[lane] * d[j];
-    __syncwarp();
-    for (int k = 0; k < n; ++k) {
-        T pivot = A[k * n + k];
-        ok = pivot > T(0);
-        if (!__all_sync(kFullMask, ok)) return false;
-        const T lkk = sqrt(pivot);
-        __syncwarp();
-        if (lane == k) A[k * n + k] = lkk;
-        if (lane > k && lane < n) A[lane * n + k] = A[lane * n + k] / lkk;
-        __syncwarp();
-        if (lane > k && lane < n) {
-            const T lik = A[lane * n + k];
-            for (int j = k + 1; j <= lane; ++j) A[lane * n + j] = A[lane * n + j] - lik * A[j * n + k];
-        }
-        __syncwarp();
-    }
-    // lane j: column j of L^-1 (forward substitution) into X (lower part)
-    if (lane < n) {
-        const int j = lane;
-        for (int i = 0; i < n; ++i) X[i * n + j] = T(0);
-        X[j * n + j] = T(1) / A[j * n + j];
-        for (int i = j + 1; i < n; ++i) {
-            T acc = T(0);
-            for (int k = j; k < i; ++k) acc = acc + A[i * n + k] * X[k * n + j];
-            X[i * n + j] = -acc / A[i * n + i];
-        }
-    }
-    __syncwarp();
-    // A^-1 = L^-T L^-1; lane i writes row i into A (A no longer needed).
-    if (lane < n) {
-        const int i = lane;
-        for (int j = 0; j < n; ++j) {
-            const int k0 = i > j ? i : j;
-            T acc = T(0);
-            for (int k = k0; k < n; ++k) acc = acc + X[k * n + i] * X[k * n + j];
-            A[i * n + j] = acc * d[i] * d[j];
-        }
-    }
-    __syncwarp();
-    if (lane < n)
-        for (int j = 0; j < n; ++j) X[lane * n + j] = A[lane * n + j];
-    __syncwarp();
-    return true;
-}
-
 // FP64 Cholesky inverse of the 12x12 quadratic Hessian with two lanes per
 // row (lane & 15 = row, lane >> 4 = half): the Jacobi-scaled factorisation,
-// L^-1 and L^-T L^-1 of cholesky_inverse, with every row's j loops and
+// L^-1 and L^-T L^-1 (L^-1 column by column), with every row's j loops and
 // k sums split by parity between the two halves (partial sums combined by
 // one shuffle), so the warp issues about half the FP64 instructions.
 __device__ bool cholesky_inverse_split(double *A, double *X, double *d, int n, int lane) {
@@ -413,12 +360,197 @@ __device__ bool cholesky_inverse_split(double *A, double *X, double *d, int n, i
     return true;
 }
 
+// ---------------------------------------------------------------- affine
+// The affine model's windows in two kernels.  A warp sums a window's 31 moments
+// (Kahan sums in FP32 pairs, 128 issue cycles a pixel step of 32: what bounds it)
+// and combines its lanes' sums by halves: each step a lane gives away half of
+// the moments it holds and keeps the other half's sums of two lanes, so 31
+// merges take the place of 155 and lane q ends with moment q.  Then a thread has
+// a window: the Jacobi-scaled 6x6 Cholesky inverse in its registers, where six
+// lanes of the summing warp went through shared memory.  The merges' trees and
+// the inverse's operations are those of the one-kernel form (bit for bit).
+// 1280 x 720, S 21 / s 7 (18,180 windows): 123 us in one kernel -> 74 + 5.
+constexpr int kAffineMoments = 32;  // 31 moments and the mean, a row per window
+
+__global__ void __launch_bounds__(128) affine_moments_kernel(PrepArgs a) {
+    constexpr int NM = Moments<kModelAffine>::count;
+    static_assert(NM == kAffineMoments - 1, "one lane per moment, and one for the mean");
+    const int lane = threadIdx.x & 31, idx = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (idx >= a.count) return;  // warp-uniform
+    const int S = a.S, npix = S * S;
+    const int gx0 = (idx % a.grid_w) * a.stride, gy0 = (idx / a.grid_w) * a.stride;
+    const float half = 0.5f * ((float)S - 1.0f);
+    // Pixel p = lane + 32 k of the window, tracked without divisions.
+    const int ldiv = 32 / S, lmod = 32 % S, col0 = lane % S, row0 = lane / S;
+    const size_t origin = (size_t)gy0 * a.W + gx0;
+    float mean;
+    {
+        float s = 0.0f, c = 0.0f;
+        int col = col0, row = row0;
+        for (int p = lane; p < npix; p += 32) {
+            kahan_add(s, c, a.weights[p] * a.intensity[origin + (size_t)row * a.W + col]);
+            col += lmod;
+            row += ldiv;
+            if (col >= S) { col -= S; ++row; }
+        }
+        warp_compensated_sum(s, c);
+        mean = __shfl_sync(kFullMask, s + c, 0) / a.weight_sum;
+    }
+    // Kahan sums of moment pairs in packed FP32 (FADD2 / FFMA2): every
+    // component follows kahan_add's sequence, a - b written as
+    // fma(b, -1, a) (an exact product, so the same rounding).
+    float2 ms2[kAffineMoments / 2], mc2[kAffineMoments / 2];
+#pragma unroll
+    for (int q = 0; q < kAffineMoments / 2; ++q) { ms2[q] = make_float2(0.0f, 0.0f); mc2[q] = make_float2(0.0f, 0.0f); }
+    {
+        int col = col0, row = row0;
+        for (int p = lane; p < npix; p += 32) {
+            const float4 v = a.plane[origin + (size_t)row * a.W + col];
+            const float f = v.x - mean, w = a.weights[p];
+            const float x = (float)col - half, y = (float)row - half;
+            const float m[3] = {1.0f, x, y};
+            float mv[NM];
+            moment_values<kModelAffine>(w, f, v.y, v.z, m, mv);
+            const float2 m1 = make_float2(-1.0f, -1.0f);
+#pragma unroll
+            for (int q = 0; q < kAffineMoments / 2; ++q) {
+                const float2 val = make_float2(mv[2 * q], 2 * q + 1 < NM ? mv[2 * q + 1] : 0.0f);
+                const float2 y2 = __ffma2_rn(mc2[q], m1, val);
+                const float2 t = __fadd2_rn(ms2[q], y2);
+                mc2[q] = __ffma2_rn(y2, m1, __ffma2_rn(ms2[q], m1, t));
+                ms2[q] = t;
+            }
+            col += lmod;
+            row += ldiv;
+            if (col >= S) { col -= S; ++row; }
+        }
+    }
+    float s[kAffineMoments], c[kAffineMoments];
+#pragma unroll
+    for (int q = 0; q < kAffineMoments / 2; ++q) {
+        s[2 * q] = ms2[q].x;
+        s[2 * q + 1] = ms2[q].y;
+        c[2 * q] = -mc2[q].x;
+        c[2 * q + 1] = -mc2[q].y;
+    }
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+        const bool upper = lane & h;
+#pragma unroll
+        for (int q = 0; q < h; ++q) {
+            const float s2 = __shfl_xor_sync(kFullMask, upper ? s[q] : s[q + h], h);
+            const float c2 = __shfl_xor_sync(kFullMask, upper ? c[q] : c[q + h], h);
+            if (upper) { s[q] = s[q + h]; c[q] = c[q + h]; }
+            twosum_merge(s[q], c[q], s2, c2);
+        }
+    }
+    a.window_moments[(size_t)idx * kAffineMoments + lane] = lane < NM ? s[0] + c[0] : mean;
+    // centre the plane for tiled (non-overlapping) grids
+    if (a.stride == S) {
+        for (int p = lane; p < npix; p += 32) {
+            float4 *dst = a.plane + origin + (size_t)(p / S) * a.W + p % S;
+            dst->x = dst->x - mean;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(64) affine_finish_kernel(PrepArgs a) {
+    constexpr int n = 6, nm = 3, P = Moments<kModelAffine>::hess;
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = idx < a.count;
+    float t[kAffineMoments];
+    {
+        const float4 *row = reinterpret_cast<const float4 *>(a.window_moments) + (size_t)(live ? idx : 0) * (kAffineMoments / 4);
+#pragma unroll
+        for (int q = 0; q < kAffineMoments / 4; ++q) {
+            const float4 v = row[q];
+            t[4 * q] = v.x; t[4 * q + 1] = v.y; t[4 * q + 2] = v.z; t[4 * q + 3] = v.w;
+        }
+    }
+    const float energy = t[0];
+    // Jacobian column q = (gradient block q / 3, monomial q % 3)
+    float A[n][n], X[n][n], d[n];
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+            const int lo = j % 3 < i % 3 ? j % 3 : i % 3, hi = j % 3 < i % 3 ? i % 3 : j % 3;
+            A[i][j] = t[1 + 4 * nm + (i / 3 + j / 3) * P + pair_index(nm, lo, hi)];
+        }
+        ok = ok && A[i][i] > 0.0f;
+        d[i] = A[i][i] > 0.0f ? 1.0f / sqrtf(A[i][i]) : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+#pragma unroll
+        for (int j = 0; j <= i; ++j) A[i][j] = A[i][j] * d[i] * d[j];
+    // Cholesky factor in place
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+        ok = ok && A[k][k] > 0.0f;
+        const float lkk = sqrtf(A[k][k]);
+        A[k][k] = lkk;
+#pragma unroll
+        for (int i = k + 1; i < n; ++i) A[i][k] = A[i][k] / lkk;
+#pragma unroll
+        for (int i = k + 1; i < n; ++i)
+#pragma unroll
+            for (int j = k + 1; j <= i; ++j) A[i][j] = A[i][j] - A[i][k] * A[j][k];
+    }
+    // L^-1, column by column
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+        X[j][j] = 1.0f / A[j][j];
+#pragma unroll
+        for (int i = j + 1; i < n; ++i) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = j; k < i; ++k) acc = acc + A[i][k] * X[k][j];
+            X[i][j] = -acc / A[i][i];
+        }
+    }
+    // A^-1 = D L^-T L^-1 D, row by row
+    float inverse[n * n];
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < n; ++i)
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+            float acc = 0.0f;
+#pragma unroll
+            for (int k = i > j ? i : j; k < n; ++k) acc = acc + X[k][i] * X[k][j];
+            inverse[i * n + j] = acc * d[i] * d[j];
+            finite = finite && isfinite(inverse[i * n + j]);
+        }
+    const bool valid = live && energy > 1e-12f && ok && finite;
+    const bool selected = live && (a.selected == nullptr || a.selected[idx] != 0);
+    if (live) {
+        float4 *inv = reinterpret_cast<float4 *>(a.inv + (size_t)idx * n * n);
+#pragma unroll
+        for (int q = 0; q < n * n / 4; ++q)
+            inv[q] = valid ? make_float4(inverse[4 * q], inverse[4 * q + 1], inverse[4 * q + 2], inverse[4 * q + 3])
+                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        // norm, validity, J^T f (6), sum J (6), mean, weight sum
+        static_assert(meta_stride(kModelAffine) == 16, "four vectors of metadata");
+        float4 *md = reinterpret_cast<float4 *>(a.meta + (size_t)idx * meta_stride(kModelAffine));
+        md[0] = make_float4(sqrtf(fmaxf(energy, 0.0f)), selected ? (valid ? 1.0f : 0.0f) : -3.0f, t[1], t[2]);
+        md[1] = make_float4(t[3], t[4], t[5], t[6]);
+        md[2] = make_float4(t[7], t[8], t[9], t[10]);
+        md[3] = make_float4(t[11], t[12], a.stride == a.S ? 0.0f : t[kAffineMoments - 1], a.weight_sum);
+        a.admissible[idx] = valid ? 1 : 0;
+    }
+    const unsigned counted = __ballot_sync(kFullMask, valid && selected);
+    if ((threadIdx.x & 31) == 0 && counted) atomicAdd(a.valid_count, (unsigned)__popc(counted));
+}
+
+// ---------------------------------------------------------------- translation, quadratic
 template <int MODEL>
 __global__ void __launch_bounds__(128) subset_prep_kernel(PrepArgs a) {
     using T = typename std::conditional<MODEL == kModelQuadratic, double, float>::type;
     constexpr int n = parameter_count(MODEL);
     constexpr int nm = Moments<MODEL>::nm, P = Moments<MODEL>::hess, NM = Moments<MODEL>::count;
-    constexpr int kChunkM = MODEL == kModelTranslation ? 8 : (MODEL == kModelQuadratic ? 36 : 32);
+    constexpr int kChunkM = MODEL == kModelTranslation ? 8 : 36;
     __shared__ float s_tot[4][NM];
     __shared__ T s_A[4][n * n];
     __shared__ T s_X[4][n * n];
@@ -504,7 +636,7 @@ __global__ void __launch_bounds__(128) subset_prep_kernel(PrepArgs a) {
 #pragma unroll
     for (int q = 0; q < n; ++q) { jtf[q] = 0.0f; sj[q] = 0.0f; }
     bool valid = energy > 1e-12f;
-    if (MODEL == kModelTranslation) {
+    if constexpr (MODEL == kModelTranslation) {
         // moments: 0 f^2, 1 gx f, 2 gy f, 3 gx, 4 gy, 5 gx^2, 6 gx gy, 7 gy^2
         jtf[0] = t[1]; jtf[3] = t[2]; sj[0] = t[3]; sj[3] = t[4];
         const float hxx = t[5], hxy = t[6], hyy = t[7];
@@ -543,9 +675,7 @@ __global__ void __launch_bounds__(128) subset_prep_kernel(PrepArgs a) {
             }
         }
         __syncwarp();
-        bool ok;
-        if constexpr (std::is_same<T, double>::value) ok = cholesky_inverse_split(A, X, s_d[warp], n, lane);
-        else ok = cholesky_inverse<T>(A, X, s_d[warp], n, lane);
+        const bool ok = cholesky_inverse_split(A, X, s_d[warp], n, lane);
         valid = valid && ok;
         if (ok) {
             bool finite = true;
@@ -584,6 +714,8 @@ cudaError_t launch_split_plane(const float4 *plane, size_t pixels, float *f, flo
 
 cudaError_t set_gauss_taps(const float *taps7) { return cudaMemcpyToSymbol(c_gauss, taps7, 7 * sizeof(float)); }
 
+size_t affine_prep_moment_floats(int count) { return (size_t)kAffineMoments * (size_t)count; }
+
 cudaError_t launch_reference_prep(const PrepArgs &a, cudaStream_t stream) {
     const int W = a.W, H = a.H;
     const bool bspline = a.interp == kInterpBspline;
@@ -613,7 +745,11 @@ cudaError_t launch_reference_prep(const PrepArgs &a, cudaStream_t stream) {
         switch (a.model) {
         case kModelTranslation: subset_prep_kernel<kModelTranslation><<<blocks, 128, 0, stream>>>(a); break;
         case kModelQuadratic: subset_prep_kernel<kModelQuadratic><<<blocks, 128, 0, stream>>>(a); break;
-        default: subset_prep_kernel<kModelAffine><<<blocks, 128, 0, stream>>>(a); break;
+        default:
+            if (!a.window_moments) return cudaErrorInvalidValue;
+            affine_moments_kernel<<<blocks, 128, 0, stream>>>(a);
+            affine_finish_kernel<<<(a.count + 63) / 64, 64, 0, stream>>>(a);
+            break;
         }
     }
     return cudaGetLastError();

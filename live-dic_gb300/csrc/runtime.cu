@@ -350,6 +350,11 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
         level.moments.ensure(quadratic_row_prep_moment_floats(level.count) * sizeof(float));
         a.moments = level.moments.as<float>();
     }
+    a.window_moments = nullptr;
+    if (model == GBDIC_MODEL_AFFINE) {
+        level.moments.ensure(affine_prep_moment_floats(level.count) * sizeof(float));
+        a.window_moments = level.moments.as<float>();
+    }
     cudaEvent_t e0, e1;
     check_cuda(cudaEventCreate(&e0), "event");
     check_cuda(cudaEventCreate(&e1), "event");

@@ -118,3 +118,49 @@ def test_flat_reference_invalid_and_finite():
         assert not engine.reference_valid.any()
     assert np.isfinite(plane).all() and np.isfinite(inverse).all() and np.isfinite(metadata).all()
     assert not inverse.any()
+
+
+@pytest.mark.parametrize("size,stride", [(90, 9), (43, 8), (36, 9), (21, 7), (33, 4), (47, 3)])
+def test_affine_moments_and_inverse_from_the_plane(size, stride):
+    """The affine moments' rows and the thread-per-window inverse against float64
+    sums over the exported plane: 2, 56 and more windows (blocks of 64), window
+    columns that wrap a warp's 32 lanes.  A term is a product of at most five
+    FP32 factors and f carries the FP32 mean's rounding, a Kahan sum adds two
+    roundings: within 2^-20 of the magnitudes' sum.  The inverse of the scaled
+    Hessian loses its condition number times 6^2 roundings."""
+    with ICGNWGPU(subset_size=size, subset_stride=stride) as engine:
+        engine.set_reference(_texture())
+        plane, inverse, metadata = engine.export_reference()
+    plane = plane.reshape(H, W, 4).astype(np.float64)
+    meta, inv = metadata.reshape(-1, 16), inverse.reshape(-1, 6, 6)
+    gw, gh = 1 + (W - size) // stride, 1 + (H - size) // stride
+    assert meta.shape[0] == gw * gh
+    offset = np.arange(size) - (size - 1) / 2
+    x, y = np.meshgrid(offset, offset)
+    mono = np.stack([np.ones_like(x), x, y])
+    for index in range(gw * gh):
+        win = plane[index // gw * stride:][:size, index % gw * stride:][:, :size]
+        value, J = win[..., 0], np.concatenate([win[..., 1] * mono, win[..., 2] * mono])
+        f = value - value.mean()
+        reach = np.abs(J) * (np.abs(value) + value.mean())
+        assert np.all(np.abs(meta[index, 2:8] - (J * f).sum((1, 2))) <= 2.0 ** -20 * reach.sum((1, 2)))
+        assert np.all(np.abs(meta[index, 8:14] - J.sum((1, 2))) <= 2.0 ** -20 * np.abs(J).sum((1, 2)))
+        assert abs(meta[index, 0] ** 2 - (f * f).sum()) <= 2.0 ** -20 * ((np.abs(value) + value.mean()) ** 2).sum()
+        assert meta[index, 1] == 1.0
+        hessian = np.einsum("ahw,bhw->ab", J, J)
+        d = 1 / np.sqrt(np.diag(hessian))
+        exact = np.linalg.inv(hessian)
+        scaled = np.abs(inv[index] - exact) / np.outer(d, d)
+        bound = 36 * 2.0 ** -20 * np.linalg.cond(hessian * np.outer(d, d)) * np.abs(exact / np.outer(d, d)).max()
+        assert scaled.max() <= bound
+
+
+def test_affine_flat_windows_are_invalid():
+    image = _texture()
+    image[20:80, 20:80] = 90
+    with ICGNWGPU(subset_size=15, subset_stride=5) as engine:
+        engine.set_reference(image)
+        _, inverse, metadata = engine.export_reference()
+    meta, inv = metadata.reshape(-1, 16), inverse.reshape(-1, 36)
+    flat = meta[:, 1] == 0.0
+    assert flat.sum() >= 4 and not inv[flat].any() and inv[~flat].any(axis=1).all()
