@@ -42,14 +42,22 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
 void fail(int code, const std::string &message) { throw Failure{code, message}; }
 
 // Bounded host wait on an event (GBDIC_ETIMEOUT after `timeout_ms`).
+// A call's launches are waited for by asking again at once for two
+// milliseconds (a frame's time; a sleep, however short, returns 50-70 us later
+// with the kernel's timer slack, a quarter of a small frame's call), then with
+// sleeps between.
+constexpr double kSpinMs = 2.0;
+
 void wait_event(cudaEvent_t ev, double timeout_ms) {
     const auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         cudaError_t err = cudaEventQuery(ev);
         if (err == cudaSuccess) return;
         if (err != cudaErrorNotReady) check_cuda(err, "device execution");
-        if (ms_since(t0) > timeout_ms) fail(GBDIC_ETIMEOUT, "device work did not complete within the wait limit");
-        std::this_thread::sleep_for(std::chrono::microseconds(20));
+        const double waited = ms_since(t0);
+        if (waited > timeout_ms) fail(GBDIC_ETIMEOUT, "device work did not complete within the wait limit");
+        if (waited < kSpinMs) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
 }
 
