@@ -584,7 +584,8 @@ int gbdic_nn_conv_gemm(const gbdic_nn_gemm_desc *desc, int32_t mode, const gbdic
  * epilogue: desc->d_bf16 (BF16, M x N, row stride ldd; d_f32 and bias NULL)
  * receives dY where y (its activations, BF16, the same rows and stride) is
  * positive and 0 elsewhere; db[n] its column sums before rounding, in a fixed
- * order.  partial: device scratch of N * M / 128 floats. */
+ * order.  partial: device scratch of N * M / 128 floats, [n][M / 128]; db NULL
+ * leaves the sums of the 128-row tiles there. */
 int gbdic_nn_conv_dgrad_relu(const gbdic_nn_gemm_desc *desc, const gbdic_nn_conv_shape *shape, const void *y,
                              float *partial, float *db, int32_t *device_error, void *stream);
 /* Weight gradient dw[Cout][Kp] = sum over output pixels of the im2col row of x
@@ -592,7 +593,8 @@ int gbdic_nn_conv_dgrad_relu(const gbdic_nn_gemm_desc *desc, const gbdic_nn_conv
  * neither operand transposed nor the im2col matrix written.  With fewer than
  * eight channels (Kp 64, Cout 32) x is the matrix gbdic_nn_im2col wrote.
  * Pixels are split over `splits` partial sums (B*OH*OW % (64 splits) == 0) in
- * `partial` (splits * Kp * Cout floats), added in split order. */
+ * `partial` (splits * Kp * Cout floats), added in split order; dw NULL leaves
+ * them there. */
 int gbdic_nn_conv_wgrad(const gbdic_nn_conv_shape *shape, const void *x, const void *dz, int32_t splits,
                         float *partial, float *dw, int32_t *device_error, void *stream);
 /* Forward GEMM operand A[(b, oy, ox)][(ky, kx, ci)] (zero beyond 9 C). */
@@ -645,6 +647,26 @@ int gbdic_nn_adam(float *param, const float *grad, float *m, float *v, int64_t c
  * gbdic_nn_adam. */
 int gbdic_nn_adam_many(float *const *params, const float *const *grads, float *const *m, float *const *v,
                        const int64_t *counts, int32_t tensors, const float *hyper, void *stream);
+/* The same with the BF16 operands of the updated weights: pack[t] (or NULL for
+ * none; wb NULL for a tensor without) receives W [cout][kp] as wb and, when wt
+ * != NULL, wt[ci][(ky, kx, co)] (row length kt) or, transposed, wt[k][co]. */
+typedef struct {
+    void *wb, *wt;
+    int32_t cout, cin, kp, kt, transposed;
+} gbdic_nn_pack_target;
+int gbdic_nn_adam_pack_many(float *const *params, const float *const *grads, float *const *m, float *const *v,
+                            const int64_t *counts, int32_t tensors, const float *hyper,
+                            const gbdic_nn_pack_target *pack, void *stream);
+/* 1 to 16 reductions in one launch, each in a fixed order: cols > 0,
+ * out[n * rows + k] = sum_s partial[(s * rows + k) * cols + n] (split-K partials
+ * of a weight gradient); cols == 0, out[c] = sum_s partial[c * splits + s]
+ * (column sums). */
+typedef struct {
+    const float *partial;
+    float *out;
+    int32_t splits, rows, cols;
+} gbdic_nn_reduction;
+int gbdic_nn_reduce_many(const gbdic_nn_reduction *jobs, int32_t count, void *stream);
 /* BF16 copy of W [Cout][Kp] and, when wt != NULL, the data-gradient operand
  * Wt[ci][(ky, kx, co)] (row length kt). */
 int gbdic_nn_pack_weights(const float *w, int32_t cout, int32_t cin, int32_t kp, void *wb, void *wt, int32_t kt,

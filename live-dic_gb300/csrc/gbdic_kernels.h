@@ -279,6 +279,12 @@ struct NnAdamArgs {
 };
 // Several tensors in one launch (passed by value with the launch).
 constexpr int kMaxAdamTensors = 16;
+// BF16 operands written from an updated weight tensor [cout][kp]: its copy wb,
+// and wt: wt[ci][(tap, co)] of row length kt, or wt[k][co] when `transposed`.
+struct NnPackInto {
+    void *wb, *wt;
+    int cout, cin, kp, kt, transposed;
+};
 struct NnAdamMany {
     float *param[kMaxAdamTensors];
     const float *grad[kMaxAdamTensors];
@@ -286,7 +292,23 @@ struct NnAdamMany {
     long long offset[kMaxAdamTensors + 1];  // element offsets of the tensors in the concatenation
     int n;
     float lr, beta1, beta2, eps, bias1, bias2, weight_decay;
+    NnPackInto pack[kMaxAdamTensors];  // wb nullptr: none
 };
+// Reductions of several partial results in one launch.  cols > 0:
+// out[n * rows + k] = sum_s partial[(s * rows + k) * cols + n]; cols == 0:
+// out[c] = sum_s partial[c * splits + s], c < rows.
+constexpr int kMaxReduceJobs = 16;
+struct NnReduceJob {
+    const float *partial;
+    float *out;
+    int splits, rows, cols;
+    int first_block;  // set by the launcher
+};
+struct NnReduceMany {
+    NnReduceJob job[kMaxReduceJobs];
+    int n;
+};
+cudaError_t launch_nn_reduce_many(const NnReduceMany &jobs, cudaStream_t s);
 cudaError_t launch_nn_adam_many(const NnAdamMany &a, cudaStream_t s);
 cudaError_t launch_nn_patches(const NnPatchArgs &a, cudaStream_t s);
 cudaError_t launch_nn_im2col(const NnConvShape &sh, const void *x, void *A, cudaStream_t s);

@@ -63,7 +63,7 @@ int gbdic_nn_conv_gemm(const gbdic_nn_gemm_desc *d, int32_t mode, const gbdic_nn
 
 int gbdic_nn_conv_dgrad_relu(const gbdic_nn_gemm_desc *d, const gbdic_nn_conv_shape *s, const void *y, float *partial,
                              float *db, int32_t *device_error, void *stream) {
-    if (!d || !valid_shape(s) || !y || !partial || !db) return invalid("data-gradient arguments are incomplete");
+    if (!d || !valid_shape(s) || !y || !partial) return invalid("data-gradient arguments are incomplete");
     if (!d->d_bf16 || d->d_f32 || d->bias || d->relu || d->accumulate)
         return invalid("the ReLU-masked data gradient is written as BF16 only");
     gbdic::TcGemmArgs a{};
@@ -77,17 +77,17 @@ int gbdic_nn_conv_dgrad_relu(const gbdic_nn_gemm_desc *d, const gbdic_nn_conv_sh
     a.column_partial = partial;
     const int code = rc(gbdic::launch_tc_gemm(a, as_stream(stream)),
                         "ReLU-masked data gradient (rows and K of the convolution, Cout % 8, ldd % 8, k_split 1)");
-    if (code != GBDIC_OK) return code;
+    if (code != GBDIC_OK || !db) return code;
     return rc(gbdic::launch_nn_bias_reduce(partial, d->M / 128, d->N, db, as_stream(stream)), "bias gradient");
 }
 
 int gbdic_nn_conv_wgrad(const gbdic_nn_conv_shape *s, const void *x, const void *dz, int32_t splits, float *partial,
                         float *dw, int32_t *device_error, void *stream) {
-    if (!valid_shape(s) || !x || !dz || !partial || !dw) return invalid("weight-gradient arguments are incomplete");
+    if (!valid_shape(s) || !x || !dz || !partial) return invalid("weight-gradient arguments are incomplete");
     gbdic::TcWgradArgs a{shape_of(s), x, dz, partial, splits, s->Kp, device_error};
     const int code = rc(gbdic::launch_tc_wgrad(a, as_stream(stream)),
                         "weight gradient (C % 8 and Cout % 64, or Kp 64 and Cout 32; B*OH*OW % (64 splits), aligned)");
-    if (code != GBDIC_OK) return code;
+    if (code != GBDIC_OK || !dw) return code;
     return rc(gbdic::launch_nn_splitk_reduce(partial, splits, s->Kp, s->Cout, s->Kp, dw, as_stream(stream)),
               "split-K reduction");
 }
@@ -180,8 +180,23 @@ int gbdic_nn_adam(float *param, const float *grad, float *m, float *v, int64_t c
     return rc(gbdic::launch_nn_adam(a, as_stream(stream)), "Adam");
 }
 
+int gbdic_nn_reduce_many(const gbdic_nn_reduction *jobs, int32_t count, void *stream) {
+    if (!jobs || count < 1 || count > gbdic::kMaxReduceJobs) return invalid("invalid reductions (1 to 16)");
+    gbdic::NnReduceMany a{};
+    a.n = count;
+    for (int j = 0; j < count; ++j)
+        a.job[j] = {jobs[j].partial, jobs[j].out, jobs[j].splits, jobs[j].rows, jobs[j].cols, 0};
+    return rc(gbdic::launch_nn_reduce_many(a, as_stream(stream)), "reductions");
+}
+
 int gbdic_nn_adam_many(float *const *params, const float *const *grads, float *const *m, float *const *v,
                        const int64_t *counts, int32_t tensors, const float *hyper, void *stream) {
+    return gbdic_nn_adam_pack_many(params, grads, m, v, counts, tensors, hyper, nullptr, stream);
+}
+
+int gbdic_nn_adam_pack_many(float *const *params, const float *const *grads, float *const *m, float *const *v,
+                            const int64_t *counts, int32_t tensors, const float *hyper,
+                            const gbdic_nn_pack_target *pack, void *stream) {
     if (!params || !grads || !m || !v || !counts || !hyper || tensors < 1 || tensors > gbdic::kMaxAdamTensors)
         return invalid("invalid Adam arguments (1 to 16 tensors)");
     gbdic::NnAdamMany a{};
@@ -191,6 +206,13 @@ int gbdic_nn_adam_many(float *const *params, const float *const *grads, float *c
         if (!params[t] || !grads[t] || !m[t] || !v[t] || counts[t] < 0) return invalid("invalid Adam tensor");
         a.param[t] = params[t]; a.grad[t] = grads[t]; a.m[t] = m[t]; a.v[t] = v[t];
         a.offset[t + 1] = a.offset[t] + counts[t];
+        if (pack && pack[t].wb) {
+            const gbdic_nn_pack_target &p = pack[t];
+            if (p.cout < 1 || p.kp < 1 || (int64_t)p.cout * p.kp != counts[t] ||
+                (p.wt && (p.transposed ? p.kt < p.cout : p.cin < 1 || p.kp < 9 * p.cin || p.kt < 9 * p.cout)))
+                return invalid("invalid packing of an Adam tensor");
+            a.pack[t] = {p.wb, p.wt, p.cout, p.cin, p.kp, p.kt, p.transposed};
+        }
     }
     a.lr = hyper[0]; a.beta1 = hyper[1]; a.beta2 = hyper[2]; a.eps = hyper[3];
     a.bias1 = hyper[4]; a.bias2 = hyper[5]; a.weight_decay = hyper[6];

@@ -389,24 +389,27 @@ __global__ void __launch_bounds__(256) im2col_t_kernel(NnConvShape s, const __nv
 // out[n][k] = sum_s partial[s][k][n] (s ascending) for k < Kp, n < N.
 // Consecutive threads take consecutive n (contiguous partial reads); the
 // loads of four splits are issued before their ordered additions.
-__global__ void splitk_reduce_kernel(const float *partial, int splits, int Kp_rows, int N, int Kp, float *out) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= N * Kp) return;
-    const int k = idx / N, n = idx - k * N;
-    const size_t stride = (size_t)Kp_rows * N;
-    const float *p = partial + (size_t)k * N + n;
+// p[0] + p[stride] + ... in that order, 32 loads in flight.
+__device__ __forceinline__ float ordered_sum(const float *p, int count, size_t stride) {
     float acc = 0.0f;
     int s = 0;
-    for (; s + 32 <= splits; s += 32) {  // loads in flight together, added in split order
+    for (; s + 32 <= count; s += 32) {
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __ldg(p + (s + j) * stride);
 #pragma unroll
         for (int j = 0; j < 32; ++j) acc += v[j];
     }
-#pragma unroll 4
-    for (; s < splits; ++s) acc += __ldg(p + s * stride);
-    out[(size_t)n * Kp + k] = acc;
+#pragma unroll 8
+    for (; s < count; ++s) acc += __ldg(p + s * stride);
+    return acc;
+}
+
+__global__ void splitk_reduce_kernel(const float *partial, int splits, int Kp_rows, int N, int Kp, float *out) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= N * Kp) return;
+    const int k = idx / N, n = idx - k * N;
+    out[(size_t)n * Kp + k] = ordered_sum(partial + (size_t)k * N + n, splits, (size_t)Kp_rows * N);
 }
 
 // One Adam element update (shared by both kernels so that they compile to
@@ -429,8 +432,50 @@ __global__ void adam_many_kernel(NnAdamMany a) {
     if (i >= a.offset[a.n]) return;
     int t = 0;
     while (i >= a.offset[t + 1]) ++t;
-    adam_element(a.param[t], a.grad[t], a.m[t], a.v[t], i - a.offset[t], a.lr, a.beta1, a.beta2, a.eps, a.bias1,
-                 a.bias2, a.weight_decay);
+    const long long e = i - a.offset[t];
+    adam_element(a.param[t], a.grad[t], a.m[t], a.v[t], e, a.lr, a.beta1, a.beta2, a.eps, a.bias1, a.bias2,
+                 a.weight_decay);
+    const NnPackInto &p = a.pack[t];
+    if (p.wb == nullptr) return;
+    // the next step's BF16 operands, as pack_weights_kernel and a transpose
+    // write them, while the weight is at hand
+    const __nv_bfloat16 v = __float2bfloat16(a.param[t][e]);
+    const int co = (int)(e / p.kp), k = (int)(e - (long long)co * p.kp);
+    static_cast<__nv_bfloat16 *>(p.wb)[e] = v;
+    if (p.wt == nullptr) return;
+    if (p.transposed) {
+        static_cast<__nv_bfloat16 *>(p.wt)[(size_t)k * p.kt + co] = v;
+    } else if (k < 9 * p.cin) {
+        const int tap = k / p.cin, ci = k - tap * p.cin;
+        static_cast<__nv_bfloat16 *>(p.wt)[(size_t)ci * p.kt + tap * p.cout + co] = v;
+    }
+}
+
+// The reductions that end a backward pass, in one launch: each alone is a few
+// blocks whose threads' chains of loads are its time (batch 512: eleven
+// launches, 36 us and the gaps between them; together 16 us).  Splits are
+// added in their order, as splitk_reduce_kernel adds them.
+__global__ void __launch_bounds__(256) reduce_many_kernel(NnReduceMany a) {
+    int j = 0;
+    while (j + 1 < a.n && (int)blockIdx.x >= a.job[j + 1].first_block) ++j;
+    const NnReduceJob &job = a.job[j];
+    const int local = (int)blockIdx.x - job.first_block, tid = threadIdx.x;
+    __shared__ float part[256];
+    float acc = 0.0f;
+    if (job.cols > 0) {
+        const int o = local * 256 + tid, k = o / job.cols, n = o - k * job.cols;
+        if (k < job.rows) job.out[(size_t)n * job.rows + k] = ordered_sum(job.partial + o, job.splits, (size_t)job.rows * job.cols);
+        return;
+    }
+#pragma unroll 8
+    for (int s = tid; s < job.splits; s += 256) acc += __ldg(job.partial + (size_t)local * job.splits + s);
+    part[tid] = acc;
+    __syncthreads();
+    for (int off = 128; off > 0; off >>= 1) {
+        if (tid < off) part[tid] += part[tid + off];
+        __syncthreads();
+    }
+    if (tid == 0) job.out[local] = part[0];
 }
 
 __global__ void adam_kernel(NnAdamArgs a) {
@@ -939,6 +984,22 @@ cudaError_t launch_nn_im2col_t(const NnConvShape &sh, const void *x, void *At, i
 cudaError_t launch_nn_splitk_reduce(const float *partial, int splits, int Kp_rows, int N, int Kp, float *out,
                                     cudaStream_t s) {
     splitk_reduce_kernel<<<blocks((long long)N * Kp, 256), 256, 0, s>>>(partial, splits, Kp_rows, N, Kp, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_nn_reduce_many(const NnReduceMany &jobs, cudaStream_t s) {
+    if (jobs.n < 1 || jobs.n > kMaxReduceJobs) return cudaErrorInvalidValue;
+    NnReduceMany a = jobs;
+    long long total = 0;
+    for (int j = 0; j < a.n; ++j) {
+        NnReduceJob &job = a.job[j];
+        if (!job.partial || !job.out || job.splits < 1 || job.rows < 1 || job.cols < 0) return cudaErrorInvalidValue;
+        job.first_block = (int)total;
+        const long long outputs = (long long)job.rows * job.cols;
+        total += job.cols > 0 ? (outputs + 255) / 256 : job.rows;
+        if (outputs >= (1ll << 31) || total >= (1ll << 31)) return cudaErrorInvalidValue;
+    }
+    reduce_many_kernel<<<(unsigned)total, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -148,6 +148,16 @@ class NnGemmDesc(C.Structure):
     ]
 
 
+class NnPackTarget(C.Structure):
+    _fields_ = [("wb", C.c_void_p), ("wt", C.c_void_p), ("cout", C.c_int32), ("cin", C.c_int32), ("kp", C.c_int32),
+                ("kt", C.c_int32), ("transposed", C.c_int32)]
+
+
+class NnReduction(C.Structure):
+    _fields_ = [("partial", C.c_void_p), ("out", C.c_void_p), ("splits", C.c_int32), ("rows", C.c_int32),
+                ("cols", C.c_int32)]
+
+
 class NnConvShape(C.Structure):
     _fields_ = [(name, C.c_int32) for name in ("B", "H", "W", "C", "OH", "OW", "Cout", "Kp")]
 
@@ -221,6 +231,8 @@ _SIGNATURES = {
     "gbdic_nn_splitk_reduce": (C.c_int, [P, I32, I32, I32, I32, P, P]),
     "gbdic_nn_adam": (C.c_int, [P, P, P, P, I64, P, P]),
     "gbdic_nn_adam_many": (C.c_int, [P, P, P, P, P, I32, P, P]),
+    "gbdic_nn_adam_pack_many": (C.c_int, [P, P, P, P, P, I32, P, C.POINTER(NnPackTarget), P]),
+    "gbdic_nn_reduce_many": (C.c_int, [C.POINTER(NnReduction), I32, P]),
     "gbdic_nn_pack_weights": (C.c_int, [P, I32, I32, I32, P, P, I32, P]),
     "gbdic_nn_regression_loss": (C.c_int, [P, I32, P, I32, I32, P, P, I32, P, P]),
     "gbdic_reduce_half": (C.c_int, [P, I32, I32, P, P]),

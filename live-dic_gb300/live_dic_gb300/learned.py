@@ -248,6 +248,13 @@ class SeedNet:
         bufs["splits"] = [self._splits(c) for c in self.convs]
         bufs["partial"] = [torch.zeros(s, c.kp, c.cout, dtype=f32, device=dev)
                            for s, c in zip(bufs["splits"], self.convs, strict=True)]
+        nconv = len(self.convs)
+        jobs = [(bufs["partial"][i], self.grads[i], bufs["splits"][i], c.kp, c.cout) for i, c in enumerate(self.convs)]
+        jobs += [(bufs["db_partial"][i], self.grads[nconv + i], c.M // 128, c.cout, 0)
+                 for i, c in enumerate(self.convs[:-1])]
+        jobs.append((bufs["dw6T"], self.grads[2 * nconv], 1, self.features, OUT_PAD))
+        bufs["reductions"] = (_native.NnReduction * len(jobs))(
+            *[(p.data_ptr(), g.data_ptr(), s, rows, cols) for p, g, s, rows, cols in jobs])
         return bufs
 
     @staticmethod
@@ -290,7 +297,6 @@ class SeedNet:
         _call(lib, "gbdic_nn_transpose", _ptr(self.y[-1]), B, F, F, _ptr(b["y5T"]), B, F, stream)
         _call(lib, "gbdic_nn_transpose", _ptr(b["dout"]), B, OUT_PAD, LOSS_PAD, _ptr(b["doutT"]), B, OUT_PAD, stream)
         self._gemm(b["y5T"], b["doutT"], F, OUT_PAD, B, d_f32=b["dw6T"], stream=stream)
-        _call(lib, "gbdic_nn_splitk_reduce", _ptr(b["dw6T"]), 1, F, OUT_PAD, F, _ptr(self.grads[2 * nconv]), stream)
         _call(lib, "gbdic_nn_bias_grad", _ptr(b["dout_f32"]), LOSS_PAD, None, B, OUT_PAD,
               _ptr(self.grads[2 * nconv + 1]), stream)
         self._gemm(b["dout"], self.w6t, B, F, LOSS_PAD, d_f32=b["dy"], stream=stream)
@@ -304,14 +310,16 @@ class SeedNet:
             # (the 2-channel input layer: from the forward's im2col matrix)
             x = self.a[0] if i == 0 else self.y[i - 1]
             _call(lib, "gbdic_nn_conv_wgrad", C.byref(self._shape(i)), _ptr(x), _ptr(dz), b["splits"][i],
-                  _ptr(b["partial"][i]), _ptr(self.grads[i]), _ptr(self.err), stream)
+                  _ptr(b["partial"][i]), None, _ptr(self.err), stream)
             if i > 0:
                 # data gradient, gathered from dZ in the kernel (implicit GEMM),
                 # with the layer below's ReLU backward and bias gradient
                 desc = _native.NnGemmDesc(dz.data_ptr(), self.wt[i].data_ptr(), c.Min, c.cin, c.kt, 1, None,
                                           b["dz"][i - 1].data_ptr(), c.cin, 0, None, 0, 0)
                 _call(lib, "gbdic_nn_conv_dgrad_relu", C.byref(desc), C.byref(self._shape(i)), _ptr(self.y[i - 1]),
-                      _ptr(b["db_partial"][i - 1]), _ptr(self.grads[nconv + i - 1]), _ptr(self.err), stream)
+                      _ptr(b["db_partial"][i - 1]), None, _ptr(self.err), stream)
+        # every layer's partial results, and dW6^T transposed, in one launch
+        _call(lib, "gbdic_nn_reduce_many", b["reductions"], len(b["reductions"]), stream)
 
     def adam_step(self, lr: float = 1e-3, *, beta1: float = 0.9, beta2: float = 0.999, eps: float = 1e-8,
                   weight_decay: float = 0.0, stream=None) -> None:
@@ -323,11 +331,20 @@ class SeedNet:
             ptrs = (C.c_void_p * n)
             self._adam_tables = (ptrs(*[p.data_ptr() for p in self.params]), ptrs(*[g.data_ptr() for g in self.grads]),
                                  ptrs(*[m.data_ptr() for m in self.m]), ptrs(*[v.data_ptr() for v in self.v]),
-                                 (C.c_int64 * n)(*[p.numel() for p in self.params]), n)
-        params, grads, ms, vs, counts, n = self._adam_tables
-        # every parameter tensor in one launch, per element gbdic_nn_adam's update
-        _call(self.lib, "gbdic_nn_adam_many", params, grads, ms, vs, counts, n, hyper, stream)
-        self.pack(stream)
+                                 (C.c_int64 * n)(*[p.numel() for p in self.params]), n,
+                                 (_native.NnPackTarget * n)(*self._pack_targets()))
+        params, grads, ms, vs, counts, n, targets = self._adam_tables
+        # every parameter tensor in one launch, per element gbdic_nn_adam's
+        # update, and the BF16 operands of the updated weights as pack() writes them
+        _call(self.lib, "gbdic_nn_adam_pack_many", params, grads, ms, vs, counts, n, hyper, targets, stream)
+
+    def _pack_targets(self) -> list[tuple]:
+        """Per parameter tensor (order of self.params) the operands of pack()."""
+        targets: list[tuple] = [(wb.data_ptr(), wt.data_ptr(), c.cout, c.cin, c.kp, c.kt, 0)
+                                for c, wb, wt in zip(self.convs, self.wb, self.wt, strict=True)]
+        targets += [(None, None, 0, 0, 0, 0, 0)] * len(self.b)
+        targets.append((self.w6b.data_ptr(), self.w6t.data_ptr(), OUT_PAD, 1, self.features, LOSS_PAD, 1))
+        return [*targets, (None, None, 0, 0, 0, 0, 0)]
 
     def check_device_errors(self) -> None:
         if int(self.err.item()) != 0:

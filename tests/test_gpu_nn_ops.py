@@ -99,3 +99,44 @@ def test_adam_many_equals_per_tensor_steps():
     torch.cuda.synchronize()
     for a, b in zip(params + ms + vs, copies[0] + copies[2] + copies[3], strict=True):
         assert torch.equal(a, b)
+
+
+def test_reductions_in_one_launch():
+    """Split-K partials of few and many splits and column sums in one launch,
+    each against float64 sums (fewer than 300 additions in a chain)."""
+    lib = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    jobs, want, outs = [], [], []
+    for splits, rows, cols in ((1, 256, 16), (8, 320, 64), (33, 64, 32), (256, 64, 32), (7, 3, 5), (4096, 32, 0),
+                               (1, 128, 0), (300, 1, 0)):
+        p = torch.randn((splits, rows, cols) if cols else (rows, splits), generator=g, device="cuda")
+        out = torch.full((max(cols, 1) * rows,), 7.0, device="cuda")
+        jobs.append(_native.NnReduction(p.data_ptr(), out.data_ptr(), splits, rows, cols))
+        d = p.double()
+        want.append((d.sum(0).T.reshape(-1), d.abs().sum(0).T.reshape(-1)) if cols else (d.sum(1), d.abs().sum(1)))
+        outs.append((out, p))
+    table = (_native.NnReduction * len(jobs))(*jobs)
+    _native.check(lib.gbdic_nn_reduce_many(table, len(jobs), None), lib.gbdic_last_error(None))
+    torch.cuda.synchronize()
+    for (out, _), (exact, magnitude) in zip(outs, want, strict=True):
+        assert bool(((out.double() - exact).abs() <= 300 * 2.0 ** -24 * magnitude).all())
+
+
+def test_adam_writes_the_packed_operands():
+    """Weights updated and packed in one launch equal pack() of the update."""
+    from live_dic_gb300.learned import SeedNet
+
+    net, twin = SeedNet(128, seed=3), SeedNet(128, seed=3)
+    for a, b in zip(net.grads, twin.grads, strict=True):
+        a.normal_()
+        b.copy_(a)
+    for _ in range(2):
+        net.adam_step(1e-2)
+        twin.adam_step(1e-2)
+        for p in [*twin.wb, *twin.wt, twin.w6b, twin.w6t]:
+            p.fill_(0.0)
+        twin.pack()
+    torch.cuda.synchronize()
+    for a, b in zip([*net.params, *net.wb, *net.wt, net.w6b, net.w6t],
+                    [*twin.params, *twin.wb, *twin.wt, twin.w6b, twin.w6t], strict=True):
+        assert torch.equal(a, b)
