@@ -6,30 +6,35 @@
 // D is FP32 and/or BF16 with row stride ldd.  M is a multiple of 128, N of
 // the tile width BN, K (per split) of 64; callers pad.
 //
-// One CTA per 128 x BN output tile (x one K split), 128 threads:
-//   * thread 0 of warp 0 issues TMA loads of 128x64 A and BNx64 B tiles
-//     (128-byte swizzle) into a 4-stage shared-memory ring, each stage
-//     guarded by a full/empty mbarrier pair;
-//   * thread 0 of warp 1 issues tcgen05.mma (M=128, N=BN, K=16, FP32
-//     accumulator in tensor memory), four per 64-wide stage, and releases
-//     each stage with tcgen05.commit on its empty barrier;
-//   * after the last commit all four warps read their 32 accumulator lanes
-//     with tcgen05.ld and apply the epilogue.
-// Convolution GEMMs can gather operand A in the kernel (implicit GEMM):
-// the CTA then has 64 + 32 kGatherWarps threads, and warps 2 and up fill
-// each stage's A tile with 16-byte cp.async copies
-// straight from the NHWC tensor (an im2col row of the forward, or the
-// data-gradient gather of the output gradient; zero-filled outside the
-// image), at the positions the 128-byte swizzle gives them, from a table of
-// the tile's 128 row origins built once per CTA; each thread's arrival on the
-// stage's full barrier follows its copies, and the MMA issuer fences them to
-// the async proxy that tcgen05.mma reads through; TMA still loads B.  The 9x-expanded im2col matrix is never
+// Persistent CTAs, up to two to an SM, walk the 128 x BN output tiles (x K
+// splits).  A CTA's warps have roles that run ahead of each other:
+//   * one thread issues TMA loads of 128x64 A and BNx64 B tiles (128-byte
+//     swizzle) into a shared-memory ring, each stage guarded by a full/empty
+//     mbarrier pair;
+//   * one thread issues tcgen05.mma (M=128, N=BN, K=16, FP32 accumulator in
+//     tensor memory), four per 64-wide stage, releases each stage with
+//     tcgen05.commit on its empty barrier, and alternates between two
+//     accumulators, so that a tile's MMAs run during the last one's epilogue;
+//   * four warps read a finished accumulator's lanes with tcgen05.ld, apply the
+//     epilogue and release it.
+// Convolution GEMMs can gather operand A in the kernel (implicit GEMM): eight
+// more warps fill each stage's A tile with 16-byte cp.async copies straight
+// from the NHWC tensor (an im2col row of the forward, or the data-gradient
+// gather of the output gradient; zero-filled outside the image), at the
+// positions the 128-byte swizzle gives them, from a table of the tile's 128 row
+// origins; each thread's arrival on the stage's full barrier follows its
+// copies, and the MMA issuer fences them to the async proxy that tcgen05.mma
+// reads through; TMA still loads B.  The 9x-expanded im2col matrix is never
 // written or read.  The data-gradient GEMM orders its rows by the input
 // pixel's stride-2 parity class and skips the K blocks of the taps that are
-// zero for the tile's class (9 of the 36 class-tap pairs remain).  The
-// ring has min(4, K blocks) stages (2 to 4 in gather mode, as many as leave
-// every CTA of the launch resident), so short K loops and launches of many
-// gathering CTAs need little shared memory.
+// zero for the tile's class (9 of the 36 class-tap pairs remain).
+// What bounds these shapes (K loops of 1 to 18 blocks) is not the tensor cores
+// but the bytes: 3 to 5 TB/s of gathers from L2, activations and results.
+// Batch 512, before (a CTA per tile, its start,
+// loop and epilogue one after the other) -> here: data gradient 32 channels
+// (4,096 tiles of 1 to 4 K blocks, masked) 72 -> 48 us, 64 channels 37 -> 24;
+// forward 2 -> 32 channels (4,096 tiles of one) 46 -> 21, 32 -> 64 34 -> 22,
+// 128 -> 64 at 2 x 2 (16 tiles of 18) 15 -> 14.
 // Every mbarrier wait is bounded: on expiry the CTA records an error code and
 // carries on, so a fault of the pipeline ends the kernel instead of hanging.
 // Before a failed CTA frees its tensor memory and exits, it waits (bounded
@@ -47,16 +52,16 @@ namespace gbdic {
 namespace {
 
 #ifndef GBDIC_GEMM_STAGES
-#define GBDIC_GEMM_STAGES 4
+#define GBDIC_GEMM_STAGES 6
 #endif
 #ifndef GBDIC_GATHER_WARPS
 #define GBDIC_GATHER_WARPS 8
 #endif
 constexpr int kStages = GBDIC_GEMM_STAGES;
-// Gather mode: warps 2 .. 2 + kGatherWarps - 1 fill operand A.
+// Warps that fill a gathered operand A.
 constexpr int kGatherWarps = GBDIC_GATHER_WARPS;
 constexpr int kGatherThreads = 32 * kGatherWarps;
-constexpr int kMaxThreads = 64 + kGatherThreads;
+constexpr int kMaxThreads = 64 + kGatherThreads;  // of the weight gradient's CTAs
 static_assert(kGatherWarps == 2 || kGatherWarps == 4 || kGatherWarps == 8, "1024 chunks per stage split evenly");
 // Weight gradient: stages of 64 pixels.
 constexpr int kWgradStages = 3;
@@ -92,6 +97,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
         if (done) return true;
     }
     return false;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // Arrives (one of the barrier's expected count) once this thread's cp.async
@@ -222,36 +231,38 @@ __host__ __device__ constexpr uint32_t instr_desc(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// The bound on registers lets as many CTAs be resident as a ring of two stages
-// leaves room for.
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+    __syncwarp();
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Warps of a CTA: 0 .. 3 epilogue (the quarter of tensor memory a warp may read
+// goes by its index), then the gatherers, the TMA producer, the MMA issuer.
+constexpr int kGatherWarp0 = 4, kTmaWarp = kGatherWarp0 + kGatherWarps, kMmaWarp = kTmaWarp + 1;
+constexpr int kGemmThreads = 32 * (kMmaWarp + 1);
+
 template <int BN>
-__global__ void __launch_bounds__(kMaxThreads, BN <= 64 ? 4 : 3) tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                         const __grid_constant__ CUtensorMap map_b,
-                                                         TcGemmArgs args) {
+__global__ void __launch_bounds__(kGemmThreads, 2) tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a,
+                                                                  const __grid_constant__ CUtensorMap map_b,
+                                                                  TcGemmArgs args) {
     constexpr uint32_t kBytesA = kBM * kBK * 2;
     constexpr uint32_t kBytesB = BN * kBK * 2;
     constexpr uint32_t kStageBytes = kBytesA + kBytesB;
-    constexpr uint32_t kTmemCols = BN < 32 ? 32 : BN;
+    constexpr uint32_t kAccCols = BN < 32 ? 32 : BN;  // columns of one of the two accumulators
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t full_bar[kStages], empty_bar[kStages], done_bar;
+    __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[2], acc_empty[2], done_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int failed;
     __shared__ int issued_kb, consumed_kb;  // K blocks whose loads were issued / consumed
-    __shared__ int2 row_tab[kBM];           // gather mode: descriptors of the tile's rows
+    __shared__ int2 row_tab[2][kBM];        // gather mode: descriptors of the tile's rows
+    __shared__ float column_sum[2][4][BN];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int n0 = blockIdx.x * BN, m0 = blockIdx.y * kBM;
-    const int k_len = args.K / args.k_split;
-    const int k_begin = blockIdx.z * k_len;
-    const int cls = gather_class(args, m0);
-    const int num_kb = kblock_count(args, k_len, cls);
-    // The ring holds min(4, K blocks) stages (launch_bn sizes the dynamic
-    // shared memory the same way), so short K loops leave room for more
-    // resident CTAs.
-    const int nst = num_kb < args.ring ? num_kb : args.ring;
+    const int n_tiles = args.N / BN, m_tiles = args.M / kBM, k_len = args.K / args.k_split;
+    const int tiles = n_tiles * m_tiles * args.k_split;
+    const int nst = args.ring;
 
-    if (args.gather && tid < kBM) row_tab[tid] = gather_row(args, m0 + tid, cls);
     if (tid == 0) {
         // Full barriers: the TMA producer's arrive (with the stage's bytes),
         // plus one arrive per gathering thread in gather mode.
@@ -259,6 +270,10 @@ __global__ void __launch_bounds__(kMaxThreads, BN <= 64 ? 4 : 3) tc_gemm_kernel(
         for (int s = 0; s < nst; ++s) {
             mbar_init(&full_bar[s], full_count);
             mbar_init(&empty_bar[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(&acc_full[a], 1);
+            mbar_init(&acc_empty[a], 4);
         }
         mbar_init(&done_bar, 1);
         failed = 0;
@@ -268,7 +283,7 @@ __global__ void __launch_bounds__(kMaxThreads, BN <= 64 ? 4 : 3) tc_gemm_kernel(
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(kTmemCols));
+                     "r"(2 * kAccCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -276,59 +291,83 @@ __global__ void __launch_bounds__(kMaxThreads, BN <= 64 ? 4 : 3) tc_gemm_kernel(
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
 
-    if (warp == 0 && lane == 0) {
-        // TMA producer.
-        int kb = 0;
-        for (; kb < num_kb; ++kb) {
-            const int s = kb % nst;
-            if (kb >= nst && !mbar_wait(&empty_bar[s], ((kb / nst) - 1) & 1)) {
-                atomicExch(&failed, 1);
-                break;
+    // Every role walks the CTA's tiles in the same order (n fastest, then m,
+    // then the K split); K blocks are numbered through all of them, block g in
+    // stage g % nst.  A role whose wait expires sets `failed` and takes no
+    // further part, but goes on to meet the named barriers of its group.
+    if (warp == kTmaWarp && lane == 0) {
+        int g = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+            const int r = t / n_tiles, z = r / m_tiles;
+            const int n0 = (t - r * n_tiles) * BN, m0 = (r - z * m_tiles) * kBM, k_begin = z * k_len;
+            const int cls = gather_class(args, m0), num_kb = kblock_count(args, k_len, cls);
+            for (int kb = 0; kb < num_kb; ++kb, ++g) {
+                const int s = g % nst;
+                if (g >= nst && !mbar_wait(&empty_bar[s], ((g / nst) - 1) & 1)) {
+                    atomicExch(&failed, 1);
+                    ok = false;
+                    break;
+                }
+                uint8_t *sa = smem + s * kStageBytes;
+                uint8_t *sb = sa + kBytesA;
+                mbar_expect_tx(&full_bar[s], args.gather ? kBytesB : kStageBytes);
+                const int kx = kblock_offset(args, kb, k_begin, cls);
+                if (!args.gather) tma_load_2d(sa, &map_a, &full_bar[s], kx, m0);
+                tma_load_2d(sb, &map_b, &full_bar[s], kx, n0);
             }
-            uint8_t *sa = smem + s * kStageBytes;
-            uint8_t *sb = sa + kBytesA;
-            mbar_expect_tx(&full_bar[s], args.gather ? kBytesB : kStageBytes);
-            const int kx = kblock_offset(args, kb, k_begin, cls);
-            if (!args.gather) tma_load_2d(sa, &map_a, &full_bar[s], kx, m0);
-            tma_load_2d(sb, &map_b, &full_bar[s], kx, n0);
         }
-        issued_kb = kb;
-    } else if (warp == 1 && lane == 0) {
-        // MMA issuer.
+        issued_kb = g;
+    } else if (warp == kMmaWarp && lane == 0) {
         constexpr uint32_t idesc = instr_desc(kBM, BN);
-        int kb = 0;
-        for (; kb < num_kb; ++kb) {
-            const int s = kb % nst;
-            if (!mbar_wait(&full_bar[s], (kb / nst) & 1)) {
+        int g = 0, i = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++i) {
+            const int m0 = (t / n_tiles) % m_tiles * kBM;
+            const int num_kb = kblock_count(args, k_len, gather_class(args, m0));
+            const int acc = i & 1;
+            if (i >= 2 && !mbar_wait(&acc_empty[acc], ((i >> 1) - 1) & 1)) {
                 atomicExch(&failed, 1);
                 break;
             }
-            // gathered bytes (generic proxy) before the MMA's reads (async proxy)
-            if (args.gather) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
-            const uint32_t b_addr = a_addr + kBytesA;
+            for (int kb = 0; kb < num_kb; ++kb, ++g) {
+                const int s = g % nst;
+                if (!mbar_wait(&full_bar[s], (g / nst) & 1)) {
+                    atomicExch(&failed, 1);
+                    ok = false;
+                    break;
+                }
+                // gathered bytes (generic proxy) before the MMA's reads (async proxy)
+                if (args.gather) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
+                const uint32_t b_addr = a_addr + kBytesA;
 #pragma unroll
-            for (int kk = 0; kk < kBK / 16; ++kk) {
-                const uint64_t da = smem_desc(a_addr + kk * 32);
-                const uint64_t db = smem_desc(b_addr + kk * 32);
-                const uint32_t accumulate = (kb > 0 || kk > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                    "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+                for (int kk = 0; kk < kBK / 16; ++kk) {
+                    const uint64_t da = smem_desc(a_addr + kk * 32);
+                    const uint64_t db = smem_desc(b_addr + kk * 32);
+                    const uint32_t accumulate = (kb > 0 || kk > 0) ? 1u : 0u;
+                    asm volatile(
+                        "{\n\t.reg .pred p;\n\t"
+                        "setp.ne.b32 p, %4, 0;\n\t"
+                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem + acc * kAccCols),
+                        "l"(da), "l"(db), "r"(idesc), "r"(accumulate));
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 smem_u32(&empty_bar[s]))
+                             : "memory");
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&empty_bar[s]))
-                         : "memory");
+            if (ok)
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                                 smem_u32(&acc_full[acc]))
+                             : "memory");
         }
-        consumed_kb = kb;
+        consumed_kb = g;
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                          smem_u32(&done_bar))
                      : "memory");
-    }
-    if (args.gather && warp >= 2) {
+    } else if (args.gather && warp >= kGatherWarp0 && warp < kTmaWarp) {
         // Operand A producers: kGatherThreads threads, thread g copies chunk
         // j = g % 8 of rows g / 8 + (kGatherThreads / 8) i of the 128 x 64
         // tile, so eight threads read one row's 128 contiguous bytes (one
@@ -337,163 +376,211 @@ __global__ void __launch_bounds__(kMaxThreads, BN <= 64 ? 4 : 3) tc_gemm_kernel(
         // 1024-byte-aligned stage, the 128-byte swizzle of the TMA loads it
         // replaces.  Each thread's arrival on the stage's full barrier is left
         // to its copies, so the ring alone limits how far the gathering runs
-        // ahead.  (Waiting for each stage's copies and fencing them here, warp
-        // by warp, cost 1 us a K block whatever the ring's depth: the fence
-        // waits for the later stages' copies too.)
+        // ahead.  (Waiting for the oldest of three stages in flight and arriving
+        // warp by warp: the 32-channel data gradient 48 -> 51 us, the 32 -> 64
+        // channel weight gradient 26 -> 33.)
         constexpr int kRowStep = kGatherThreads / 8, kRowsPerThread = kBM / kRowStep;
-        const int g = tid - 64, j = g & 7, r0 = g >> 3;
-        const uint4 *src = static_cast<const uint4 *>(args.a);
-        int base[kRowsPerThread], mask[kRowsPerThread];
-#pragma unroll
-        for (int i = 0; i < kRowsPerThread; ++i) {
-            const int2 row = row_tab[r0 + kRowStep * i];
-            base[i] = row.x;
-            mask[i] = row.y;
-        }
-        const uint32_t place = (uint32_t)(r0 * 128 + ((j ^ (r0 & 7)) << 4));  // rows step by multiples of 8
         static_assert(kRowStep % 8 == 0, "a thread's rows share their swizzle phase");
-        // The chunk's tap and its chunk within the tap, advanced by 8 chunks a K
-        // block (class mode: over the class's taps).
+        const int gt = tid - 32 * kGatherWarp0, j = gt & 7, r0 = gt >> 3;
+        const uint4 *src = static_cast<const uint4 *>(args.a);
+        const uint32_t place = (uint32_t)(r0 * 128 + ((j ^ (r0 & 7)) << 4));  // rows step by multiples of 8
         const bool classes = args.gather == kGatherDgradClasses;
         const int per_tap = (args.gather == kGatherIm2col ? args.conv.C : args.conv.Cout) / 8;
-        const int q = kblock_offset(args, 0, k_begin, cls) / 8 + j;
-        const int kx_first = classes && !(cls & 1) ? 1 : 0, kx_step = classes ? 2 : 1;
-        const int ky_step = classes && (cls >> 1) ? 2 : 1;
-        int tap = q / per_tap, c8 = q - tap * per_tap, ky = tap / 3, kx = tap - 3 * ky;
-        int delta = gather_tap(args, ky, kx, cls);
-        for (int kb = 0; kb < num_kb; ++kb) {
-            const int s = kb % nst;
-            if (kb >= nst) {
-                int ok = 1;
-                if (lane == 0) ok = mbar_wait(&empty_bar[s], ((kb / nst) - 1) & 1) ? 1 : 0;
-                ok = __shfl_sync(0xffffffffu, ok, 0);
-                if (!ok) {
-                    if (lane == 0) atomicExch(&failed, 1);
-                    break;
-                }
-            }
-            const uint32_t dst = smem_u32(smem + s * kStageBytes) + place;
-            const int offset = delta + c8, bit = 3 * ky + kx;  // beyond the ninth tap (K padding): no bit is set
+        int g = 0, i = 0;
+        bool dead = false;
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
+            const int r = t / n_tiles, z = r / m_tiles;
+            const int m0 = (r - z * m_tiles) * kBM, k_begin = z * k_len;
+            const int cls = gather_class(args, m0), num_kb = kblock_count(args, k_len, cls);
+            // The tile's row descriptors; the other table is still being read
+            // at most by threads that have not passed this barrier.
+            if (gt < kBM) row_tab[i & 1][gt] = gather_row(args, m0 + gt, cls);
+            named_barrier(1, kGatherThreads);
+            if (dead) continue;
+            int base[kRowsPerThread], mask[kRowsPerThread];
 #pragma unroll
-            for (int i = 0; i < kRowsPerThread; ++i) {
-                const bool in = (mask[i] >> bit) & 1;
-                cp_async_16(dst + (uint32_t)(kRowStep * i * 128), src + (in ? base[i] + offset : 0), in ? 16u : 0u);
+            for (int k = 0; k < kRowsPerThread; ++k) {
+                const int2 row = row_tab[i & 1][r0 + kRowStep * k];
+                base[k] = row.x;
+                mask[k] = row.y;
             }
-            mbar_arrive_copies(&full_bar[s]);
-            c8 += 8;
-            if (c8 >= per_tap) {
-                do {
-                    c8 -= per_tap;
-                    kx += kx_step;
-                    if (kx > 2) {
-                        kx = kx_first;
-                        ky += ky_step;
+            // The chunk's tap and its chunk within the tap, advanced by 8 chunks a K
+            // block (class mode: over the class's taps).
+            const int q = kblock_offset(args, 0, k_begin, cls) / 8 + j;
+            const int kx_first = classes && !(cls & 1) ? 1 : 0, kx_step = classes ? 2 : 1;
+            const int ky_step = classes && (cls >> 1) ? 2 : 1;
+            int tap = q / per_tap, c8 = q - tap * per_tap, ky = tap / 3, kx = tap - 3 * ky;
+            int delta = gather_tap(args, ky, kx, cls);
+            for (int kb = 0; kb < num_kb; ++kb, ++g) {
+                const int s = g % nst;
+                if (g >= nst) {
+                    int ok = 1;
+                    if (lane == 0) ok = mbar_wait(&empty_bar[s], ((g / nst) - 1) & 1) ? 1 : 0;
+                    ok = __shfl_sync(0xffffffffu, ok, 0);
+                    if (!ok) {
+                        if (lane == 0) atomicExch(&failed, 1);
+                        dead = true;
+                        break;
                     }
-                } while (c8 >= per_tap);
-                delta = gather_tap(args, ky, kx, cls);
+                }
+                const uint32_t dst = smem_u32(smem + s * kStageBytes) + place;
+                const int offset = delta + c8, bit = 3 * ky + kx;  // beyond the ninth tap (K padding): no bit is set
+#pragma unroll
+                for (int k = 0; k < kRowsPerThread; ++k) {
+                    const bool in = (mask[k] >> bit) & 1;
+                    cp_async_16(dst + (uint32_t)(kRowStep * k * 128), src + (in ? base[k] + offset : 0), in ? 16u : 0u);
+                }
+                mbar_arrive_copies(&full_bar[s]);
+                c8 += 8;
+                if (c8 >= per_tap) {
+                    do {
+                        c8 -= per_tap;
+                        kx += kx_step;
+                        if (kx > 2) {
+                            kx = kx_first;
+                            ky += ky_step;
+                        }
+                    } while (c8 >= per_tap);
+                    delta = gather_tap(args, ky, kx, cls);
+                }
             }
         }
         // Drain: every issued copy lands before the warp moves on (also after
         // a failed wait, so no copy is left writing into shared memory).
         asm volatile("cp.async.wait_all;" ::: "memory");
-    }
-    __syncwarp();
-    // Epilogue: warp w < 4 owns accumulator lanes (rows) 32w .. 32w + 31.
-    __shared__ float column_sum[4][BN];
-    const int row = output_row(args, m0 + warp * 32 + lane, cls);
-    if (args.mask != nullptr && warp < 4) {
-        // the row's activations, on their way while the last MMAs finish
-        const char *m = reinterpret_cast<const char *>(static_cast<const __nv_bfloat16 *>(args.mask) +
-                                                       (size_t)row * args.ldd + n0);
+    } else if (warp < 4) {
+        // Epilogue: warp w owns accumulator lanes (rows) 32w .. 32w + 31.
+        const bool wide = args.ldd % 8 == 0 && (args.k_split == 1 || args.split_stride % 8 == 0) &&
+                          (reinterpret_cast<uintptr_t>(args.d_bf16) & 15) == 0;
+        int i = 0;
+        bool dead = false;
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
+            const int rest = t / n_tiles, z = rest / m_tiles, m_tile = rest - z * m_tiles;
+            const int n0 = (t - rest * n_tiles) * BN, m0 = m_tile * kBM, acc = i & 1;
+            const int row = output_row(args, m0 + warp * 32 + lane, gather_class(args, m0));
+            if (!dead) {
+                if (args.mask != nullptr) {
+                    // the row's activations, on their way while the last MMAs finish
+                    const char *m = reinterpret_cast<const char *>(static_cast<const __nv_bfloat16 *>(args.mask) +
+                                                                   (size_t)row * args.ldd + n0);
 #pragma unroll
-        for (int b = 0; b < 2 * BN; b += 64) asm volatile("prefetch.global.L1 [%0];" ::"l"(m + b));
-    }
-    if (!mbar_wait(&done_bar, 0)) atomicExch(&failed, 1);
-    __syncwarp();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+                    for (int b = 0; b < 2 * BN; b += 64) asm volatile("prefetch.global.L1 [%0];" ::"l"(m + b));
+                }
+                if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (i >> 1) & 1))) {
+                    if (lane == 0) atomicExch(&failed, 1);
+                    dead = true;
+                }
+            }
+            if (!dead) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t lane_base = tmem + acc * kAccCols + ((uint32_t)(warp * 32) << 16);
 #pragma unroll 1
-    for (int c = 0; c < (warp < 4 ? BN : 0); c += 16) {
-        uint32_t r[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-            "%14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(tmem + lane_base + (uint32_t)c));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        float v[16];
+                for (int c = 0; c < BN; c += 16) {
+                    uint32_t r[16];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                        "%14, %15}, [%16];"
+                        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                        : "r"(lane_base + (uint32_t)c));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float v[16];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-            v[j] = __uint_as_float(r[j]);
-            if (args.bias) v[j] = v[j] + args.bias[n0 + c + j];
-            if (args.relu) v[j] = fmaxf(v[j], 0.0f);
-        }
-        if (args.mask != nullptr) {
-            // ReLU backward where the row's activation is zero, and the sums
-            // over the warp's 32 rows: halves of the columns go to halves of
-            // the lanes, until lane pair l holds column l / 2.
-            const uint4 *m = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(args.mask) +
-                                                             (size_t)row * args.ldd + n0 + c);
-            const uint4 m0 = __ldg(m), m1 = __ldg(m + 1);
-            const uint32_t words[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+                    for (int j = 0; j < 16; ++j) {
+                        v[j] = __uint_as_float(r[j]);
+                        if (args.bias) v[j] = v[j] + args.bias[n0 + c + j];
+                        if (args.relu) v[j] = fmaxf(v[j], 0.0f);
+                    }
+                    if (args.mask != nullptr) {
+                        // ReLU backward where the row's activation is zero, and the sums
+                        // over the warp's 32 rows: halves of the columns go to halves of
+                        // the lanes, until lane pair l holds column l / 2.
+                        const uint4 *m = reinterpret_cast<const uint4 *>(static_cast<const __nv_bfloat16 *>(args.mask) +
+                                                                         (size_t)row * args.ldd + n0 + c);
+                        const uint4 m0 = __ldg(m), m1 = __ldg(m + 1);
+                        const uint32_t words[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const __nv_bfloat162 y = *reinterpret_cast<const __nv_bfloat162 *>(&words[j]);
-                if (!(__bfloat162float(y.x) > 0.0f)) v[2 * j] = 0.0f;
-                if (!(__bfloat162float(y.y) > 0.0f)) v[2 * j + 1] = 0.0f;
-            }
-            float t[16];
+                        for (int j = 0; j < 8; ++j) {
+                            const __nv_bfloat162 y = *reinterpret_cast<const __nv_bfloat162 *>(&words[j]);
+                            if (!(__bfloat162float(y.x) > 0.0f)) v[2 * j] = 0.0f;
+                            if (!(__bfloat162float(y.y) > 0.0f)) v[2 * j + 1] = 0.0f;
+                        }
+                        float t[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) t[j] = v[j];
+                        for (int j = 0; j < 16; ++j) t[j] = v[j];
 #pragma unroll
-            for (int half = 8; half >= 1; half >>= 1) {
-                const bool upper = lane & (2 * half);
+                        for (int half = 8; half >= 1; half >>= 1) {
+                            const bool upper = lane & (2 * half);
 #pragma unroll
-                for (int j = 0; j < half; ++j) {
-                    const float keep = upper ? t[j + half] : t[j], send = upper ? t[j] : t[j + half];
-                    t[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
+                            for (int j = 0; j < half; ++j) {
+                                const float keep = upper ? t[j + half] : t[j], send = upper ? t[j] : t[j + half];
+                                t[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
+                            }
+                        }
+                        t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
+                        if ((lane & 1) == 0) column_sum[acc][warp][c + (lane >> 1)] = t[0];
+                    }
+                    const size_t base = (size_t)z * (size_t)args.split_stride + (size_t)row * args.ldd + n0 + c;
+                    if (args.d_f32) {
+                        float4 *o = reinterpret_cast<float4 *>(args.d_f32 + base);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            float4 x = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                            if (args.accumulate) {
+                                const float4 y = o[j];
+                                x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+                            }
+                            o[j] = x;
+                        }
+                    }
+                    if (args.d_bf16) {
+                        // A store instruction per four bytes of a row touched 32 lines
+                        // for 128 bytes and was these kernels' time: 16-byte ones
+                        // where the rows allow it.
+                        uint32_t w[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                            w[j] = *reinterpret_cast<const uint32_t *>(&two);
+                        }
+                        __nv_bfloat16 *o = static_cast<__nv_bfloat16 *>(args.d_bf16) + base;
+                        if (wide) {
+                            reinterpret_cast<uint4 *>(o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+                            reinterpret_cast<uint4 *>(o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) reinterpret_cast<uint32_t *>(o)[j] = w[j];
+                        }
+                    }
                 }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[acc]);
             }
-            t[0] += __shfl_xor_sync(0xffffffffu, t[0], 1);
-            if ((lane & 1) == 0) column_sum[warp][c + (lane >> 1)] = t[0];
-        }
-        const size_t base = (size_t)blockIdx.z * (size_t)args.split_stride + (size_t)row * args.ldd + n0 + c;
-        if (args.d_f32) {
-            float4 *o = reinterpret_cast<float4 *>(args.d_f32 + base);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float4 x = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                if (args.accumulate) {
-                    const float4 y = o[j];
-                    x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-                }
-                o[j] = x;
+            if (args.mask != nullptr) {
+                named_barrier(2, 128);
+                if (!dead)
+                    for (int c = tid; c < BN; c += 128) {
+                        const float(*sum)[BN] = column_sum[acc];
+                        args.column_partial[(size_t)(n0 + c) * m_tiles + m_tile] =
+                            (sum[0][c] + sum[1][c]) + (sum[2][c] + sum[3][c]);
+                    }
             }
-        }
-        if (args.d_bf16) {
-            __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(static_cast<__nv_bfloat16 *>(args.d_bf16) + base);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
         }
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (args.mask != nullptr)
-        for (int c = tid; c < BN; c += blockDim.x)
-            args.column_partial[(size_t)(n0 + c) * gridDim.y + blockIdx.y] =
-                (column_sum[0][c] + column_sum[1][c]) + (column_sum[2][c] + column_sum[3][c]);
     if (warp == 0) {
         if (lane == 0 && failed) {
-            // The producer runs at most kStages K blocks ahead of the issuer,
+            // The producer runs at most nst K blocks ahead of the issuer,
             // so the unconsumed blocks occupy distinct stages.
             for (int kb = consumed_kb; kb < issued_kb; ++kb) mbar_wait(&full_bar[kb % nst], (kb / nst) & 1);
             mbar_wait(&done_bar, 0);
         }
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * kAccCols));
     }
     if (tid == 0 && failed && args.error) atomicExch(args.error, 1);
 }
@@ -731,29 +818,22 @@ bool make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int box_row
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Stages of the gathering ring.  A launch with more CTAs than fit at once hides
-// the copies' latency behind other CTAs, and a ring of two stages lets the most
-// of them be resident; one with fewer takes the deepest ring that still leaves
-// every CTA resident.  Batch 512, 16 CTAs of 18 K blocks (128 -> 64 channels at
-// 2 x 2): 26 us with two stages and a wait per stage, 20 with four and the
-// arrivals left to the copies, 15 with the taps stepped instead of divided out;
-// 64 CTAs of 18 (128 -> 128 at 4 x 4): 29 -> 24 -> 18.
-int gather_ring(long long ctas, size_t stage_bytes) {
-    const long long per_sm = (ctas + 151) / 152;
-    for (int ring = kStages; ring > 2; --ring)
-        if (per_sm * (long long)(ring * stage_bytes + 8192) <= 224 * 1024) return ring;
-    return 2;
-}
+// CTAs walk their tiles, two CTAs to an SM where there are tiles for them.  The
+// ring is as deep as their shared memory allows, whatever the length of a tile's
+// K loop: it runs on into the next tile, whose gathering and MMAs overlap this
+// one's epilogue.
+constexpr int kSms = 152;
+constexpr int kRingBytes = 216 * 1024;  // of an SM's 227 KB, beside the CTAs' static arrays
 
 template <int BN>
 cudaError_t launch_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemmArgs &args, cudaStream_t stream) {
     TcGemmArgs a = args;
-    const long long ctas = (long long)(a.N / BN) * (a.M / kBM) * a.k_split;
-    a.ring = a.gather ? gather_ring(ctas, kBM * kBK * 2 + BN * kBK * 2) : kStages;
-    const int num_kb = a.K / a.k_split / kBK;
-    const int nst = num_kb < a.ring ? num_kb : a.ring;
-    const size_t smem = (size_t)nst * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
-    const size_t smem_max = (size_t)kStages * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
+    constexpr int kStageBytes = kBM * kBK * 2 + BN * kBK * 2;
+    const long long tiles = (long long)(a.N / BN) * (a.M / kBM) * a.k_split;
+    const int per_sm = tiles > kSms ? 2 : 1;
+    a.ring = kRingBytes / per_sm / kStageBytes < kStages ? kRingBytes / per_sm / kStageBytes : kStages;
+    const size_t smem = (size_t)a.ring * kStageBytes + 1024;
+    const size_t smem_max = (size_t)kStages * kStageBytes + 1024;
     // The attribute is per device; set it once per device and tile width.
     static thread_local int configured_device = -1;
     int device = 0;
@@ -764,8 +844,8 @@ cudaError_t launch_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemm
         if (err != cudaSuccess) return err;
         configured_device = device;
     }
-    dim3 grid(a.N / BN, a.M / kBM, a.k_split);
-    tc_gemm_kernel<BN><<<grid, a.gather ? kMaxThreads : 128, smem, stream>>>(ma, mb, a);
+    const int grid = (int)(tiles < 2 * kSms ? tiles : 2 * kSms);
+    tc_gemm_kernel<BN><<<grid, kGemmThreads, smem, stream>>>(ma, mb, a);
     return cudaGetLastError();
 }
 
