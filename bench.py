@@ -416,7 +416,7 @@ def run_batch_workload(args) -> None:
         "tuning_ms": batch.tuning_ms or None,
         "clocks": {"sm_mhz": summary["sm_mhz"], "sm_max_mhz": summary["sm_max_mhz"], "reasons": summary["reasons"]},
         "gpu_launches": (2 * len(batch.jobs) + 1) * args.steps,
-        "roofline": {"bound": "fp32", "kernel": "icgn_batch_any_kernel (every job, shape function per job)",
+        "roofline": {"bound": "fp32", "kernel": "icgn_band_kernel / icgn_kernel (a launch per job, concurrent) or icgn_batch_any_kernel",
                      "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s", "frac": achieved / peak.value,
                      "solver_ms": solver_ms, "flops_per_step": flops, "traffic": None},
         "e2e": {"value": selected / e2e_s, "unit": "subsets/s",
@@ -538,7 +538,8 @@ def measure_quadratic(args, local: int, world: int, dist, *, steps: int, warmup:
         "accuracy_pair": "the last timed pair, against the FP64 sinusoid field",
         "clocks": clocks.line(),
         "gpu_launches": profile["launches"],
-        "roofline": {"bound": "fp32", "kernel": f"icgn_kernel<quadratic,bspline,{args.lanes} lanes>",
+        "roofline": {"bound": "fp32", "kernel": f"icgn_band_kernel<quadratic,{args.lanes} lanes>" if args.lanes <= 32
+                     else f"icgn_kernel<quadratic,bspline,{args.lanes} lanes>",
                      "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s",
                      "frac": None if achieved is None else achieved / peak.value,
                      "solver_ms_per_pair": profile["solver_ms"] / max(1, steps)},
@@ -895,7 +896,7 @@ def main() -> None:
         traffic = json.loads(traffic_file.read_text()).get("icgn_solver_dram_bytes_per_launch")
     roofline = {
         "bound": "fp32",
-        "kernel": {"exact": "icgn_kernel", "fast": "icgn_fast_kernel", "staged": "icgn_staged_kernel",
+        "kernel": {"exact": "icgn_band_kernel" if args.lanes <= 32 else "icgn_kernel", "fast": "icgn_fast_kernel", "staged": "icgn_staged_kernel",
                    "staged-wide": "icgn_staged_kernel"}[args.solver_mode]
         + f"<affine,bspline,{args.lanes} lanes> (all pyramid levels)",
         "achieved": achieved,
@@ -905,8 +906,8 @@ def main() -> None:
         "peak_source": "measured in this run by gbdic_fp32_peak_probe (FMA chains on every SM); "
                        "MEASURED_PEAKS.json has no FP32 figure",
         "traffic": traffic,
-        "traffic_source": "profiles/traffic_per_launch.json (one ncu capture of the finest level, scaled by units "
-                          "processed to the average launch)",
+        "traffic_source": "profiles/traffic_per_launch.json (one ncu capture of a frame's three launches, the "
+                          "average launch)",
         "flops_per_launch": flops / launches,
         "avg_launch_ms": profile["solver_ms"] / launches,
         "solver_share_of_step": profile["solver_ms"] / ms_profiled if ms_profiled > 0 else None,
