@@ -233,7 +233,10 @@ int gbdic_set_reference_arrays(gbdic_engine *e, int32_t width, int32_t height, c
 namespace {
 
 // Frame stages of the single-scale engine on slot k (after the upload).
-void enqueue_frame(gbdic_engine *e, int k, const gbdic_solver_cfg &cfg, bool seeded, bool preserve, bool prefilter) {
+// `waits`: the call waits for the field, which the outlier pass (where there is
+// one) then leaves in the slot's pinned memory itself.
+void enqueue_frame(gbdic_engine *e, int k, const gbdic_solver_cfg &cfg, bool seeded, bool preserve, bool prefilter,
+                   bool waits = true) {
     auto &rt = *e->rt;
     auto &lvl = e->level;
     auto &slot = *lvl.slots[k];
@@ -242,7 +245,8 @@ void enqueue_frame(gbdic_engine *e, int k, const gbdic_solver_cfg &cfg, bool see
     check_cuda(cudaEventRecord(h.begin, s), "event");
     if (prefilter) rt.enqueue_prefilter(lvl, slot, nullptr, s);
     rt.enqueue_solve(lvl, slot, cfg, seeded, preserve, nullptr, nullptr, s);
-    rt.enqueue_uod(lvl, slot, false, nullptr, s);
+    if (waits) h.out.ensure((size_t)lvl.count * gbdic::state_stride(rt.opts().o.motion_model) * sizeof(float));
+    rt.enqueue_uod(lvl, slot, false, nullptr, s, waits ? h.out.as<float>() : nullptr);
     check_cuda(cudaEventRecord(h.end, s), "event");
 }
 
@@ -251,9 +255,9 @@ void readback(gbdic_engine *e, int k, float *out_state, gbdic_timing *timing, st
     auto &lvl = e->level;
     auto &h = e->host[k];
     const size_t bytes = (size_t)lvl.count * gbdic::state_stride(rt.opts().o.motion_model) * sizeof(float);
-    h.out.ensure(bytes);
-    check_cuda(cudaMemcpyAsync(h.out.as<float>(), rt.output_state(*lvl.slots[k]), bytes, cudaMemcpyDeviceToHost,
-                               rt.stream()), "state readback");
+    if (rt.opts().o.outlier_policy == GBDIC_OUTLIER_DISABLED)
+        check_cuda(cudaMemcpyAsync(h.out.as<float>(), rt.output_state(*lvl.slots[k]), bytes, cudaMemcpyDeviceToHost,
+                                   rt.stream()), "state readback");
     check_cuda(cudaEventRecord(h.done, rt.stream()), "event");
     gbdic::wait_event(h.done, gbdic::kWaitMs);
     const double exec_ms = gbdic::ms_since(t_exec);
@@ -421,7 +425,7 @@ int gbdic_submit(gbdic_engine *e, int32_t slot_index, const uint8_t *frame, int6
         check_cuda(cudaEventRecord(h.uploaded, e->upload), "event");
         check_cuda(cudaStreamWaitEvent(s, h.uploaded, 0), "upload wait");
         h.upload_ms = gbdic::ms_since(h.submitted);
-        enqueue_frame(e, slot_index, *cfg, false, false, true);
+        enqueue_frame(e, slot_index, *cfg, false, false, true, false);
         check_cuda(cudaEventRecord(h.computed, s), "event");
         auto &lvl = e->level;
         const size_t bytes = (size_t)lvl.count * gbdic::state_stride(e->rt->opts().o.motion_model) * sizeof(float);

@@ -169,7 +169,9 @@ class Runtime {
     void enqueue_solve_list(Level &level, LevelSlot &slot, const gbdic_solver_cfg &cfg, const int *list,
                             int length, const unsigned *list_count, int lanes, const uint8_t *frame, float *state,
                             cudaStream_t stream);
-    void enqueue_uod(Level &level, LevelSlot &slot, bool seed_mode, float *out, cudaStream_t stream);
+    // host_out: pinned memory that receives the field beside the device (or nullptr).
+    void enqueue_uod(Level &level, LevelSlot &slot, bool seed_mode, float *out, cudaStream_t stream,
+                     float *host_out = nullptr);
     const float *output_state(LevelSlot &slot) const;
     void upload_frame(Level &level, LevelSlot &slot, const uint8_t *frame, int64_t row_stride,
                       HostBuffer &staging, cudaStream_t stream);

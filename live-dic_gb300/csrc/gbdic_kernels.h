@@ -72,6 +72,7 @@ cudaError_t launch_icgn_batch_any(const BatchSolveArgs &b, int lanes, int grid, 
 struct UodArgs {
     const float *state;
     float *out;
+    float *host_out;      // pinned host copy of `out`, or nullptr
     const float *meta;
     const float *links;   // 4 floats per subset (ROI), or nullptr
     int grid_w, grid_h, count;

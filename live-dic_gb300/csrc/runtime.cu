@@ -609,11 +609,12 @@ void Runtime::enqueue_solve_list(Level &level, LevelSlot &slot, const gbdic_solv
     check_cuda(launch_icgn(a, model, interp, lanes, gauss, grid, s), "listed solver launch");
 }
 
-void Runtime::enqueue_uod(Level &level, LevelSlot &slot, bool seed_mode, float *out, cudaStream_t s) {
+void Runtime::enqueue_uod(Level &level, LevelSlot &slot, bool seed_mode, float *out, cudaStream_t s, float *host_out) {
     if (opt_.o.outlier_policy == GBDIC_OUTLIER_DISABLED) return;
     UodArgs u{};
     u.state = slot.state.as<float>();
     u.out = out ? out : slot.filtered.as<float>();
+    u.host_out = host_out;
     u.meta = level.meta.as<float>();
     u.links = level.links.get() ? level.links.as<float>() : nullptr;
     u.grid_w = level.gw; u.grid_h = level.gh; u.count = level.count;

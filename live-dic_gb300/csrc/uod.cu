@@ -101,6 +101,14 @@ __device__ void store_state(float *dst, int ss, const float *src) {
     for (int k = 0; k < ss / 4; ++k) d4[k] = make_float4(src[4 * k], src[4 * k + 1], src[4 * k + 2], src[4 * k + 3]);
 }
 
+// A subset's filtered state into the field and, for a call that waits for its
+// result on the host, straight into pinned host memory: the copy that followed
+// the pass cost its start and end, 8 to 12 us of a small frame's call.
+__device__ __forceinline__ void publish_state(const UodArgs &a, int index, int ss, const float *src) {
+    store_state(a.out + (size_t)index * ss, ss, src);
+    if (a.host_out != nullptr) store_state(a.host_out + (size_t)index * ss, ss, src);
+}
+
 // icgn.wgsl:1192-1323
 __device__ void median_motion(const UodArgs &a, int index) {
     const int ss = state_stride(a.model);
@@ -154,7 +162,7 @@ __device__ void median_motion(const UodArgs &a, int index) {
             }
         }
     }
-    store_state(a.out + (size_t)index * ss, ss, out);
+    publish_state(a, index, ss, out);
 }
 
 // Windows of 7x7 and 9x9: too many values for registers.
@@ -247,7 +255,7 @@ __global__ void __launch_bounds__(128) median_field_kernel(UodArgs a) {
             if (a.seed_mode && own_status < 0.5f) own[sat] = 0.0f;
         }
     }
-    store_state(a.out + (size_t)index * ss, ss, own);
+    publish_state(a, index, ss, own);
 }
 
 template <int MODEL>
@@ -316,7 +324,7 @@ __device__ __noinline__ void quadratic_uod_unordered(const UodArgs &a, int index
             }
         }
     }
-    store_state(a.out + (size_t)index * ss, ss, out);
+    publish_state(a, index, ss, out);
 }
 
 // Stable sort of 8 values (odd-even transposition, swap only when strictly
@@ -456,7 +464,7 @@ __global__ void __launch_bounds__(128) uod3_kernel(UodArgs a) {
             }
         }
     }
-    store_state(a.out + (size_t)index * ss, ss, own);
+    publish_state(a, index, ss, own);
 }
 
 }  // namespace

@@ -170,3 +170,21 @@ def test_median_fields_in_registers_bit_exact(pairs, model, size, scope):
     expected = oracle_c.uod(state.reshape(-1, stride), metadata, grid=(gw, gh), subset_stride=10, model=model,
                             policy="median", median_size=size, scope_all=scope == "all")
     np.testing.assert_array_equal(got.reshape(-1, stride), expected)
+
+
+@pytest.mark.parametrize("policy,size", [("replace", 3), ("flag", 3), ("median", 3), ("median", 5), ("median", 7),
+                                         ("disabled", 3)])
+@pytest.mark.parametrize("model", ["translation", "affine", "quadratic"])
+def test_waiting_and_pipelined_calls_return_one_field(pairs, model, policy, size):
+    """A waiting call's field is written to pinned memory by the outlier pass, a
+    pipelined one's is copied: the same field, frame after frame."""
+    ref, _ = pairs
+    frames = [np.ascontiguousarray(np.roll(ref, k, 1)) for k in (1, 2, 0)]
+    with ICGNWGPU(subset_size=21, subset_stride=10, motion_model=model, outlier_policy=policy,
+                  median_filter_size=size) as engine:
+        engine.set_reference(ref)
+        waiting = [engine.register(f) for f in frames]
+        for a, b in zip(waiting, engine.register_stream(frames), strict=True):
+            np.testing.assert_array_equal(a.parameters, b.parameters)
+            np.testing.assert_array_equal(a.status, b.status)
+            np.testing.assert_array_equal(a.iterations, b.iterations)
