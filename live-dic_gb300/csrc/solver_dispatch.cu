@@ -173,6 +173,7 @@ cudaError_t launch_icgn(const SolveArgs &a, int model, int interp, int lanes, bo
         return launch_icgn_fast(a, model, lanes, gauss, grid, stream, nullptr);
     if (a.staged_tile > 0 && icgn_staged_supported(model, interp, lanes, a.W))
         return launch_icgn_staged(a, model, lanes, gauss, a.staged_tile, grid, stream, nullptr);
+    if (icgn_blocks_fit(a, model, interp, lanes)) return launch_icgn_blocks(a, model, interp, lanes, gauss, stream);
     return dispatch(a, model, interp, lanes, gauss, grid, stream, nullptr);
 }
 

@@ -1,6 +1,7 @@
-// IC-GN over partial-support ROI windows (reference: solve_partial /
+// A block to a window: IC-GN over partial-support ROI windows, and over the
+// complete windows of a launch too small to fill the chip otherwise (reference: solve_partial /
 // solve_partial_seeded / retry_partial_seeded, shaders/icgn.wgsl:1042-1085):
-// the complete-window solver's iteration with the window's support bits,
+// for those, the complete-window solver's iteration with the window's support bits,
 // support box and partial metadata (validity -4, partial mean and weight
 // sum).  One launch over the partial windows, after the complete-window launch
 // of the same frame.
@@ -23,6 +24,13 @@ namespace gbdic {
 namespace {
 
 constexpr int kPartialThreads = 256;
+// Complete windows of a launch up to which a block has one too.  Device time of a
+// frame, other loops -> blocks (16 lanes): affine B-spline S 21, 324 windows 81 ->
+// 73 us, 676 120 -> 110, 1,156 126 -> 133; S 31 88 -> 58, 103 -> 77, 101 -> 92,
+// 1,764 134 -> 127, 2,704 128 -> 161; affine linear S 21 (direct loop) 676 98 -> 64,
+// 1,764 124 -> 93, 2,704 125 -> 119, 4,356 138 -> 154; translation linear S 15 676
+// 73 -> 53, 1,764 75 -> 66, 2,704 77 -> 79.
+constexpr int kBlockWindowsBspline = 912, kBlockWindows = 2128;
 // Pixels sampled between two accumulations: a multiple of the lane counts (lanes
 // keep their pixels); a whole window up to S = 32.  The arrays' pitch puts the
 // two halves of a warp, which read different arrays, on different banks.
@@ -69,8 +77,8 @@ __device__ __forceinline__ int factor_y(int k) {  // -1: one
     return k == 4 || k == 7 ? kLx : k == 5 || k == 8 ? kLy : -1;
 }
 
-template <int MODEL, int INTERP, int LANES, bool GAUSS>
-__global__ void __launch_bounds__(kPartialThreads) partial_window_kernel(SolveArgs a) {
+template <int MODEL, int INTERP, int LANES, bool GAUSS, bool PART>
+__global__ void __launch_bounds__(kPartialThreads) window_block_kernel(SolveArgs a) {
     constexpr int N = SumCount<MODEL>::value, PARTS = kPartialThreads / LANES, PER = (N + PARTS - 1) / PARTS;
     constexpr int n = parameter_count(MODEL), META = meta_stride(MODEL);
     __shared__ float factors[kFactors * kPartialPitch];
@@ -78,9 +86,9 @@ __global__ void __launch_bounds__(kPartialThreads) partial_window_kernel(SolveAr
     __shared__ float md[META], hi[n * n];
     __shared__ float update[8];
     const int tid = threadIdx.x, lane = tid % LANES, part = tid / LANES;
-    const int group = blockIdx.x, idx = __ldg(a.partial_index + group);
-    const uint32_t *support = a.support + (size_t)group * a.support_words;
-    const float4 box = __ldg(a.support_box + group);
+    const int group = blockIdx.x, idx = PART ? __ldg(a.partial_index + group) : group;
+    const uint32_t *support = PART ? a.support + (size_t)group * a.support_words : nullptr;
+    const float4 box = PART ? __ldg(a.support_box + group) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int i = tid; i < META + n * n; i += kPartialThreads) {
         if (i < META) md[i] = __ldg(a.meta + (size_t)idx * META + i);
         else hi[i - META] = __ldg(a.inv + (size_t)idx * n * n + i - META);
@@ -96,19 +104,22 @@ __global__ void __launch_bounds__(kPartialThreads) partial_window_kernel(SolveAr
     }
     if (MODEL == kModelTranslation) { w.l0 = w.l1 = w.l2 = w.l3 = 0.0f; }
     __syncthreads();
-    float status = enabled && md[1] == -4.0f ? 0.0f : -1.0f;
+    const bool valid = enabled && (PART ? md[1] == -4.0f : md[1] >= 0.5f);
+    float status = valid ? 0.0f : !PART && a.roi_enabled ? fminf(-1.0f, md[1]) : -1.0f;
     float iters = 0.0f;
     const int S = a.S, npix = S * S, W = a.W, H = a.H;
     const int px0 = (idx % a.grid_w) * a.stride, py0 = (idx / a.grid_w) * a.stride;
     const unsigned origin = (unsigned)py0 * (unsigned)W + (unsigned)px0;
     const float half = 0.5f * ((float)S - 1.0f), ox = (float)px0 + half, oy = (float)py0 + half;
-    const float ref_mean = md[14], wsum = md[3 + 2 * n];
+    const float ref_mean = PART || a.use_mean ? md[14] : 0.0f;
+    const float wsum = PART || GAUSS ? md[3 + 2 * n] : (float)(S * S);
     float prev_change = 3.402823e38f;
     unsigned stalled = 0u;
 
     for (int it = 0; it < 30; ++it) {  // the block's threads hold the same state
         if (!(a.div_patience != 0 && status == 3.0f)) {
-            if (!warp_inside_box<MODEL>(w, px0, py0, half, box, W, H)) {
+            if (!(PART ? warp_inside_box<MODEL>(w, px0, py0, half, box, W, H)
+                       : warp_inside<MODEL>(w, px0, py0, S, half, W, H))) {
                 if (!a.roi_enabled || status > -2.5f) status = -1.0f;
             }
         }
@@ -125,7 +136,7 @@ __global__ void __launch_bounds__(kPartialThreads) partial_window_kernel(SolveAr
                 const int p = base + i;
                 const float lx = q.col - half, ly = q.row - half;
                 float wc = 0.0f, wf = 0.0f, gxg = 0.0f, gyg = 0.0f, g = 0.0f;
-                if ((__ldg(support + (p >> 5)) >> (p & 31)) & 1u) {
+                if (!PART || ((__ldg(support + (p >> 5)) >> (p & 31)) & 1u)) {
                     const float4 rv = __ldg(a.plane + q.index);
                     const float wt = GAUSS ? __ldg(a.weights + p) : 1.0f, f = rv.x - ref_mean;
                     float dx, dy;
@@ -219,7 +230,10 @@ __global__ void __launch_bounds__(kPartialThreads) partial_window_kernel(SolveAr
 
 template <int MODEL, int INTERP, int LANES, bool GAUSS>
 cudaError_t go(const SolveArgs &a, cudaStream_t s) {
-    partial_window_kernel<MODEL, INTERP, LANES, GAUSS><<<a.count, kPartialThreads, 0, s>>>(a);
+    if (a.partial_index != nullptr)
+        window_block_kernel<MODEL, INTERP, LANES, GAUSS, true><<<a.count, kPartialThreads, 0, s>>>(a);
+    else
+        window_block_kernel<MODEL, INTERP, LANES, GAUSS, false><<<a.count, kPartialThreads, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -250,6 +264,16 @@ cudaError_t by_weight(const SolveArgs &a, int interp, int lanes, bool gauss, cud
 }
 
 }  // namespace
+
+bool icgn_blocks_fit(const SolveArgs &a, int model, int interp, int lanes) {
+    return model != kModelQuadratic && lanes <= 32 && !a.persistent && a.subset_list == nullptr &&
+           a.list_count == nullptr && a.count <= (interp == kInterpBspline ? kBlockWindowsBspline : kBlockWindows);
+}
+
+cudaError_t launch_icgn_blocks(const SolveArgs &args, int model, int interp, int lanes, bool gauss, cudaStream_t stream) {
+    return model == kModelAffine ? by_weight<kModelAffine>(args, interp, lanes, gauss, stream)
+                                 : by_weight<kModelTranslation>(args, interp, lanes, gauss, stream);
+}
 
 cudaError_t launch_icgn_partial(const SolveArgs &args, int model, int interp, int lanes, bool gauss,
                                 cudaStream_t stream) {

@@ -188,3 +188,31 @@ def test_waiting_and_pipelined_calls_return_one_field(pairs, model, policy, size
             np.testing.assert_array_equal(a.parameters, b.parameters)
             np.testing.assert_array_equal(a.status, b.status)
             np.testing.assert_array_equal(a.iterations, b.iterations)
+
+
+@pytest.mark.parametrize("lanes", [16, 32])
+@pytest.mark.parametrize("model,interp,weighting,subset,stride", [
+    ("affine", "bspline", "uniform", 21, 11), ("affine", "bspline", "gaussian", 33, 33), ("affine", "cubic", "uniform", 15, 9),
+    ("affine", "linear", "gaussian", 16, 13), ("translation", "bspline", "uniform", 41, 20),
+    ("translation", "linear", "uniform", 12, 12)])
+def test_few_windows_by_blocks_bit_exact(pairs, model, interp, weighting, subset, stride, lanes):
+    """Launches of few windows, a block each: odd and even sides, more than one
+    sampled chunk, tiled grids, windows that leave the frame, a masked reference."""
+    ref, _ = pairs
+    tgt = np.ascontiguousarray(np.roll(np.roll(ref, 2, 1), -1, 0))
+    mask = None
+    if weighting == "uniform":
+        mask = np.ones(ref.shape, bool)
+        mask[30:70, 40:110] = False
+    with ICGNWGPU(subset_size=subset, subset_stride=stride, motion_model=model, interpolation=interp,
+                  spatial_weighting=weighting, outlier_policy="disabled", solver_workgroup_size=lanes) as engine:
+        engine.set_reference(ref, roi_mask=mask)
+        result = engine.register(tgt)
+        plane, inverse, metadata = engine.export_reference()
+        coef = engine.export_coefficients() if interp == "bspline" else None
+        weights = engine.export_weights() if weighting == "gaussian" else None
+    assert result.status.size <= 912
+    expected = oracle_c.solve(tgt, coef, plane, metadata, inverse, subset_size=subset, subset_stride=stride, model=model,
+                              interpolation=interp, lanes=lanes, roi_enabled=mask is not None, weights=weights)
+    got = np.concatenate([result.parameters, result.status[..., None], result.iterations[..., None]], -1)
+    np.testing.assert_array_equal(got.reshape(-1, 8), expected.reshape(-1, 8))
