@@ -168,12 +168,13 @@ struct gbdic_batch {
             q.models.ensure(models.size() * sizeof(int));
             q.first.ensure(first.size() * sizeof(int));
             q.counter.ensure(sizeof(unsigned));
-            check_cuda(cudaMemcpy(q.args.get(), args.data(), args.size() * sizeof(gbdic::SolveArgs),
-                                  cudaMemcpyHostToDevice), "batch table");
-            check_cuda(cudaMemcpy(q.models.get(), models.data(), models.size() * sizeof(int), cudaMemcpyHostToDevice),
-                       "batch table");
-            check_cuda(cudaMemcpy(q.first.get(), first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice),
-                       "batch table");
+            check_cuda(cudaMemcpyAsync(q.args.get(), args.data(), args.size() * sizeof(gbdic::SolveArgs),
+                                       cudaMemcpyHostToDevice, stream), "batch table");
+            check_cuda(cudaMemcpyAsync(q.models.get(), models.data(), models.size() * sizeof(int),
+                                       cudaMemcpyHostToDevice, stream), "batch table");
+            check_cuda(cudaMemcpyAsync(q.first.get(), first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                       stream), "batch table");
+            check_cuda(cudaStreamSynchronize(stream), "batch tables");
             const int resident =
                 cls == 2 ? gbdic::icgn_batch_any_occupancy(lanes) : gbdic::icgn_batch_occupancy(lanes, cls == 1);
             if (resident <= 0) fail(GBDIC_ECUDA, "batch solver occupancy query failed");

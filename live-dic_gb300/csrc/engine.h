@@ -180,6 +180,7 @@ class Runtime {
     bool banded() const { return band_plans_[0].rows > 0 || band_plans_[1].rows > 0; }
     void ensure_plane(Level &level);
     void split_plane(Level &level, bool gradients);
+    void upload(const DeviceBuffer &dst, const void *src, size_t bytes, const char *what);
     // Switch the solver variant (lanes per subset, persistent queue).
     void set_variant(int lanes, bool persistent);
     // Switch the pixel loop (GBDIC_SOLVER_*).

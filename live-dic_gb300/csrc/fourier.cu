@@ -755,12 +755,13 @@ int gbdic_fourier_create(int32_t device, const uint8_t *window, const uint8_t *a
         std::vector<double> taper((size_t)f->half);
         const double pi = 3.14159265358979323846;
         for (int k = 0; k < f->half; ++k) taper[(size_t)k] = 0.5 - 0.5 * cos(2.0 * pi * k / (double)(f->half - 1));
-        check_cuda(cudaMemcpy(f->taper.get(), taper.data(), taper.size() * sizeof(double), cudaMemcpyHostToDevice), "taper");
-        check_cuda(cudaMemcpy(f->window.get(), window, px, cudaMemcpyHostToDevice), "window");
+        check_cuda(cudaMemcpyAsync(f->taper.get(), taper.data(), taper.size() * sizeof(double), cudaMemcpyHostToDevice,
+                                   f->stream), "taper");
+        check_cuda(cudaMemcpyAsync(f->window.get(), window, px, cudaMemcpyHostToDevice, f->stream), "window");
         const uint8_t *allow = nullptr;
         if (allowed) {
             f->allowed.ensure(px);
-            check_cuda(cudaMemcpy(f->allowed.get(), allowed, px, cudaMemcpyHostToDevice), "ROI window");
+            check_cuda(cudaMemcpyAsync(f->allowed.get(), allowed, px, cudaMemcpyHostToDevice, f->stream), "ROI window");
             allow = f->allowed.as<uint8_t>();
         }
         f->sized([&](auto logn) { f->reference_spectrum<decltype(logn)::value>(allow); });

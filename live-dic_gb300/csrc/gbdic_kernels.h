@@ -9,7 +9,7 @@
 namespace gbdic {
 
 // ------------------------------------------------------------ prefilter
-cudaError_t set_fir_taps(const float *taps25);
+cudaError_t set_fir_taps(const float *taps25, cudaStream_t stream);
 cudaError_t launch_fir_prefilter(const uint8_t *img, int W, int H, int pitch, float *coef,
                                  cudaStream_t stream);
 

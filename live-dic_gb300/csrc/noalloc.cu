@@ -69,7 +69,8 @@ int scratch_for_current_device(float **coefficients, std::string &error) {
         }
         float taps[25];
         gbdic::fir_taps(taps);
-        err = gbdic::set_fir_taps(taps);
+        err = gbdic::set_fir_taps(taps, nullptr);
+        if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
         if (err != cudaSuccess) {
             error = std::string("FIR taps upload failed: ") + cudaGetErrorString(err);
             return GBDIC_ECUDA;

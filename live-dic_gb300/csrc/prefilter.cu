@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(kThreads) fir_prefilter_kernel(const uint8_t *
 }
 }  // namespace
 
-cudaError_t set_fir_taps(const float *taps25) {
-    return cudaMemcpyToSymbol(c_fir, taps25, 25 * sizeof(float));
+cudaError_t set_fir_taps(const float *taps25, cudaStream_t stream) {
+    return cudaMemcpyToSymbolAsync(c_fir, taps25, 25 * sizeof(float), 0, cudaMemcpyHostToDevice, stream);
 }
 
 cudaError_t launch_fir_prefilter(const uint8_t *img, int W, int H, int pitch, float *coef,

@@ -153,23 +153,25 @@ void reset_temporal(gbdic_pyramid *p, cudaStream_t s) {
     const int model = p->po.base.motion_model, ss = gbdic::state_stride(model);
     std::vector<float> state((size_t)count * ss, 0.0f);
     for (int i = 0; i < count; ++i) state[(size_t)i * ss + gbdic::parameter_count(model)] = -1.0f;
-    check_cuda(cudaMemcpy(p->history.get(), state.data(), state.size() * sizeof(float), cudaMemcpyHostToDevice), "history");
-    check_cuda(cudaMemset(p->ages.get(), 0xff, (size_t)count * sizeof(uint32_t)), "ages");
+    check_cuda(cudaMemcpyAsync(p->history.get(), state.data(), state.size() * sizeof(float), cudaMemcpyHostToDevice, s),
+               "history");
+    check_cuda(cudaMemsetAsync(p->ages.get(), 0xff, (size_t)count * sizeof(uint32_t), s), "ages");
     if (p->velocity()) {
-        check_cuda(cudaMemcpy(p->prev_history.get(), state.data(), state.size() * sizeof(float), cudaMemcpyHostToDevice),
-                   "history");
-        check_cuda(cudaMemset(p->prev_ages.get(), 0xff, (size_t)count * sizeof(uint32_t)), "ages");
+        check_cuda(cudaMemcpyAsync(p->prev_history.get(), state.data(), state.size() * sizeof(float),
+                                   cudaMemcpyHostToDevice, s), "history");
+        check_cuda(cudaMemsetAsync(p->prev_ages.get(), 0xff, (size_t)count * sizeof(uint32_t), s), "ages");
     }
+    std::vector<float> coarse;
     if (p->fine_correction()) {
         const int cc = p->levels.back()->count;
-        std::vector<float> coarse((size_t)cc * ss, 0.0f);
+        coarse.assign((size_t)cc * ss, 0.0f);
         for (int i = 0; i < cc; ++i) coarse[(size_t)i * ss + gbdic::parameter_count(model)] = -1.0f;
-        check_cuda(cudaMemcpy(p->coarse_history.get(), coarse.data(), coarse.size() * sizeof(float),
-                              cudaMemcpyHostToDevice), "history");
-        check_cuda(cudaMemset(p->coarse_ages.get(), 0xff, (size_t)cc * sizeof(uint32_t)), "ages");
+        check_cuda(cudaMemcpyAsync(p->coarse_history.get(), coarse.data(), coarse.size() * sizeof(float),
+                                   cudaMemcpyHostToDevice, s), "history");
+        check_cuda(cudaMemsetAsync(p->coarse_ages.get(), 0xff, (size_t)cc * sizeof(uint32_t), s), "ages");
     }
+    check_cuda(cudaStreamSynchronize(s), "history reset");
     p->active_levels = p->L();
-    (void)s;
 }
 
 // Everything a frame does after its finest target is resident at `frame0`.
@@ -521,7 +523,7 @@ int gbdic_pyramid_set_reference(gbdic_pyramid *p, const uint8_t *image, int32_t 
             if (l < L - 1 && rois && rois[l].seed_links) {
                 const size_t b = (size_t)p->levels[l]->count * sizeof(uint32_t);
                 p->seed_links[l]->ensure(b);
-                check_cuda(cudaMemcpy(p->seed_links[l]->get(), rois[l].seed_links, b, cudaMemcpyHostToDevice), "links");
+                check_cuda(cudaMemcpyAsync(p->seed_links[l]->get(), rois[l].seed_links, b, cudaMemcpyHostToDevice, s), "links");
                 p->has_seed_links[l] = true;
             }
         }
@@ -529,7 +531,7 @@ int gbdic_pyramid_set_reference(gbdic_pyramid *p, const uint8_t *image, int32_t 
         if (temporal_links) {
             const size_t b = (size_t)p->levels[L - 1]->count * sizeof(uint32_t);
             p->temporal_links.ensure(b);
-            check_cuda(cudaMemcpy(p->temporal_links.get(), temporal_links, b, cudaMemcpyHostToDevice), "links");
+            check_cuda(cudaMemcpyAsync(p->temporal_links.get(), temporal_links, b, cudaMemcpyHostToDevice, s), "links");
             p->has_temporal_links = true;
         }
         if (p->temporal()) {
@@ -552,8 +554,9 @@ int gbdic_pyramid_set_reference(gbdic_pyramid *p, const uint8_t *image, int32_t 
                 if (rois && rois[0].selected)
                     for (int i = 0; i < n; ++i) links[i] = rois[0].selected[i] ? 31u : 0u;
                 p->fine_links.ensure((size_t)n * sizeof(uint32_t));
-                check_cuda(cudaMemcpy(p->fine_links.get(), links.data(), links.size() * sizeof(uint32_t),
-                                      cudaMemcpyHostToDevice), "links");
+                check_cuda(cudaMemcpyAsync(p->fine_links.get(), links.data(), links.size() * sizeof(uint32_t),
+                                           cudaMemcpyHostToDevice, s), "links");
+                check_cuda(cudaStreamSynchronize(s), "links");
             }
             reset_temporal(p, s);
         }

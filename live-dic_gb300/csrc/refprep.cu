@@ -741,7 +741,9 @@ cudaError_t launch_split_plane(const float4 *plane, size_t pixels, float *f, flo
     return cudaGetLastError();
 }
 
-cudaError_t set_gauss_taps(const float *taps7) { return cudaMemcpyToSymbol(c_gauss, taps7, 7 * sizeof(float)); }
+cudaError_t set_gauss_taps(const float *taps7, cudaStream_t stream) {
+    return cudaMemcpyToSymbolAsync(c_gauss, taps7, 7 * sizeof(float), 0, cudaMemcpyHostToDevice, stream);
+}
 
 size_t affine_prep_moment_floats(int count) { return (size_t)kAffineMoments * (size_t)count; }
 

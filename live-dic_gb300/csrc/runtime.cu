@@ -20,7 +20,7 @@
 
 namespace gbdic {
 
-cudaError_t set_gauss_taps(const float *taps7);
+cudaError_t set_gauss_taps(const float *taps7, cudaStream_t stream);
 
 namespace {
 
@@ -143,12 +143,12 @@ Runtime::Runtime(const gbdic_options &options) {
     check_cuda(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     float taps[25];
     std::memcpy(taps, kFirBits, sizeof taps);
-    check_cuda(set_fir_taps(taps), "FIR taps");
+    check_cuda(set_fir_taps(taps, stream_), "FIR taps");
     double g[7], gs = 0.0;
     for (int k = 0; k < 7; ++k) { g[k] = std::exp(-0.5 * (k - 3) * (k - 3)); gs += g[k]; }
     float gf[7];
     for (int k = 0; k < 7; ++k) gf[k] = (float)(g[k] / gs);
-    check_cuda(set_gauss_taps(gf), "Gaussian taps");
+    check_cuda(set_gauss_taps(gf, stream_), "Gaussian taps");
     const int S = options.subset_size;
     opt_.weights.resize((size_t)S * S);
     double wsum = 0.0;
@@ -165,15 +165,14 @@ Runtime::Runtime(const gbdic_options &options) {
         }
     opt_.weight_sum = (float)wsum;
     weights_.ensure(opt_.weights.size() * sizeof(float));
-    check_cuda(cudaMemcpy(weights_.get(), opt_.weights.data(), opt_.weights.size() * sizeof(float),
-                          cudaMemcpyHostToDevice), "weights upload");
+    upload(weights_, opt_.weights.data(), opt_.weights.size() * sizeof(float), "weights upload");
     // exp(-(x^2 + y^2) / 2 sigma^2) = exp(-x^2 / 2 sigma^2) exp(-y^2 / 2 sigma^2)
     std::vector<float> axis((size_t)S, 1.0f);
     if (options.spatial_weighting == 1)
         for (int k = 0; k < S; ++k) axis[k] = (float)std::exp(-0.5 * (k - half) * (k - half) / (sigma * sigma));
     axis_weights_.ensure(axis.size() * sizeof(float));
-    check_cuda(cudaMemcpy(axis_weights_.get(), axis.data(), axis.size() * sizeof(float), cudaMemcpyHostToDevice),
-               "axis weights upload");
+    upload(axis_weights_, axis.data(), axis.size() * sizeof(float), "axis weights upload");
+    check_cuda(cudaStreamSynchronize(stream_), "weights upload");
     for (int k = 0; k < 2; ++k) band_plans_[k] = plan_bands(S, options.motion_model, options.interpolation, 16 << k, sm_count_);
     if (options.persistent) persistent_grid(opt_.lanes);
 }
@@ -383,6 +382,14 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
     return ms;
 }
 
+// A host-to-device copy in the order of the engine's stream.  cudaMemcpy from
+// pageable memory may return before its DMA has landed, and the stream, which
+// does not block on the default one, would not wait for it either.  The caller
+// synchronises before `src` goes.
+void Runtime::upload(const DeviceBuffer &dst, const void *src, size_t bytes, const char *what) {
+    check_cuda(cudaMemcpyAsync(dst.get(), src, bytes, cudaMemcpyHostToDevice, stream_), what);
+}
+
 void Runtime::upload_reference_arrays(Level &level, const float *plane, const float *meta, const float *inverse,
                                       const float *links) {
     const int model = opt_.o.motion_model, n = parameter_count(model);
@@ -391,21 +398,15 @@ void Runtime::upload_reference_arrays(Level &level, const float *plane, const fl
     level.meta.ensure((size_t)level.count * meta_stride(model) * sizeof(float));
     level.inv.ensure((size_t)level.count * n * n * sizeof(float));
     level.partial_count = 0;
-    check_cuda(cudaMemcpy(level.plane.get(), plane, px * sizeof(float4), cudaMemcpyHostToDevice), "plane upload");
+    upload(level.plane, plane, px * sizeof(float4), "plane upload");
     level.solver_f = nullptr;
-    if (banded()) {
-        split_plane(level, true);
-        check_cuda(cudaStreamSynchronize(stream_), "plane split");
-    }
-    check_cuda(cudaMemcpy(level.meta.get(), meta, (size_t)level.count * meta_stride(model) * sizeof(float),
-                          cudaMemcpyHostToDevice), "metadata upload");
-    check_cuda(cudaMemcpy(level.inv.get(), inverse, (size_t)level.count * n * n * sizeof(float),
-                          cudaMemcpyHostToDevice), "inverse upload");
+    if (banded()) split_plane(level, true);
+    upload(level.meta, meta, (size_t)level.count * meta_stride(model) * sizeof(float), "metadata upload");
+    upload(level.inv, inverse, (size_t)level.count * n * n * sizeof(float), "inverse upload");
     level.roi = links != nullptr;
     if (links) {
         level.links.ensure((size_t)level.count * 4 * sizeof(float));
-        check_cuda(cudaMemcpy(level.links.get(), links, (size_t)level.count * 4 * sizeof(float),
-                              cudaMemcpyHostToDevice), "links upload");
+        upload(level.links, links, (size_t)level.count * 4 * sizeof(float), "links upload");
     } else {
         level.links.reset();
     }
@@ -420,7 +421,8 @@ void Runtime::upload_reference_arrays(Level &level, const float *plane, const fl
     }
     level.valid_count = valid;
     level.admissible.ensure((size_t)level.count);
-    check_cuda(cudaMemcpy(level.admissible.get(), adm.data(), adm.size(), cudaMemcpyHostToDevice), "admissibility upload");
+    upload(level.admissible, adm.data(), adm.size(), "admissibility upload");
+    check_cuda(cudaStreamSynchronize(stream_), "reference upload");
 }
 
 void Runtime::set_partial_support(Level &level, int count, const int32_t *indices, const uint32_t *words,
@@ -447,22 +449,20 @@ void Runtime::set_partial_support(Level &level, int count, const int32_t *indice
         std::memcpy(&inv[i * n * n], inverse_rows + (size_t)k * n * n, (size_t)n * n * sizeof(float));
         adm[i] = meta[i * ms + 1] == -4.0f ? 1 : 0;
     }
-    check_cuda(cudaMemcpy(level.meta.get(), meta.data(), meta.size() * sizeof(float), cudaMemcpyHostToDevice), "metadata");
-    check_cuda(cudaMemcpy(level.inv.get(), inv.data(), inv.size() * sizeof(float), cudaMemcpyHostToDevice), "inverse");
-    check_cuda(cudaMemcpy(level.admissible.get(), adm.data(), adm.size(), cudaMemcpyHostToDevice), "admissibility");
+    upload(level.meta, meta.data(), meta.size() * sizeof(float), "metadata");
+    upload(level.inv, inv.data(), inv.size() * sizeof(float), "inverse");
+    upload(level.admissible, adm.data(), adm.size(), "admissibility");
     level.partial_count = count;
     level.support_words = words_per_window;
     if (count > 0) {
         level.partial_index.ensure((size_t)count * sizeof(int32_t));
         level.partial_words.ensure((size_t)count * words_per_window * sizeof(uint32_t));
         level.partial_boxes.ensure((size_t)count * 4 * sizeof(float));
-        check_cuda(cudaMemcpy(level.partial_index.get(), indices, (size_t)count * sizeof(int32_t), cudaMemcpyHostToDevice),
-                   "partial indices");
-        check_cuda(cudaMemcpy(level.partial_words.get(), words, (size_t)count * words_per_window * sizeof(uint32_t),
-                              cudaMemcpyHostToDevice), "support words");
-        check_cuda(cudaMemcpy(level.partial_boxes.get(), boxes, (size_t)count * 4 * sizeof(float), cudaMemcpyHostToDevice),
-                   "support boxes");
+        upload(level.partial_index, indices, (size_t)count * sizeof(int32_t), "partial indices");
+        upload(level.partial_words, words, (size_t)count * words_per_window * sizeof(uint32_t), "support words");
+        upload(level.partial_boxes, boxes, (size_t)count * 4 * sizeof(float), "support boxes");
     }
+    check_cuda(cudaStreamSynchronize(stream_), "partial support upload");
     int valid = 0;
     for (int i = 0; i < level.count; ++i) valid += meta[(size_t)i * ms + 1] > 0.5f;
     level.valid_count = valid;
@@ -558,8 +558,10 @@ void Runtime::set_profiling(bool enable) {
 void Runtime::profile_reset() {
     profile_used_ = 0;
     profile_launches_ = 0;
-    if (profile_iterations_.get())
-        check_cuda(cudaMemset(profile_iterations_.get(), 0, sizeof(unsigned long long)), "profile reset");
+    if (profile_iterations_.get()) {
+        check_cuda(cudaMemsetAsync(profile_iterations_.get(), 0, sizeof(unsigned long long), stream_), "profile reset");
+        check_cuda(cudaStreamSynchronize(stream_), "profile reset");
+    }
 }
 
 void Runtime::profile_read(double &solver_ms, long long &launches, long long &timed, unsigned long long &iterations) {

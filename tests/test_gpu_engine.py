@@ -215,3 +215,26 @@ def test_register_pair_one_shot(c0_pair):
     np.testing.assert_array_equal(one.parameters, expected.parameters)
     np.testing.assert_array_equal(one.status, expected.status)
     assert (one.status >= 1).mean() > 0.9
+
+
+@pytest.mark.parametrize("subset,stride", [(21, 10), (24, 24)])
+def test_uploaded_references_replace_one_another(subset, stride):
+    """References uploaded as arrays, one after the other on one engine
+    (overlapping windows, and tiled ones, whose plane is centred): every field
+    is that of the engine that prepared the arrays."""
+    first, sp = synthetic.reference_image(1280, 960, seed=91, device="cpu")
+    tgt = synthetic.deformed_image(sp, synthetic.affine_field(0.4, 1e-3, 0.0, -0.3, 0.0, -6e-4), noise_seed=92,
+                                   device="cpu")
+    frames = [(first, tgt), (np.ascontiguousarray(first[::-1]), np.ascontiguousarray(tgt[::-1]))]
+    options = dict(subset_size=subset, subset_stride=stride, outlier_policy="disabled")
+    prepared = []
+    for ref, cur in frames:
+        with ICGNWGPU(**options) as engine:
+            engine.set_reference(ref)
+            prepared.append((engine.export_reference(), _packed(engine.register(cur))))
+    with ICGNWGPU(**options) as engine:
+        for k in (0, 1, 0, 1, 1, 0):
+            plane, inverse, metadata = prepared[k][0]
+            engine.set_reference_arrays(1280, 960, plane, metadata, inverse)
+            np.testing.assert_array_equal(_packed(engine.register(frames[k][1])), prepared[k][1])
+    assert (prepared[0][1][..., 6] == 1.0).mean() > 0.9 and prepared[0][1][..., 6].size > 912

@@ -413,3 +413,18 @@ def test_batch_modes_and_split_k_choice():
     assert learned.SeedNet._forward_splits(conv4) == 3   # 64 tiles -> 192
     assert learned.SeedNet._forward_splits(conv5) == 18  # 16 tiles -> 288
     assert learned.SeedNet._forward_splits(conv2) == 1   # 1024 tiles fill the GPU
+
+
+def test_uploads_follow_their_stream():
+    """Engine streams do not block on the default stream, and a copy from
+    pageable memory (a fill, a constant) issued there may land after the call
+    returned: a launch that follows must be in the same stream's order."""
+    sources = sorted((ROOT / "live-dic_gb300" / "csrc").glob("*.cu*"))
+    assert len(sources) > 20
+    found = []
+    for path in sources:
+        text = path.read_text()
+        for call in re.finditer(r"\b(cudaMemcpy|cudaMemset|cudaMemcpyToSymbol)\(([^;]*);", text):
+            if call.group(1) != "cudaMemcpy" or "cudaMemcpyHostToDevice" in call.group(2):
+                found.append(f"{path.name}:{text.count(chr(10), 0, call.start()) + 1}")
+    assert found == []
