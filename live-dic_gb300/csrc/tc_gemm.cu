@@ -764,13 +764,17 @@ __global__ void __launch_bounds__(GATHER ? kMaxThreads : 128, 1)
               "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
             : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (k0 + row >= args.k_rows) continue;
-        float4 *o = reinterpret_cast<float4 *>(args.partial + ((size_t)blockIdx.z * args.k_rows + k0 + row) * s.Cout +
-                                               n0 + c);
+        // Rows beyond Kp are not stored; their lanes stay for the next load,
+        // which the whole warp issues (Kp need not be a multiple of 32).
+        if (k0 + row < args.k_rows) {
+            float4 *o = reinterpret_cast<float4 *>(args.partial +
+                                                   ((size_t)blockIdx.z * args.k_rows + k0 + row) * s.Cout + n0 + c);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            o[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
-                               __uint_as_float(r[4 * j + 3]));
+            for (int j = 0; j < 4; ++j)
+                o[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]),
+                                   __uint_as_float(r[4 * j + 3]));
+        }
+        __syncwarp();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -251,3 +251,32 @@ def test_masked_data_gradient_epilogue(B, H, Cin, Cout):
     assert torch.equal(out, masked.to(torch.bfloat16))
     bound = Min * 2.0 ** -24 * masked.double().abs().sum(0)
     assert bool(((db.double() - masked.double().sum(0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("B,H,Cin,Cout,Kp,splits", [(8, 16, 8, 64, 72, 4), (8, 16, 24, 128, 216, 2),
+                                                  (8, 16, 16, 64, 145, 8), (16, 8, 32, 192, 300, 1)])
+def test_weight_gradient_with_a_reduction_of_any_length(B, H, Cin, Cout, Kp, splits):
+    """Kp from 9 C on without padding to the tiles: the last warp of a tile
+    stores some of its rows, and those beyond 9 C are zero."""
+    lib = _native.load()
+    OH = (H + 1) // 2
+    shape, g = _native.NnConvShape(B, H, H, Cin, OH, OH, Cout, Kp), torch.Generator(device="cuda").manual_seed(Kp)
+    M = B * OH * OH
+    x = torch.randn(B, H, H, Cin, generator=g, device="cuda").to(torch.bfloat16)
+    dz = torch.randn(M, Cout, generator=g, device="cuda").to(torch.bfloat16)
+    taps = torch.nn.functional.pad(x.float(), (0, 0, 1, 1, 1, 1))
+    a = torch.stack([taps[:, ky:ky + 2 * OH:2, kx:kx + 2 * OH:2] for ky in range(3) for kx in range(3)], -2)
+    a = torch.nn.functional.pad(a.reshape(M, 9 * Cin), (0, Kp - 9 * Cin)).double()
+    partial = torch.full((splits + 1, Kp, Cout), 7.0, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _native.check(lib.gbdic_nn_conv_wgrad(C.byref(shape), C.c_void_p(x.data_ptr()), C.c_void_p(dz.data_ptr()), splits,
+                                          C.c_void_p(partial.data_ptr()), None, C.c_void_p(err.data_ptr()), None),
+                  lib.gbdic_last_error(None))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    rows = M // splits
+    for s in range(splits):
+        part, z = a[s * rows:(s + 1) * rows], dz[s * rows:(s + 1) * rows].double()
+        bound = rows * 2.0 ** -24 * (part.abs().T @ z.abs())
+        assert bool(((partial[s].double() - part.T @ z).abs() <= bound).all())
+    assert bool((partial[splits] == 7.0).all())
