@@ -192,7 +192,7 @@ class SeedNet:
         """Inference copies: run the 2-channel input layer as one direct
         convolution (gbdic_nn_conv_c2_direct) with the current BF16 weights,
         read to the host once here; later weight updates are not seen, and
-        the layer's im2col operand (needed by backward) is not written."""
+        backward writes the layer's im2col operand itself."""
         torch = _torch()
         c = self.convs[0]
         w = self.w[0][:, :9 * c.cin].to(torch.bfloat16).float().cpu().numpy()
@@ -303,6 +303,9 @@ class SeedNet:
         last = self.convs[-1]
         _call(lib, "gbdic_nn_relu_bias_backward", _ptr(b["dy"]), last.cout, _ptr(self.y[-1]), last.M, last.cout,
               _ptr(b["dz"][-1]), None, _ptr(b["db_partial"][-1]), _ptr(self.grads[2 * nconv - 1]), stream)
+        if getattr(self, "_direct", None) is not None:
+            # the direct first layer of the forward does not write its im2col operand
+            _call(lib, "gbdic_nn_im2col", C.byref(self._shape(0)), _ptr(self.x0), _ptr(self.a[0]), stream)
         for i in range(nconv - 1, -1, -1):
             c = self.convs[i]
             dz = b["dz"][i]

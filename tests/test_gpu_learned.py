@@ -399,3 +399,34 @@ def _graph_and_list_identity(net, ref, frames, lanes):
                 "reseeding"} <= set(stages)
         assert all(v >= 0.0 for v in stages.values())
         assert abs(sum(v for k, v in stages.items() if k != "total") - stages["total"]) <= 1e-3 * stages["total"] + 1e-3
+
+
+def test_gradients_after_a_direct_first_layer():
+    """With the input layer run as a direct convolution the weight gradient of
+    that layer is still that of the current input: float64 sums of the input's
+    im2col rows times dZ, within the FP32 sums of a split and over the splits.
+    An earlier forward of the GEMM path on another input leaves its im2col
+    operand behind."""
+    B = 128
+    net = learned.SeedNet(batch=B, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    target = torch.randn(B, 6, generator=g, device="cuda")
+    net.x0.copy_(torch.randn(net.x0.shape, generator=g, device="cuda"))
+    net.forward()
+    net.use_direct_first_layer()
+    net.x0.copy_(torch.randn(net.x0.shape, generator=g, device="cuda"))
+    net.forward()
+    net.loss_and_grad(target)
+    net.backward()
+    torch.cuda.synchronize()
+    net.check_device_errors()
+    c, dz = net.convs[0], net._bwd["dz"][0].double()
+    x = torch.nn.functional.pad(net.x0.double(), (0, 0, 1, 1, 1, 1))
+    rows = torch.stack([x[:, ky:ky + 2 * c.OH:2, kx:kx + 2 * c.OH:2] for ky in range(3) for kx in range(3)], -2)
+    rows = rows.reshape(c.M, 9 * c.cin)
+    splits = net._bwd["splits"][0]
+    bound = (c.M // splits + splits) * 2.0 ** -24 * (dz.abs().T @ rows.abs())
+    got = net.grads[0][:, :9 * c.cin].double()
+    want = dz.T @ rows
+    assert bool(((got - want).abs() <= bound).all())
+    assert float(want.norm()) > 10.0 * float(bound.norm())
