@@ -102,13 +102,13 @@ struct Level {
     int W = 0, H = 0, gw = 0, gh = 0, count = 0;
     bool roi = false;
     DeviceBuffer plane, meta, inv, links, selected;
-    // For the banded solver loop: f where the intensity plane is not it, and,
+    // For the banded solver loop: f (solver_f) is the intensity plane, or plane_f where the plane is centred, and,
     // behind the plane in its allocation, (gx, gy) and the window's pixel table.
     DeviceBuffer plane_f;
     float2 *plane_grad = nullptr;
     float4 *pixel_table = nullptr;
     std::vector<float4> host_table;
-    const float *solver_f = nullptr;
+    float *solver_f = nullptr;
     DeviceBuffer intensity, spline, scratch, valid;  // preparation scratch
     DeviceBuffer admissible;                         // u8 per subset, ROI ignored
     DeviceBuffer moments;                            // affine, quadratic row path: moments per subset
@@ -179,6 +179,7 @@ class Runtime {
     const BandPlan &band_plan(int lanes) const { return band_plans_[lanes == 16 ? 0 : (lanes == 32 ? 1 : 2)]; }
     bool banded() const { return band_plans_[0].rows > 0 || band_plans_[1].rows > 0; }
     void ensure_plane(Level &level);
+    void place_plane_f(Level &level);
     void split_plane(Level &level, bool gradients);
     void upload(const DeviceBuffer &dst, const void *src, size_t bytes, const char *what);
     // Switch the solver variant (lanes per subset, persistent queue).

@@ -276,14 +276,18 @@ void Runtime::ensure_plane(Level &level) {
                                cudaMemcpyHostToDevice, stream_), "pixel table upload");
 }
 
-// f of the plane for the banded loop: the intensity plane, or a copy where
-// the preparation centred the windows of a tiled grid in the plane.
+// f of the plane for the banded loop: the intensity plane, or, where the
+// windows of a tiled grid are centred in the plane, a copy.  Its place depends
+// on the options alone, not on the way a reference came in.
+void Runtime::place_plane_f(Level &level) {
+    DeviceBuffer &f = opt_.o.subset_stride == opt_.o.subset_size ? level.plane_f : level.intensity;
+    f.ensure((size_t)level.W * level.H * sizeof(float));
+    level.solver_f = f.as<float>();
+}
+
 void Runtime::split_plane(Level &level, bool gradients) {
-    const size_t px = (size_t)level.W * level.H;
-    level.plane_f.ensure(px * sizeof(float));
-    check_cuda(launch_split_plane(level.plane.as<float4>(), px, level.plane_f.as<float>(),
+    check_cuda(launch_split_plane(level.plane.as<float4>(), (size_t)level.W * level.H, level.solver_f,
                                   gradients ? level.plane_grad : nullptr, stream_), "plane split");
-    level.solver_f = level.plane_f.as<float>();
 }
 
 void Runtime::ensure_slots(Level &level, int slots) {
@@ -367,7 +371,7 @@ double Runtime::prepare_reference(Level &level, const uint8_t *device_image, con
     check_cuda(cudaEventCreate(&e1), "event");
     cudaEventRecord(e0, stream_);
     check_cuda(launch_reference_prep(a, stream_), "reference preparation launch");
-    level.solver_f = banded() ? level.intensity.as<float>() : nullptr;
+    if (banded()) place_plane_f(level);
     if (banded() && a.stride == a.S) split_plane(level, false);
     cudaEventRecord(e1, stream_);
     unsigned valid = 0;
@@ -399,8 +403,10 @@ void Runtime::upload_reference_arrays(Level &level, const float *plane, const fl
     level.inv.ensure((size_t)level.count * n * n * sizeof(float));
     level.partial_count = 0;
     upload(level.plane, plane, px * sizeof(float4), "plane upload");
-    level.solver_f = nullptr;
-    if (banded()) split_plane(level, true);
+    if (banded()) {
+        place_plane_f(level);
+        split_plane(level, true);
+    }
     upload(level.meta, meta, (size_t)level.count * meta_stride(model) * sizeof(float), "metadata upload");
     upload(level.inv, inverse, (size_t)level.count * n * n * sizeof(float), "inverse upload");
     level.roi = links != nullptr;

@@ -237,4 +237,11 @@ def test_uploaded_references_replace_one_another(subset, stride):
             plane, inverse, metadata = prepared[k][0]
             engine.set_reference_arrays(1280, 960, plane, metadata, inverse)
             np.testing.assert_array_equal(_packed(engine.register(frames[k][1])), prepared[k][1])
+        # and with references prepared on the engine in between
+        for k in (1, 0):
+            engine.set_reference(frames[k][0])
+            np.testing.assert_array_equal(_packed(engine.register(frames[k][1])), prepared[k][1])
+            plane, inverse, metadata = prepared[1 - k][0]
+            engine.set_reference_arrays(1280, 960, plane, metadata, inverse)
+            np.testing.assert_array_equal(_packed(engine.register(frames[1 - k][1])), prepared[1 - k][1])
     assert (prepared[0][1][..., 6] == 1.0).mean() > 0.9 and prepared[0][1][..., 6].size > 912
