@@ -190,18 +190,26 @@ __global__ void __launch_bounds__(128, kBandBlocks) final_zncc_band_kernel(Solve
 // A thread has 4 x 4 outputs: for each of its 11 source rows the four
 // horizontal sums as byte dot products of 16 bytes loaded as words, added into
 // the rows' vertical sums as they come; nothing goes through shared memory.
-// Threads whose columns are reflected or not on a word boundary gather bytes.
-// UHD: 15 us by bytes through shared memory -> 9.3 us
-// beside the prefilter that shares the frame (8.3 MB read: 1.2 us).
+// A border thread mends its one reflected word from the neighbouring one, so
+// that the words' warps do not diverge; where rows are not whole words, and in
+// the last thread of a row that its outputs do not fill, bytes are gathered
+// (a kernel of its own for the former: the word loads beside it cost it 10 to 20 %).
+// By bytes through shared memory -> here, us a launch: 3840 x 2160 21.2 -> 7.3
+// (8.3 MB read: 1.2), 1920 x 1080 7.4 -> 4.6, 640 x 360 7.0 -> 4.8, 160 x 90
+// 5.8 -> 4.2; of bytes 3839 x 2159 21.2 -> 15.3, 1919 x 1080 7.4 -> 6.5, 321 x 181
+// 7.1 -> 5.3, 81 x 45 5.1 -> 4.6.  With the border threads gathering bytes beside
+// the others' words a warp took both ways: 1920 x 1080 8.2, 640 x 360 8.1.
 constexpr int kRX = 4, kRY = 4;
 
+template <bool WORDS>  // rows are whole words
 __global__ void __launch_bounds__(128) reduce_half_kernel(const uint8_t *__restrict__ src, int W, int H,
                                                           uint8_t *__restrict__ dst) {
     const int W2 = W / 2, H2 = H / 2;
     const int X = kRX * (int)(blockIdx.x * 32 + threadIdx.x), Y = kRY * (int)(blockIdx.y * 4 + threadIdx.y);
     if (X >= W2 || Y >= H2) return;
     const int c0 = 2 * X - 4;  // the words cover columns c0 .. c0 + 15; the sums use c0 + 2 .. c0 + 12
-    const bool words = c0 >= 0 && c0 + 16 <= W && (W & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 3) == 0;
+    const bool words = WORDS && c0 + 12 <= W;
+    const int first = c0 < 0 ? 1 : 0, last = c0 + 16 <= W ? 3 : 2;  // words inside the row
     unsigned acc[kRY][kRX] = {};
 #pragma unroll
     for (int k = 0; k < 2 * kRY + 3; ++k) {
@@ -209,7 +217,10 @@ __global__ void __launch_bounds__(128) reduce_half_kernel(const uint8_t *__restr
         uint32_t w[4];
         if (words) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[q] = __ldg(reinterpret_cast<const uint32_t *>(row + c0) + q);
+            for (int q = 0; q < 4; ++q)
+                w[q] = __ldg(reinterpret_cast<const uint32_t *>(row + c0) + min(max(q, first), last));
+            if (first == 1) w[0] = __byte_perm(w[1], 0u, 0x1244);  // columns -1, -2 are 1, 2
+            if (last == 2) w[3] = __byte_perm(w[2], 0u, 0x4442);   // column W is W - 2
         } else {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -525,7 +536,11 @@ cudaError_t launch_reduce_half(const uint8_t *src, int W, int H, uint8_t *dst, c
     const int W2 = W / 2, H2 = H / 2;
     if (W2 <= 0 || H2 <= 0) return cudaSuccess;
     const int cx = 32 * kRX, cy = 4 * kRY;
-    reduce_half_kernel<<<dim3((W2 + cx - 1) / cx, (H2 + cy - 1) / cy), dim3(32, 4), 0, stream>>>(src, W, H, dst);
+    const dim3 grid((W2 + cx - 1) / cx, (H2 + cy - 1) / cy), block(32, 4);
+    if ((W & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 3) == 0)
+        reduce_half_kernel<true><<<grid, block, 0, stream>>>(src, W, H, dst);
+    else
+        reduce_half_kernel<false><<<grid, block, 0, stream>>>(src, W, H, dst);
     return cudaGetLastError();
 }
 

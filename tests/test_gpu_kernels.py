@@ -202,3 +202,22 @@ def test_reduce_half_bit_exact(width, height):
                   lib.gbdic_last_error(None))
     torch.cuda.synchronize()
     np.testing.assert_array_equal(dst.cpu().numpy(), oracle_c.reduce(img))
+
+
+@pytest.mark.parametrize("width", [4, 8, 12, 16, 20, 24, 28, 32, 36, 520, 1000])
+@pytest.mark.parametrize("height", [2, 3, 9, 16, 71])
+def test_reduce_half_of_whole_words(width, height):
+    """Rows of whole words: the border threads' reflected columns, one thread
+    with both borders, and rows whose last thread has outputs to spare."""
+    import torch
+
+    from live_dic_gb300 import _native
+
+    image = np.random.default_rng(width * height).integers(0, 256, (height, width), dtype=np.uint8)
+    lib = _native.load()
+    src = torch.from_numpy(image).cuda()
+    dst = torch.full((height // 2, width // 2), 7, dtype=torch.uint8, device="cuda")
+    _native.check(lib.gbdic_reduce_half(src.data_ptr(), width, height, dst.data_ptr(), None),
+                  lib.gbdic_last_error(None))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(dst.cpu().numpy(), oracle_c.reduce(image))
