@@ -181,6 +181,7 @@ struct SolveArgs {
     // warp), 2 wide (72 x 56).
     int staged_tile;
     BandPlan band;
+    int sm_count;
     // List mode (exact loop, complete windows): group g solves subset
     // subset_list[g] for g < count, or g < min(count, *list_count) when
     // list_count is set (a device count written by an earlier kernel).

@@ -45,12 +45,13 @@ cudaError_t launch_icgn_staged(const SolveArgs &a, int model, int lanes, bool ga
                                cudaStream_t stream, int *occupancy_only);
 int icgn_staged_occupancy(int model, int lanes, bool gauss, int tile);
 
-// Partial-support windows (a.count = number of partial windows; a.partial_index,
-// a.support, a.support_box, a.support_words set); translation and affine.
-// Few complete windows of affine and translation warps: a block to a window, as
-// the partial ones are solved (the same fields as the other loops').
+// Few complete windows of affine and translation warps: a block to a window
+// (the same fields as the other loops').
 bool icgn_blocks_fit(const SolveArgs &a, int model, int interp, int lanes);
 cudaError_t launch_icgn_blocks(const SolveArgs &args, int model, int interp, int lanes, bool gauss, cudaStream_t stream);
+// Partial-support windows (a.count = number of partial windows; a.partial_index,
+// a.support, a.support_box, a.support_words set), few of them a block each as
+// well; translation and affine.
 cudaError_t launch_icgn_partial(const SolveArgs &a, int model, int interp, int lanes, bool gauss,
                                 cudaStream_t stream);
 

@@ -45,13 +45,14 @@ constexpr int kMaxDevices = 64;
 struct DeviceScratch {
     bool ready = false;
     float *coefficients = nullptr;  // device address of g_noalloc_coefficients
+    int sm_count = 0;
 };
 DeviceScratch g_scratch[kMaxDevices];
 std::mutex g_scratch_mutex;
 
 // Once per device, with that device current: the array's device address
 // (the host-side symbol is only a stand-in) and the FIR taps.
-int scratch_for_current_device(float **coefficients, std::string &error) {
+int scratch_for_current_device(float **coefficients, int *sm_count, std::string &error) {
     int device = -1;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess || device < 0 || device >= kMaxDevices) {
@@ -75,10 +76,16 @@ int scratch_for_current_device(float **coefficients, std::string &error) {
             error = std::string("FIR taps upload failed: ") + cudaGetErrorString(err);
             return GBDIC_ECUDA;
         }
+        err = cudaDeviceGetAttribute(&s.sm_count, cudaDevAttrMultiProcessorCount, device);
+        if (err != cudaSuccess) {
+            error = std::string("device attribute: ") + cudaGetErrorString(err);
+            return GBDIC_ECUDA;
+        }
         s.coefficients = static_cast<float *>(address);
         s.ready = true;
     }
     *coefficients = s.coefficients;
+    *sm_count = s.sm_count;
     return GBDIC_OK;
 }
 
@@ -113,7 +120,8 @@ extern "C" int gbdic_register_noalloc(const gbdic_noalloc_frame *f, float *devic
                                            "-pixel scratch of gbdic_register_noalloc");
     float *coefficients = nullptr;
     std::string error;
-    const int rc = scratch_for_current_device(&coefficients, error);
+    int sm_count = 0;
+    const int rc = scratch_for_current_device(&coefficients, &sm_count, error);
     if (rc != GBDIC_OK) return fail_with(rc, error);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (f->interpolation == gbdic::kInterpBspline) {
@@ -134,6 +142,7 @@ extern "C" int gbdic_register_noalloc(const gbdic_noalloc_frame *f, float *devic
     a.roi_enabled = f->roi_enabled ? 1 : 0;
     a.use_mean = f->subset_stride != f->subset_size;
     a.div_min = 4;
+    a.sm_count = sm_count;
     cudaError_t err = gbdic::launch_icgn(a, f->motion_model, f->interpolation, f->threads_per_subset,
                                          f->weights != nullptr, 0, s);
     if (err != cudaSuccess) return fail_with(GBDIC_ECUDA, std::string("solver launch: ") + cudaGetErrorString(err));

@@ -491,6 +491,7 @@ SolveArgs Runtime::solve_args(Level &level, LevelSlot &slot, const gbdic_solver_
     a.plane_grad = level.plane_grad;
     a.pixel_table = level.pixel_table;
     a.band = band_plan(opt_.lanes);
+    a.sm_count = sm_count_;
     a.meta = level.meta.as<float>();
     a.inv = level.inv.as<float>();
     a.weights = opt_.o.spatial_weighting == 1 ? weights_.as<float>() : nullptr;

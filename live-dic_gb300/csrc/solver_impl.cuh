@@ -645,7 +645,8 @@ __device__ __forceinline__ float2 sample_bspline_pair_tile(const float *tile, in
     return value;
 }
 
-template <int MODEL, int INTERP, int LANES, bool GAUSS, int TW = 0, int TH = 0>
+// PART: partial-support ROI windows (solver_partial.cu).
+template <int MODEL, int INTERP, int LANES, bool GAUSS, bool PART = false, int TW = 0, int TH = 0>
 __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int glane, int lane_in_warp,
                                             float *red, const StageTile *st = nullptr, StageState *ss = nullptr) {
     constexpr int N = SumCount<MODEL>::value;
@@ -653,12 +654,16 @@ __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int g
     constexpr bool kClamp = MODEL == kModelQuadratic;
     // Pixel pairs with packed FP32 arithmetic: B-spline sampling of
     // complete windows.
-    constexpr bool kPair = GBDIC_SOLVER_PAIRS && INTERP == kInterpBspline &&
+    constexpr bool kPair = GBDIC_SOLVER_PAIRS && INTERP == kInterpBspline && !PART &&
                            (MODEL != kModelQuadratic || GBDIC_QUAD_PAIRS);
-    const int live = a.list_count != nullptr ? min(a.count, (int)__ldg(a.list_count)) : a.count;
+    const int live = (!PART && a.list_count != nullptr) ? min(a.count, (int)__ldg(a.list_count)) : a.count;
     const bool exists = group < live;
-    // List mode: group -> listed subset.
-    const int idx = a.subset_list != nullptr ? (exists ? __ldg(a.subset_list + group) : 0) : group;
+    // List mode: group -> listed subset.  Partial windows: group -> window
+    // index; support words and box.
+    const int idx = PART ? (exists ? __ldg(a.partial_index + group) : 0)
+                         : (a.subset_list != nullptr ? (exists ? __ldg(a.subset_list + group) : 0) : group);
+    const uint32_t *support = PART ? a.support + (size_t)(exists ? group : 0) * a.support_words : nullptr;
+    const float4 box = PART ? __ldg(a.support_box + (exists ? group : 0)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const int sidx = exists ? idx : 0;
     const float *md = a.meta + (size_t)sidx * meta_stride(MODEL);
     const float *hi = a.inv + (size_t)sidx * parameter_count(MODEL) * parameter_count(MODEL);
@@ -677,8 +682,8 @@ __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int g
     }
     if (MODEL == kModelTranslation) { w.l0 = w.l1 = w.l2 = w.l3 = 0.0f; }
     const float mvalid = __ldg(md + 1);
-    const bool valid = enabled && mvalid >= 0.5f;
-    const float rejected = a.roi_enabled ? fminf(-1.0f, mvalid) : -1.0f;
+    const bool valid = enabled && (PART ? mvalid == -4.0f : mvalid >= 0.5f);
+    const float rejected = (a.roi_enabled && !PART) ? fminf(-1.0f, mvalid) : -1.0f;
     float status = valid ? 0.0f : rejected;
     float iters = 0.0f;
     bool done = !exists;
@@ -686,8 +691,8 @@ __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int g
     const int gx = sidx % a.grid_w, gy = sidx / a.grid_w;
     const int px0 = gx * a.stride, py0 = gy * a.stride;
     const float half = 0.5f * ((float)S - 1.0f);
-    const float ref_mean = a.use_mean ? __ldg(md + (MODEL == kModelQuadratic ? 26 : 14)) : 0.0f;
-    const float wsum = GAUSS ? __ldg(md + 3 + 2 * parameter_count(MODEL)) : (float)(S * S);
+    const float ref_mean = (a.use_mean || PART) ? __ldg(md + (MODEL == kModelQuadratic ? 26 : 14)) : 0.0f;
+    const float wsum = (GAUSS || PART) ? __ldg(md + 3 + 2 * parameter_count(MODEL)) : (float)(S * S);
     float prev_change = 3.402823e38f;
     unsigned stalled = 0u;
     const int npix = S * S;
@@ -709,7 +714,8 @@ __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int g
     for (int it = 0; it < 30; ++it) {
         if (!done) {
             if (!(a.div_patience != 0 && status == 3.0f)) {
-                if (!warp_inside<MODEL>(w, px0, py0, S, half, W, H)) {
+                if (!(PART ? warp_inside_box<MODEL>(w, px0, py0, half, box, W, H)
+                           : warp_inside<MODEL>(w, px0, py0, S, half, W, H))) {
                     if (!a.roi_enabled || status > -2.5f) status = -1.0f;
                 }
             }
@@ -780,6 +786,13 @@ __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int g
                 }
             }
             for (; p < npix; p += LANES) {
+                if (PART && !((__ldg(support + (p >> 5)) >> (p & 31)) & 1u)) {
+                    fcol += flmod;
+                    frow += fldiv;
+                    ridx += rstep;
+                    if (fcol >= fS) { fcol -= fS; frow += 1.0f; ridx += rwrap; }
+                    continue;
+                }
                 const float lx = fcol - half, ly = frow - half;
                 float hx2 = 0.0f, xy = 0.0f, hy2 = 0.0f;
                 if (MODEL == kModelQuadratic) {
@@ -821,7 +834,7 @@ __device__ __forceinline__ void solve_group(const SolveArgs &a, int group, int g
     }
 }
 
-template <int MODEL, int INTERP, int LANES, bool GAUSS>
+template <int MODEL, int INTERP, int LANES, bool GAUSS, bool PART = false>
 __global__ void __launch_bounds__(128, MODEL == kModelQuadratic ? GBDIC_QUAD_MIN_BLOCKS : GBDIC_SOLVER_MIN_BLOCKS) icgn_kernel(SolveArgs a) {
     constexpr bool kBlock = LANES > 32;
     constexpr int kUnitThreads = kBlock ? 128 : 32;
@@ -836,7 +849,7 @@ __global__ void __launch_bounds__(128, MODEL == kModelQuadratic ? GBDIC_QUAD_MIN
     const int units_per_block = 128 / kUnitThreads;
     const long long unit = (long long)blockIdx.x * units_per_block + tid / kUnitThreads;
     float *red = red_smem + (kBlock ? group_in_unit * LANES * N : 0);
-    const int count = a.list_count != nullptr ? min(a.count, (int)__ldg(a.list_count)) : a.count;
+    const int count = (!PART && a.list_count != nullptr) ? min(a.count, (int)__ldg(a.list_count)) : a.count;
     for (;;) {
         int base;
         if (a.persistent) {
@@ -854,7 +867,7 @@ __global__ void __launch_bounds__(128, MODEL == kModelQuadratic ? GBDIC_QUAD_MIN
             base = unit * kGroups < (long long)count ? (int)(unit * kGroups) : count;
         }
         if (base >= count) break;
-        solve_group<MODEL, INTERP, LANES, GAUSS>(a, base + group_in_unit, glane, lane_in_warp, red);
+        solve_group<MODEL, INTERP, LANES, GAUSS, PART>(a, base + group_in_unit, glane, lane_in_warp, red);
         if (!a.persistent) break;
     }
 }

@@ -1,20 +1,21 @@
-// A block to a window: IC-GN over partial-support ROI windows, and over the
-// complete windows of a launch too small to fill the chip otherwise (reference: solve_partial /
+// IC-GN over partial-support ROI windows (reference: solve_partial /
 // solve_partial_seeded / retry_partial_seeded, shaders/icgn.wgsl:1042-1085):
-// for those, the complete-window solver's iteration with the window's support bits,
+// the complete-window solver's iteration with the window's support bits,
 // support box and partial metadata (validity -4, partial mean and weight
 // sum).  One launch over the partial windows, after the complete-window launch
-// of the same frame.
+// of the same frame.  Few windows, partial or complete, take a block each.
 //
-// Partial windows are the few along an ROI's edge, so a launch of one group of
-// lanes to a window leaves the chip nearly idle and lasts as long as one
-// window's chain: every lane took its pixels one after the other, each with its
-// taps' latency.  Here a block of 256 threads has the window.  All of them
-// sample the supported pixels and leave each pixel's factors in shared memory;
-// then lane l of the reference's LANES accumulates its pixels from there in the
-// reference's order, the sums dealt out over the 256 / LANES threads that share
-// the lane, and one warp takes the update.  Each sum's chain and the reduction
-// tree are the reference's, so the result is the same bit for bit.
+// A launch of few windows with one group of lanes to a window leaves the chip
+// nearly idle and lasts as long as one window's chain: every lane takes its
+// pixels one after the other, each with its taps' latency.  A block of 256
+// threads to a window shortens the chain.  All of them sample the supported
+// pixels and leave each pixel's factors in shared memory; then lane l of the
+// reference's LANES accumulates its pixels from there in the reference's
+// order, the sums dealt out over the 256 / LANES threads that share the lane,
+// and one warp takes the update.  Each sum's chain and the reduction tree are
+// the reference's, so the result is the same bit for bit.  Where there are
+// many windows, or a lane has few pixels, the block's synchronisations cost
+// more than the shorter chain gives (kBlockRule).
 // 1279 x 717, S 25 / s 12 Gaussian, 349 partial windows, 16 lanes: 208 us ->
 // 119 with the factors formed in the accumulation and 128 threads -> 53.
 #include "gbdic_kernels.h"
@@ -24,13 +25,6 @@ namespace gbdic {
 namespace {
 
 constexpr int kPartialThreads = 256;
-// Complete windows of a launch up to which a block has one too.  Device time of a
-// frame, other loops -> blocks (16 lanes): affine B-spline S 21, 324 windows 81 ->
-// 73 us, 676 120 -> 110, 1,156 126 -> 133; S 31 88 -> 58, 103 -> 77, 101 -> 92,
-// 1,764 134 -> 127, 2,704 128 -> 161; affine linear S 21 (direct loop) 676 98 -> 64,
-// 1,764 124 -> 93, 2,704 125 -> 119, 4,356 138 -> 154; translation linear S 15 676
-// 73 -> 53, 1,764 75 -> 66, 2,704 77 -> 79.
-constexpr int kBlockWindowsBspline = 912, kBlockWindows = 2128;
 // Pixels sampled between two accumulations: a multiple of the lane counts (lanes
 // keep their pixels); a whole window up to S = 32.  The arrays' pitch puts the
 // two halves of a warp, which read different arrays, on different banks.
@@ -228,51 +222,114 @@ __global__ void __launch_bounds__(kPartialThreads) window_block_kernel(SolveArgs
     }
 }
 
+// Windows up to which a block each is faster than a group of lanes each: per SM
+// gain * (pixels - start)^2, at most `most`, where `pixels` are a lane's (the
+// chain that a block shortens) and `start` those that its synchronisations
+// outweigh.  Fitted to measurements over S 5 to 81, 9 to 4,096 complete and 15 to
+// 6,300 partial windows: of 5,000 frames 84 are over 3 % slower than the better
+// of the two.  The measured device times of a frame (with its prefilter), a group
+// of lanes each : a block each, affine, us:
+//   complete, 16 lanes   B-spline S 9    196 windows  72 : 70         900  75 : 108
+//                                 S 15   900         112 : 114      2,116  127 : 164
+//                                 S 31   900         102 : 69       2,116  103 : 107
+//                        linear   S 9    196          55 : 57       2,116  61 : 158
+//                                 S 31   900          83 : 45       3,364  110 : 113
+//                        cubic    S 15   900         130 : 92       4,096  218 : 227
+//   complete, 32 lanes   B-spline S 15   196          75 : 70         900  88 : 113
+//                                 S 31   900          80 : 73       1,444  81 : 92
+//                        linear   S 15   196          58 : 65       2,116  75 : 132
+//   partial, 16 lanes    B-spline S 9  1,007          95 : 135         S 15  999  161 : 113
+//                        linear   S 9  1,006          68 : 111         S 15  999  107 : 89
+//   partial, 32 lanes    B-spline S 9  1,007          81 : 143         S 31  988  134 : 82
+//   partial, 64 lanes    B-spline S 9    391          94 : 93          S 31  988  100 : 85
+//                                 S 9  1,007         109 : 155         S 31  2,268  135 : 151
+// 128 lanes: partial windows 0.95 to 1.5 times as long by blocks; complete windows
+// of 64 and 128 lanes have a block's loop in any case.
+struct BlockRule {
+    float start, gain, most;
+};
+enum { kComplete16, kComplete32, kPartial16, kPartial32, kPartial64, kBlockRules };
+// [launch][affine, translation][B-spline, linear, cubic]
+constexpr BlockRule kBlockRule[kBlockRules][2][3] = {
+    {{{1.0f, 0.045f, 6.0f}, {1.0f, 0.045f, 14.0f}, {1.0f, 0.12f, 14.0f}},
+     {{1.0f, 0.3f, 6.0f}, {2.0f, 0.15f, 14.0f}, {2.0f, 0.4f, 14.0f}}},
+    {{{2.0f, 0.06f, 6.0f}, {6.0f, 0.06f, 8.0f}, {2.0f, 0.09f, 10.0f}},
+     {{3.0f, 0.7f, 5.0f}, {2.0f, 0.09f, 12.0f}, {3.0f, 1.5f, 10.0f}}},
+    {{{0.0f, 0.09f, 42.0f}, {0.0f, 0.06f, 28.0f}, {0.0f, 0.09f, 42.0f}},
+     {{0.0f, 0.3f, 42.0f}, {0.0f, 0.15f, 42.0f}, {0.0f, 0.4f, 42.0f}}},
+    {{{1.0f, 0.15f, 16.0f}, {2.0f, 0.09f, 16.0f}, {1.0f, 0.15f, 16.0f}},
+     {{2.0f, 1.0f, 16.0f}, {2.0f, 0.3f, 16.0f}, {2.0f, 0.7f, 16.0f}}},
+    {{{0.0f, 1.5f, 7.0f}, {0.0f, 1.5f, 5.0f}, {0.0f, 1.5f, 5.0f}},
+     {{0.0f, 1.5f, 7.0f}, {1.0f, 1.5f, 7.0f}, {1.0f, 1.5f, 3.0f}}},
+};
+
+bool block_each(const SolveArgs &a, int model, int interp, int lanes, bool partial) {
+    if (model == kModelQuadratic || lanes > (partial ? 64 : 32)) return false;
+    const int launch = partial ? (lanes == 16 ? kPartial16 : lanes == 32 ? kPartial32 : kPartial64)
+                               : (lanes == 16 ? kComplete16 : kComplete32);
+    const BlockRule &r = kBlockRule[launch][model == kModelTranslation ? 1 : 0]
+                                   [interp == kInterpBspline ? 0 : interp == kInterpLinear ? 1 : 2];
+    const float excess = fmaxf((float)(a.S * a.S) / (float)lanes - r.start, 0.0f);
+    return (float)a.count <= fminf(r.gain * excess * excess, r.most) * (float)a.sm_count;
+}
+
+// blocks: a block to a window; else a group of LANES lanes to a partial one.
 template <int MODEL, int INTERP, int LANES, bool GAUSS>
-cudaError_t go(const SolveArgs &a, cudaStream_t s) {
-    if (a.partial_index != nullptr)
-        window_block_kernel<MODEL, INTERP, LANES, GAUSS, true><<<a.count, kPartialThreads, 0, s>>>(a);
-    else
+cudaError_t go(const SolveArgs &a, bool blocks, cudaStream_t s) {
+    if (a.partial_index != nullptr && !blocks) {
+        icgn_kernel<MODEL, INTERP, LANES, GAUSS, true><<<icgn_grid(a.count, LANES), 128, 0, s>>>(a);
+        return cudaGetLastError();
+    }
+    if constexpr (LANES <= 64) {
+        if (a.partial_index != nullptr) {
+            window_block_kernel<MODEL, INTERP, LANES, GAUSS, true><<<a.count, kPartialThreads, 0, s>>>(a);
+            return cudaGetLastError();
+        }
+    }
+    if constexpr (LANES <= 32) {
         window_block_kernel<MODEL, INTERP, LANES, GAUSS, false><<<a.count, kPartialThreads, 0, s>>>(a);
-    return cudaGetLastError();
+        return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
 }
 
 template <int MODEL, int INTERP, bool GAUSS>
-cudaError_t by_lanes(const SolveArgs &a, int lanes, cudaStream_t s) {
+cudaError_t by_lanes(const SolveArgs &a, int lanes, bool blocks, cudaStream_t s) {
     switch (lanes) {
-    case 16: return go<MODEL, INTERP, 16, GAUSS>(a, s);
-    case 32: return go<MODEL, INTERP, 32, GAUSS>(a, s);
-    case 64: return go<MODEL, INTERP, 64, GAUSS>(a, s);
-    case 128: return go<MODEL, INTERP, 128, GAUSS>(a, s);
+    case 16: return go<MODEL, INTERP, 16, GAUSS>(a, blocks, s);
+    case 32: return go<MODEL, INTERP, 32, GAUSS>(a, blocks, s);
+    case 64: return go<MODEL, INTERP, 64, GAUSS>(a, blocks, s);
+    case 128: return go<MODEL, INTERP, 128, GAUSS>(a, blocks, s);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <int MODEL, bool GAUSS>
-cudaError_t by_interp(const SolveArgs &a, int interp, int lanes, cudaStream_t s) {
+cudaError_t by_interp(const SolveArgs &a, int interp, int lanes, bool blocks, cudaStream_t s) {
     switch (interp) {
-    case kInterpBspline: return by_lanes<MODEL, kInterpBspline, GAUSS>(a, lanes, s);
-    case kInterpLinear: return by_lanes<MODEL, kInterpLinear, GAUSS>(a, lanes, s);
-    case kInterpKeys: return by_lanes<MODEL, kInterpKeys, GAUSS>(a, lanes, s);
+    case kInterpBspline: return by_lanes<MODEL, kInterpBspline, GAUSS>(a, lanes, blocks, s);
+    case kInterpLinear: return by_lanes<MODEL, kInterpLinear, GAUSS>(a, lanes, blocks, s);
+    case kInterpKeys: return by_lanes<MODEL, kInterpKeys, GAUSS>(a, lanes, blocks, s);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <int MODEL>
-cudaError_t by_weight(const SolveArgs &a, int interp, int lanes, bool gauss, cudaStream_t s) {
-    return gauss ? by_interp<MODEL, true>(a, interp, lanes, s) : by_interp<MODEL, false>(a, interp, lanes, s);
+cudaError_t by_weight(const SolveArgs &a, int interp, int lanes, bool gauss, bool blocks, cudaStream_t s) {
+    return gauss ? by_interp<MODEL, true>(a, interp, lanes, blocks, s)
+                 : by_interp<MODEL, false>(a, interp, lanes, blocks, s);
 }
 
 }  // namespace
 
 bool icgn_blocks_fit(const SolveArgs &a, int model, int interp, int lanes) {
-    return model != kModelQuadratic && lanes <= 32 && !a.persistent && a.subset_list == nullptr &&
-           a.list_count == nullptr && a.count <= (interp == kInterpBspline ? kBlockWindowsBspline : kBlockWindows);
+    return !a.persistent && a.subset_list == nullptr && a.list_count == nullptr &&
+           block_each(a, model, interp, lanes, false);
 }
 
-cudaError_t launch_icgn_blocks(const SolveArgs &args, int model, int interp, int lanes, bool gauss, cudaStream_t stream) {
-    return model == kModelAffine ? by_weight<kModelAffine>(args, interp, lanes, gauss, stream)
-                                 : by_weight<kModelTranslation>(args, interp, lanes, gauss, stream);
+cudaError_t launch_icgn_blocks(const SolveArgs &a, int model, int interp, int lanes, bool gauss, cudaStream_t stream) {
+    return model == kModelAffine ? by_weight<kModelAffine>(a, interp, lanes, gauss, true, stream)
+                                 : by_weight<kModelTranslation>(a, interp, lanes, gauss, true, stream);
 }
 
 cudaError_t launch_icgn_partial(const SolveArgs &args, int model, int interp, int lanes, bool gauss,
@@ -280,9 +337,12 @@ cudaError_t launch_icgn_partial(const SolveArgs &args, int model, int interp, in
     if (args.count <= 0) return cudaSuccess;
     if (!args.partial_index || !args.support || !args.support_box || args.support_words <= 0)
         return cudaErrorInvalidValue;
+    SolveArgs a = args;
+    a.persistent = 0;
+    const bool blocks = block_each(a, model, interp, lanes, true);
     switch (model) {
-    case kModelAffine: return by_weight<kModelAffine>(args, interp, lanes, gauss, stream);
-    case kModelTranslation: return by_weight<kModelTranslation>(args, interp, lanes, gauss, stream);
+    case kModelAffine: return by_weight<kModelAffine>(a, interp, lanes, gauss, blocks, stream);
+    case kModelTranslation: return by_weight<kModelTranslation>(a, interp, lanes, gauss, blocks, stream);
     default: return cudaErrorInvalidValue;  // the ROI supports translation and affine windows only
     }
 }

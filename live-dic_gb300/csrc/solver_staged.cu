@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(128, GBDIC_SOLVER_MIN_BLOCKS)
             base = unit * kGroups < (long long)a.count ? (int)(unit * kGroups) : a.count;
         }
         if (base >= a.count) break;
-        solve_group<MODEL, kInterpBspline, LANES, GAUSS, TW, TH>(a, base + group_in_warp, glane, lane, nullptr,
+        solve_group<MODEL, kInterpBspline, LANES, GAUSS, false, TW, TH>(a, base + group_in_warp, glane, lane, nullptr,
                                                                           &st, &ss);
         if (!a.persistent) break;
     }

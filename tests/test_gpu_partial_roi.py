@@ -153,3 +153,34 @@ def test_selective_recovery_keeps_partial_policy(pair):
     cut = np.zeros(info.roi.selected.shape, bool)
     cut.ravel()[info.roi.partial_indices] = True
     assert (result.status[cut] == 1).mean() > 0.8
+
+
+@pytest.mark.parametrize("lanes", [16, 32, 64, 128])
+@pytest.mark.parametrize("model,interp,weighting,subset,stride", [
+    ("affine", "bspline", "uniform", 9, 4), ("affine", "cubic", "gaussian", 7, 5), ("affine", "linear", "uniform", 11, 4),
+    ("translation", "bspline", "gaussian", 8, 4), ("translation", "linear", "uniform", 7, 4)])
+def test_many_small_partial_windows_bit_exact(pair, model, interp, weighting, subset, stride, lanes):
+    """More small windows cut by the mask than take a block each (holes all over
+    the specimen): a group of lanes each, against the oracle."""
+    ref, tgt = pair
+    mask = np.ones(ref.shape, bool)
+    for y in range(2, H, subset):
+        for x in range(3, W, subset):
+            mask[y:y + 1 + y % 2, x:x + 1 + x % 3] = False
+    with ICGNWGPU(subset_size=subset, subset_stride=stride, motion_model=model, interpolation=interp,
+                  spatial_weighting=weighting, outlier_policy="disabled", solver_workgroup_size=lanes) as engine:
+        info = engine.set_reference(ref, roi_mask=mask, roi_policy="partial")
+        result = engine.register(tgt)
+        plane, inverse, metadata = engine.export_reference()
+        coef = engine.export_coefficients() if interp == "bspline" else None
+        weights = engine.export_weights() if weighting == "gaussian" else None
+    plan = info.roi
+    kw = dict(subset_size=subset, subset_stride=stride, model=model, interpolation=interp, lanes=lanes,
+              roi_enabled=True, weights=weights)
+    state = oracle_c.solve(tgt, coef, plane, metadata, inverse, **kw)
+    state = oracle_c.solve(tgt, coef, plane, metadata, inverse, state=state,
+                           partial=(plan.partial_indices, plan.support_words, plan.support_boxes), **kw)
+    got = _packed(result)
+    np.testing.assert_array_equal(got, state.reshape(got.shape[0], got.shape[1], -1)[..., : got.shape[-1]])
+    assert plan.partial_indices.size > 1100
+    assert (got.reshape(-1, got.shape[-1])[plan.partial_indices, 6] == 1).sum() > 100
