@@ -253,8 +253,8 @@ enum { kComplete16, kComplete32, kPartial16, kPartial32, kPartial64, kBlockRules
 constexpr BlockRule kBlockRule[kBlockRules][2][3] = {
     {{{1.0f, 0.045f, 6.0f}, {1.0f, 0.045f, 14.0f}, {1.0f, 0.12f, 14.0f}},
      {{1.0f, 0.3f, 6.0f}, {2.0f, 0.15f, 14.0f}, {2.0f, 0.4f, 14.0f}}},
-    {{{2.0f, 0.06f, 6.0f}, {6.0f, 0.06f, 8.0f}, {2.0f, 0.09f, 10.0f}},
-     {{3.0f, 0.7f, 5.0f}, {2.0f, 0.09f, 12.0f}, {3.0f, 1.5f, 10.0f}}},
+    {{{2.0f, 0.06f, 6.0f}, {6.0f, 0.06f, 7.0f}, {2.0f, 0.09f, 10.0f}},
+     {{3.0f, 0.7f, 5.0f}, {2.0f, 0.09f, 10.0f}, {3.0f, 1.5f, 10.0f}}},
     {{{0.0f, 0.09f, 42.0f}, {0.0f, 0.06f, 28.0f}, {0.0f, 0.09f, 42.0f}},
      {{0.0f, 0.3f, 42.0f}, {0.0f, 0.15f, 42.0f}, {0.0f, 0.4f, 42.0f}}},
     {{{1.0f, 0.15f, 16.0f}, {2.0f, 0.09f, 16.0f}, {1.0f, 0.15f, 16.0f}},
