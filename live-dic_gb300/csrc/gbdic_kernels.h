@@ -22,7 +22,7 @@ int icgn_grid(int count, int lanes);
 int icgn_band_grid(const SolveArgs &a, int lanes);
 // The banded loop's plan for complete B-spline windows of side S, or rows 0
 // where the direct loop is the better one.
-BandPlan plan_bands(int S, int model, int interp, int lanes, int sm_count);
+BandPlan plan_bands(int S, int model, int interp, int lanes, bool gauss, int sm_count);
 // Resident CTAs per SM of the solver variant (for persistent grids).
 int icgn_occupancy(int model, int interp, int lanes, bool gauss, int S, const BandPlan &band);
 cudaError_t launch_icgn(const SolveArgs &a, int model, int interp, int lanes, bool gauss,

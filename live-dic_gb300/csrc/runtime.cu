@@ -173,7 +173,9 @@ Runtime::Runtime(const gbdic_options &options) {
     axis_weights_.ensure(axis.size() * sizeof(float));
     upload(axis_weights_, axis.data(), axis.size() * sizeof(float), "axis weights upload");
     check_cuda(cudaStreamSynchronize(stream_), "weights upload");
-    for (int k = 0; k < 2; ++k) band_plans_[k] = plan_bands(S, options.motion_model, options.interpolation, 16 << k, sm_count_);
+    for (int k = 0; k < 2; ++k)
+        band_plans_[k] = plan_bands(S, options.motion_model, options.interpolation, 16 << k,
+                                    options.spatial_weighting == 1, sm_count_);
     if (options.persistent) persistent_grid(opt_.lanes);
 }
 

@@ -76,7 +76,7 @@ static double band_steps(int S, int rows, int samplers, int &run, int &segments)
     return best;
 }
 
-BandPlan plan_bands(int S, int model, int interp, int lanes, int sm_count) {
+BandPlan plan_bands(int S, int model, int interp, int lanes, bool gauss, int sm_count) {
     BandPlan best{};
     if (interp != kInterpBspline || lanes > 32 || S > kMaxBandFloats) return best;
     double steps = 1e30;
@@ -97,8 +97,16 @@ BandPlan plan_bands(int S, int model, int interp, int lanes, int sm_count) {
     // (S 31), 0.94 at 1.20 (S 41), 1.00 at 1.26 (S 51), 1.03 at 1.34 (S 33),
     // 1.08 at 1.49 (S 65); 32 lanes 0.95 at 1.31 (S 16), 1.02 at 1.35 (S 51);
     // translation and quadratic 0.82 and 0.85 at 1.49, and with 32 lanes 1.11
-    // and 1.04 at 1.70.
-    const double limit = model != kModelAffine ? 1.6 : (lanes == 16 ? 1.25 : 1.34);
+    // and 1.04 at 1.70.  Affine plans of several bands lose their lead sooner,
+    // with Gaussian weights (which the direct loop loads beside the plane, the
+    // banded one with its pixel table) later.  8,800 windows, band / direct,
+    // uniform and Gaussian: 16 lanes 0.99 and 0.83 at 1.20 (S 41), 1.04 and 0.90
+    // at 1.23 (S 45); 32 lanes 0.96 and 0.90 at 1.22 (S 41), 1.03 and 0.96 at 1.29
+    // (S 55), 1.02 and 0.95 at 1.31 (S 45), 1.13 and 1.04 at 1.33 (S 81).
+    const bool several = best.rows < S;
+    const double limit = model != kModelAffine ? 1.6
+                         : lanes == 16         ? (several && !gauss ? 1.21 : 1.25)
+                                               : (several ? (gauss ? 1.32 : 1.25) : 1.34);
     if (steps * 2 * lanes > limit * S * S) return BandPlan{};
     band_steps(S, best.rows, 32, best.run32, best.segments32);
     best.magic = ((1u << 20) + S - 1) / S;
