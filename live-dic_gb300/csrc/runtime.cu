@@ -7,6 +7,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
@@ -41,22 +42,55 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
 
 void fail(int code, const std::string &message) { throw Failure{code, message}; }
 
-// Bounded host wait on an event (GBDIC_ETIMEOUT after `timeout_ms`).
 // A call's launches are waited for by asking again at once for two
 // milliseconds (a frame's time; a sleep, however short, returns 50-70 us later
 // with the kernel's timer slack, a quarter of a small frame's call), then with
-// sleeps between.
-constexpr double kSpinMs = 2.0;
+// sleeps between.  Asking keeps a core busy, so at most a quarter of the
+// machine's cores do that for so long at once; callers beyond them sleep after a
+// fifth of a millisecond, a small frame's wait.
+// 16 cores, time a call over all callers and CPU time a call, us: 512 x 512, one
+// caller 349 / 134 with sleeps alone -> 196 / 196; 1920 x 1080, eight callers 392 /
+// 446 -> 301 / 1,408 (2,110 with all of them asking).
+constexpr double kSpinMs = 2.0, kShortSpinMs = 0.2;
 
+namespace {
+
+class SpinSlot {
+  public:
+    SpinSlot() : held_(used_.fetch_add(1, std::memory_order_relaxed) < limit()) {
+        if (!held_) used_.fetch_sub(1, std::memory_order_relaxed);
+    }
+    ~SpinSlot() { release(); }
+    bool held() const { return held_; }
+    void release() {
+        if (held_) used_.fetch_sub(1, std::memory_order_relaxed);
+        held_ = false;
+    }
+
+  private:
+    static int limit() {
+        static const int cores = (int)std::thread::hardware_concurrency();
+        return std::max(1, cores / 4);
+    }
+    static std::atomic<int> used_;
+    bool held_;
+};
+std::atomic<int> SpinSlot::used_{0};
+
+}  // namespace
+
+// Bounded host wait on an event (GBDIC_ETIMEOUT after `timeout_ms`).
 void wait_event(cudaEvent_t ev, double timeout_ms) {
     const auto t0 = std::chrono::steady_clock::now();
+    SpinSlot spin;
     for (;;) {
         cudaError_t err = cudaEventQuery(ev);
         if (err == cudaSuccess) return;
         if (err != cudaErrorNotReady) check_cuda(err, "device execution");
         const double waited = ms_since(t0);
         if (waited > timeout_ms) fail(GBDIC_ETIMEOUT, "device work did not complete within the wait limit");
-        if (waited < kSpinMs) std::this_thread::yield();
+        if (waited >= kSpinMs) spin.release();
+        if (spin.held() || waited < kShortSpinMs) std::this_thread::yield();
         else std::this_thread::sleep_for(std::chrono::microseconds(20));
     }
 }

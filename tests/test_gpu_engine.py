@@ -245,3 +245,43 @@ def test_uploaded_references_replace_one_another(subset, stride):
             engine.set_reference_arrays(1280, 960, plane, metadata, inverse)
             np.testing.assert_array_equal(_packed(engine.register(frames[1 - k][1])), prepared[1 - k][1])
     assert (prepared[0][1][..., 6] == 1.0).mean() > 0.9 and prepared[0][1][..., 6].size > 912
+
+
+def test_waiting_callers_leave_cores_free():
+    """Callers that wait at the same time: at most a quarter of the cores keep
+    asking for the whole of a frame's time (half of the cores have a caller)."""
+    import os
+    import threading
+    import time
+
+    cores = len(os.sched_getaffinity(0))
+    if cores < 16 or cores != os.cpu_count():
+        pytest.skip("needs 16 cores of its own")
+    callers = cores // 2
+    ref, sp = synthetic.reference_image(1920, 1080, seed=93, device="cpu")
+    tgt = synthetic.deformed_image(sp, synthetic.affine_field(0.4, 1e-3, 0.0, -0.3, 0.0, -6e-4), noise_seed=94,
+                                   device="cpu")
+    engines = [ICGNWGPU(subset_size=21, subset_stride=10) for _ in range(callers)]
+    busy = []
+    try:
+        for engine in engines:
+            engine.set_reference(ref)
+            engine.register(tgt)
+
+        def run(engine, until):
+            while time.perf_counter() < until:
+                engine.register(tgt)
+
+        for _ in range(3):
+            wall, cpu = time.perf_counter(), time.process_time()
+            threads = [threading.Thread(target=run, args=(engine, wall + 0.5)) for engine in engines]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+            busy.append((time.process_time() - cpu) / (time.perf_counter() - wall))
+    finally:
+        for engine in engines:
+            engine.close()
+    # the quarter, and copies, results and short waits of the others
+    assert min(busy) < cores / 4 + 2, busy
