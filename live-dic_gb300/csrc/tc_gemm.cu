@@ -826,7 +826,6 @@ bool make_map(CUtensorMap *map, const void *ptr, int rows, int cols, int box_row
 // ring is as deep as their shared memory allows, whatever the length of a tile's
 // K loop: it runs on into the next tile, whose gathering and MMAs overlap this
 // one's epilogue.
-constexpr int kSms = 152;
 constexpr int kRingBytes = 216 * 1024;  // of an SM's 227 KB, beside the CTAs' static arrays
 
 template <int BN>
@@ -834,21 +833,22 @@ cudaError_t launch_bn(const CUtensorMap &ma, const CUtensorMap &mb, const TcGemm
     TcGemmArgs a = args;
     constexpr int kStageBytes = kBM * kBK * 2 + BN * kBK * 2;
     const long long tiles = (long long)(a.N / BN) * (a.M / kBM) * a.k_split;
-    const int per_sm = tiles > kSms ? 2 : 1;
-    a.ring = kRingBytes / per_sm / kStageBytes < kStages ? kRingBytes / per_sm / kStageBytes : kStages;
-    const size_t smem = (size_t)a.ring * kStageBytes + 1024;
     const size_t smem_max = (size_t)kStages * kStageBytes + 1024;
     // The attribute is per device; set it once per device and tile width.
-    static thread_local int configured_device = -1;
+    static thread_local int configured_device = -1, sms = 0;
     int device = 0;
     cudaError_t err = cudaGetDevice(&device);
     if (err != cudaSuccess) return err;
     if (configured_device != device) {
         err = cudaFuncSetAttribute(tc_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+        if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         if (err != cudaSuccess) return err;
         configured_device = device;
     }
-    const int grid = (int)(tiles < 2 * kSms ? tiles : 2 * kSms);
+    const int per_sm = tiles > sms ? 2 : 1;
+    a.ring = kRingBytes / per_sm / kStageBytes < kStages ? kRingBytes / per_sm / kStageBytes : kStages;
+    const size_t smem = (size_t)a.ring * kStageBytes + 1024;
+    const int grid = (int)(tiles < 2 * sms ? tiles : 2 * sms);
     tc_gemm_kernel<BN><<<grid, kGemmThreads, smem, stream>>>(ma, mb, a);
     return cudaGetLastError();
 }
