@@ -280,3 +280,105 @@ def test_weight_gradient_with_a_reduction_of_any_length(B, H, Cin, Cout, Kp, spl
         bound = rows * 2.0 ** -24 * (part.abs().T @ z.abs())
         assert bool(((partial[s].double() - part.T @ z).abs() <= bound).all())
     assert bool((partial[splits] == 7.0).all())
+
+
+def _chunks(M):
+    """Row ranges whose tiles have a CTA each."""
+    return [(m, min(m + 128 * 64, M)) for m in range(0, M, 128 * 64)]
+
+
+def _many(tiles):
+    """Every CTA (two to an SM) takes three tiles or more, the last round uneven."""
+    ctas = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert tiles > 2 * ctas and tiles % ctas
+    return True
+
+
+@pytest.mark.parametrize("N,K", [(128, 128), (64, 320), (32, 64), (16, 192)])
+def test_gemm_of_many_tiles(N, K):
+    """The ring, the two accumulators and their hand-back through a CTA's tiles:
+    the product of the same rows a tile to a CTA, bit for bit."""
+    M = 128 * 701
+    assert _many(701)
+    a, b, ref = _operands(M, N, K, N + K)
+    want = torch.empty(M, N, device="cuda")
+    for lo, hi in _chunks(M):
+        _gemm(a[lo:hi], b, d_f32=want[lo:hi])
+    assert (want - ref).abs().max().item() <= 2e-3 * ref.abs().max().item()
+    got, got16 = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    bias = torch.randn(N, device="cuda")
+    _gemm(a, b, d_f32=got)
+    assert torch.equal(got, want)
+    _gemm(a, b, d_f32=got, d_bf16=got16, bias=bias, relu=True)
+    assert torch.equal(got, torch.relu(want + bias))
+    assert torch.equal(got16, got.to(torch.bfloat16))
+    split = torch.empty(2, M, N, device="cuda") if K % 128 == 0 else None
+    if split is not None:
+        _gemm(a, b, d_f32=split, k_split=2, split_stride=M * N)
+        for s in range(2):
+            part = torch.empty(M, N, device="cuda")
+            half = slice(s * K // 2, (s + 1) * K // 2)
+            x, w = a[:, half].contiguous(), b[:, half].contiguous()
+            for lo, hi in _chunks(M):
+                _gemm(x[lo:hi], w, d_f32=part[lo:hi])
+            assert torch.equal(split[s], part)
+
+
+@pytest.mark.parametrize("B,H,Cin,Cout", [(344, 32, 32, 64), (352, 32, 8, 128), (1376, 16, 64, 64)])
+def test_implicit_im2col_gemm_of_many_tiles(B, H, Cin, Cout):
+    lib = _native.load()
+    shape, g = _conv_case(B, H, Cin, Cout, B + Cin)
+    M = B * shape.OH * shape.OW
+    assert M % 128 == 0 and _many(M // 128)
+    x = torch.randn(B, H, H, Cin, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(Cout, shape.Kp, generator=g, device="cuda").to(torch.bfloat16)
+    a = torch.empty(M, shape.Kp, dtype=torch.bfloat16, device="cuda")
+    _native.check(lib.gbdic_nn_im2col(C.byref(shape), C.c_void_p(x.data_ptr()), C.c_void_p(a.data_ptr()), None),
+                  lib.gbdic_last_error(None))
+    want = torch.empty(M, Cout, device="cuda")
+    for lo, hi in _chunks(M):
+        _gemm(a[lo:hi], w, d_f32=want[lo:hi])
+    got = torch.empty(M, Cout, device="cuda")
+    _conv_gemm(x, w, 1, shape, M, shape.Kp, got)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("B,H,Cin,Cout", [(84, 32, 32, 64), (84, 32, 64, 128), (384, 15, 16, 64)])
+def test_data_gradients_of_many_tiles(B, H, Cin, Cout):
+    """By parity classes and, with the odd side, plain; with the ReLU mask's
+    column sums of every tile (class tiles hold one parity's pixels)."""
+    lib = _native.load()
+    shape, g = _conv_case(B, H, Cin, Cout, B + Cout)
+    OH, Min = shape.OH, B * H * H
+    assert Min % 128 == 0 and _many(Min // 128)
+    dz = torch.randn(B, OH, OH, Cout, generator=g, device="cuda").to(torch.bfloat16)
+    wt = torch.randn(Cin, 9 * Cout, generator=g, device="cuda").to(torch.bfloat16)
+    gmat = torch.empty(Min, 9 * Cout, dtype=torch.bfloat16, device="cuda")
+    _native.check(lib.gbdic_nn_dgrad_gather(C.byref(shape), C.c_void_p(dz.data_ptr()), C.c_void_p(gmat.data_ptr()),
+                                            None), lib.gbdic_last_error(None))
+    want = torch.empty(Min, Cin, device="cuda")
+    for lo, hi in _chunks(Min):
+        _gemm(gmat[lo:hi], wt, d_f32=want[lo:hi])
+    got = torch.empty(Min, Cin, device="cuda")
+    _conv_gemm(dz, wt, 2, shape, Min, 9 * Cout, got)
+    assert torch.equal(got, want)
+    y = torch.relu(torch.randn(Min, Cin, generator=g, device="cuda")).to(torch.bfloat16)
+    out = torch.full((Min, Cin), 7.0, dtype=torch.bfloat16, device="cuda")
+    partial = torch.full((Cin, Min // 128), 7.0, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    desc = _native.NnGemmDesc(dz.data_ptr(), wt.data_ptr(), Min, Cin, 9 * Cout, 1, None, out.data_ptr(), Cin, 0, None,
+                              0, 0)
+    _native.check(lib.gbdic_nn_conv_dgrad_relu(C.byref(desc), C.byref(shape), C.c_void_p(y.data_ptr()),
+                                               C.c_void_p(partial.data_ptr()), None, C.c_void_p(err.data_ptr()), None),
+                  lib.gbdic_last_error(None))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    masked = torch.where(y > 0, want, torch.zeros_like(want))
+    assert torch.equal(out, masked.to(torch.bfloat16))
+    rows = masked.double()
+    if H % 2 == 0:
+        image = rows.view(B, H, H, Cin)
+        rows = torch.cat([image[:, py::2, px::2].reshape(-1, Cin) for py in range(2) for px in range(2)])
+    tiles = rows.view(-1, 128, Cin)
+    bound = 128 * 2.0 ** -24 * tiles.abs().sum(1)
+    assert bool(((partial.double().T - tiles.sum(1)).abs() <= bound).all())

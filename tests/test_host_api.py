@@ -428,3 +428,22 @@ def test_uploads_follow_their_stream():
             if call.group(1) != "cudaMemcpy" or "cudaMemcpyHostToDevice" in call.group(2):
                 found.append(f"{path.name}:{text.count(chr(10), 0, call.start()) + 1}")
     assert found == []
+
+
+@pytest.mark.parametrize("count", [0, 1, 5, 3000])
+def test_field_summary_gathers_the_accepted_subsets(count):
+    """The selection that the field's means are taken over, in grid order."""
+    lib = _native.load()
+    rng = np.random.default_rng(count)
+    packed = np.zeros((max(count, 1), 8), np.float32)
+    packed[:count] = rng.normal(0, 1, (count, 8))
+    packed[:count, 6] = rng.choice(np.array([1.0, 2.0, 0.0, -1.0], np.float32), count)
+    picked = np.full((3, max(count, 1)), 7.0, np.float32)
+    accepted, replaced = ctypes.c_int64(-1), ctypes.c_int64(-1)
+    _native.check(lib.gbdic_field_summary(
+        _native.ptr(packed), count, 8, 6, _native.ptr(picked[0]), _native.ptr(picked[1]), _native.ptr(picked[2]),
+        ctypes.byref(accepted), ctypes.byref(replaced)), lib.gbdic_last_error(None))
+    keep = packed[:count][packed[:count, 6] > 0.5]
+    assert accepted.value == len(keep) and replaced.value == int((keep[:, 6] > 1.5).sum())
+    for row, column in enumerate((0, 3, 7)):
+        np.testing.assert_array_equal(picked[row, :len(keep)], keep[:, column])
