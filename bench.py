@@ -389,7 +389,7 @@ def run_batch_workload(args) -> None:
     accepted = sum(int((r.status >= 1).sum()) for r in results)
     summary = clocks.summary()
     line = {
-        "metric": "batched uneven workload subsets/s (one persistent launch over every job vs one launch per pair)",
+        "metric": "batched uneven workload subsets/s (one captured step over every job vs one launch per pair)",
         "value": value,
         "unit": "subsets/s",
         "n_gpus": world,
@@ -415,8 +415,11 @@ def run_batch_workload(args) -> None:
         "accepted_fraction": accepted / max(1, selected),
         "tuning_ms": batch.tuning_ms or None,
         "clocks": {"sm_mhz": summary["sm_mhz"], "sm_max_mhz": summary["sm_max_mhz"], "reasons": summary["reasons"]},
-        "gpu_launches": (2 * len(batch.jobs) + 1) * args.steps,
-        "roofline": {"bound": "fp32", "kernel": "icgn_band_kernel / icgn_kernel (a launch per job, concurrent) or icgn_batch_any_kernel",
+        # a prefilter and an outlier pass per job beside the solver's launches
+        "gpu_launches": (2 * len(batch.jobs) + batch.solver_launches) * args.steps,
+        "roofline": {"bound": "fp32",
+                     "kernel": "icgn_batch_any_kernel (every job, shape function per job)" if batch.solver_launches == 1
+                     else "icgn_band_kernel, icgn_kernel, window_block_kernel (a launch per job, concurrent)",
                      "achieved": achieved, "peak": peak.value, "unit": "TFLOP/s", "frac": achieved / peak.value,
                      "solver_ms": solver_ms, "flops_per_step": flops, "traffic": None},
         "e2e": {"value": selected / e2e_s, "unit": "subsets/s",
@@ -896,7 +899,8 @@ def main() -> None:
         traffic = json.loads(traffic_file.read_text()).get("icgn_solver_dram_bytes_per_launch")
     roofline = {
         "bound": "fp32",
-        "kernel": {"exact": "icgn_band_kernel" if args.lanes <= 32 else "icgn_kernel", "fast": "icgn_fast_kernel", "staged": "icgn_staged_kernel",
+        "kernel": {"exact": "icgn_kernel" if args.lanes > 32 else "icgn_band_kernel" if args.subset == 31
+                   else "icgn_band_kernel or icgn_kernel (by subset size)", "fast": "icgn_fast_kernel", "staged": "icgn_staged_kernel",
                    "staged-wide": "icgn_staged_kernel"}[args.solver_mode]
         + f"<affine,bspline,{args.lanes} lanes> (all pyramid levels)",
         "achieved": achieved,

@@ -489,6 +489,8 @@ int gbdic_batch_load_device(gbdic_batch *batch, int32_t job, const uint8_t *devi
  * `profile` set the stages are launched directly rather than as the graph,
  * and timing->device_ms is the solver launches' time alone. */
 int gbdic_batch_run_device(gbdic_batch *batch, void *stream, int32_t profile, gbdic_timing *timing);
+/* Solver launches of a step: one over every job or per class, or one per job. */
+int gbdic_batch_solver_launches(gbdic_batch *batch, int32_t *launches);
 /* Copy job j's GBDIC_EXPORT_* array to host memory (OUTPUT_STATE, RAW_STATE,
  * METADATA, ADMISSIBLE). */
 int gbdic_batch_export(gbdic_batch *batch, int32_t job, int32_t what, void *host_out, int64_t bytes);

@@ -40,6 +40,8 @@ constexpr int kBranches = 8;
 // subsets 2,968 -> 2,352; 32 jobs of affine S 33 (direct loop) 3,545 -> 2,848; eight
 // uneven jobs 3,090 -> 2,820.  Affine S 15 (direct loop, 11,844 subsets): 8 jobs
 // 2,358 -> 2,395, 32 jobs 8,825 -> 8,844.  64 lanes, 8 jobs of S 21: 2,420 -> 2,637.
+// Translation and quadratic jobs of S 15 have banded plans (quadratic 8 jobs of
+// 640 x 480 6,164 -> 4,480, translation 1,735 -> 1,068, the loop's gain with it).
 constexpr double kBranchShare = 0.25;
 
 bool is_quadratic(const BatchJobHost &j) { return j.desc.motion_model == GBDIC_MODEL_QUADRATIC; }
@@ -57,9 +59,9 @@ struct gbdic_batch {
     int lanes = 16, mode = GBDIC_BATCH_SINGLE, ctas_per_sm = 0;
     ClassQueue light, heavy, all;  // per-class queues, and the single queue
     // GBDIC_BATCH_SINGLE with as many CTAs as are resident, where enough of the
-    // windows gain: the jobs run concurrently, each as its own launch (the one launch over jobs of every kind has the direct loop only; a
-    // banded loop in it lost more to its size than it gave).  Every job's upload,
-    // prefilter, solve, outlier pass and readback are a branch of the step, so
+    // windows gain: the jobs run concurrently, each as its own launch (the one
+    // launch over jobs of every kind has the direct loop only; a banded loop in it
+    // lost more to its size than it gave).  Every job's upload, prefilter, solve, outlier pass and readback are a branch of the step, so
     // the copies and short passes of one job run beside the solves of others.
     bool branched = false;
     std::vector<int> branch_order;
@@ -498,6 +500,15 @@ int gbdic_batch_load_device(gbdic_batch *b, int32_t j, const uint8_t *device_fra
                                      cudaMemcpyDeviceToDevice, s),
                    "frame copy");
         if (!stream) check_cuda(cudaStreamSynchronize(s), "frame copy");
+    });
+}
+
+int gbdic_batch_solver_launches(gbdic_batch *b, int32_t *launches) {
+    return guarded(b, [&] {
+        if (!launches) fail(GBDIC_EINVAL, "output is required");
+        b->rebuild();
+        if (b->branched || b->mode == GBDIC_BATCH_PER_JOB) *launches = (int32_t)b->jobs.size();
+        else *launches = (b->light.grid > 0) + (b->heavy.grid > 0) + (b->all.grid > 0);
     });
 }
 

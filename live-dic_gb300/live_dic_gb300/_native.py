@@ -212,6 +212,7 @@ _SIGNATURES = {
     "gbdic_batch_register": (C.c_int, [P, P, P, P, C.POINTER(Timing)]),
     "gbdic_batch_load_device": (C.c_int, [P, I32, P, I64, P]),
     "gbdic_batch_run_device": (C.c_int, [P, P, I32, C.POINTER(Timing)]),
+    "gbdic_batch_solver_launches": (C.c_int, [P, C.POINTER(I32)]),
     "gbdic_batch_export": (C.c_int, [P, I32, I32, P, I64]),
     "gbdic_affine_frontier": (C.c_int, [P, P, P, P, P]),
     "gbdic_spatial_choose": (C.c_int, [P, P, P, P, C.POINTER(ChooseCfg), P, P, P]),

@@ -8,9 +8,10 @@ weighting, zero seed, the job's outlier pass) and a step runs all jobs as one
 CUDA graph: every target's prefilter, one persistent IC-GN launch per
 shape-function class over a device work queue ("persistent"), or one
 persistent launch over every job with the shape function dispatched per job
-("single"), then the outlier passes.  Unless most of the pixels are in
-windows up to 16 x 16, "single" without a limit on CTAs runs the jobs as
-concurrent branches of the graph instead, upload to readback.
+("single"), then the outlier passes.  "single" runs two or more jobs as
+concurrent branches of the graph instead, upload to readback, where that is
+faster: without a limit on CTAs, with 16 or 32 lanes, and with a quarter or
+more of the pixels in windows over 16 x 16 or of the banded loop.
 A job's result is bit-identical to ICGNWGPU.register with the same lanes per
 subset.
 
@@ -149,8 +150,8 @@ class ICGNBatch:
 
     def set_variant(self, lanes: int, mode: str = "single", ctas_per_sm: int = 0) -> None:
         """Lanes per subset, step mode ('persistent': a persistent queue per
-        shape-function class, 'single': one persistent queue over every job,
-        'per-job': one launch per job) and persistent CTAs per SM (0: all
+        shape-function class, 'single': one persistent queue over every job
+        or concurrent branches, 'per-job': one launch per job) and persistent CTAs per SM (0: all
         resident)."""
         self._require_open()
         self._check_variant(lanes, mode, ctas_per_sm)
@@ -214,6 +215,14 @@ class ICGNBatch:
                                                      int(bool(profile)),
                                                      C.byref(timing) if timing is not None else None))
         return None if timing is None else timing.device_ms
+
+    @property
+    def solver_launches(self) -> int:
+        """Solver launches of a step of the current jobs and variant."""
+        self._require_open()
+        launches = C.c_int32()
+        self._check(self._lib.gbdic_batch_solver_launches(self._handle, C.byref(launches)))
+        return int(launches.value)
 
     def export_state(self, job: int, *, raw: bool = False) -> np.ndarray:
         self._require_open()

@@ -160,3 +160,22 @@ def test_batch_branches_equal_the_single_launch(pairs, lanes):
         for j, want in enumerate(expected):
             got = batch.export_state(j)
             np.testing.assert_array_equal(got[..., : want.shape[-1]], want)
+
+
+def test_solver_launches_of_a_step(pairs):
+    """What a step launches: the one queue, a queue per class, a launch per job,
+    and branches where the rule takes them."""
+    small = [dict(j, subset_size=15, subset_stride=7, motion_model="affine") for j in pairs[:3]]
+    with _batch(pairs, solver_workgroup_size=16) as batch:
+        batch.set_variant(16, "single", 2)
+        assert batch.solver_launches == 1
+        batch.set_variant(16, "persistent")
+        assert batch.solver_launches == 2
+        batch.set_variant(16, "per-job")
+        assert batch.solver_launches == len(pairs)
+        batch.set_variant(16, "single")
+        assert batch.solver_launches == len(pairs)
+        batch.set_variant(64, "single")
+        assert batch.solver_launches == 1
+    with _batch(small, solver_workgroup_size=16) as batch:
+        assert batch.solver_launches == 1
