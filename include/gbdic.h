@@ -368,7 +368,9 @@ int gbdic_pyramid_register(gbdic_pyramid *pyramid, const uint8_t *frame, int64_t
 /* Resident variant: device frame in, device state out, no host sync. */
 int gbdic_pyramid_register_device(gbdic_pyramid *pyramid, const uint8_t *device_frame,
                                   float *device_state, void *stream);
-/* ICGNWGPUFullPyramid.reset_temporal_state (full_pyramid_backend.py:676-694). */
+/* ICGNWGPUFullPyramid.reset_temporal_state (full_pyramid_backend.py:676-694).
+ * Takes effect at once: wait for frames that gbdic_pyramid_register_device has
+ * in flight on a stream of the caller's first. */
 int gbdic_pyramid_reset_temporal(gbdic_pyramid *pyramid);
 /* Copies one level's internal buffer (GBDIC_EXPORT_*). */
 int gbdic_pyramid_export(gbdic_pyramid *pyramid, int32_t level, int32_t what, void *host_out,

@@ -147,31 +147,33 @@ int pguarded(gbdic_pyramid *p, F &&f) {
     }
 }
 
+// The histories are cleared at once, by the default stream: frames that a caller
+// still has in flight on a stream of its own are not waited for.  The copies have
+// landed on return.
 void reset_temporal(gbdic_pyramid *p, cudaStream_t s) {
     if (!p->temporal()) return;
     const int count = p->levels[0]->count;
     const int model = p->po.base.motion_model, ss = gbdic::state_stride(model);
     std::vector<float> state((size_t)count * ss, 0.0f);
     for (int i = 0; i < count; ++i) state[(size_t)i * ss + gbdic::parameter_count(model)] = -1.0f;
-    check_cuda(cudaMemcpyAsync(p->history.get(), state.data(), state.size() * sizeof(float), cudaMemcpyHostToDevice, s),
-               "history");
-    check_cuda(cudaMemsetAsync(p->ages.get(), 0xff, (size_t)count * sizeof(uint32_t), s), "ages");
+    check_cuda(cudaMemcpy(p->history.get(), state.data(), state.size() * sizeof(float), cudaMemcpyHostToDevice), "history");
+    check_cuda(cudaMemset(p->ages.get(), 0xff, (size_t)count * sizeof(uint32_t)), "ages");
     if (p->velocity()) {
-        check_cuda(cudaMemcpyAsync(p->prev_history.get(), state.data(), state.size() * sizeof(float),
-                                   cudaMemcpyHostToDevice, s), "history");
-        check_cuda(cudaMemsetAsync(p->prev_ages.get(), 0xff, (size_t)count * sizeof(uint32_t), s), "ages");
+        check_cuda(cudaMemcpy(p->prev_history.get(), state.data(), state.size() * sizeof(float), cudaMemcpyHostToDevice),
+                   "history");
+        check_cuda(cudaMemset(p->prev_ages.get(), 0xff, (size_t)count * sizeof(uint32_t)), "ages");
     }
-    std::vector<float> coarse;
     if (p->fine_correction()) {
         const int cc = p->levels.back()->count;
-        coarse.assign((size_t)cc * ss, 0.0f);
+        std::vector<float> coarse((size_t)cc * ss, 0.0f);
         for (int i = 0; i < cc; ++i) coarse[(size_t)i * ss + gbdic::parameter_count(model)] = -1.0f;
-        check_cuda(cudaMemcpyAsync(p->coarse_history.get(), coarse.data(), coarse.size() * sizeof(float),
-                                   cudaMemcpyHostToDevice, s), "history");
-        check_cuda(cudaMemsetAsync(p->coarse_ages.get(), 0xff, (size_t)cc * sizeof(uint32_t), s), "ages");
+        check_cuda(cudaMemcpy(p->coarse_history.get(), coarse.data(), coarse.size() * sizeof(float),
+                              cudaMemcpyHostToDevice), "history");
+        check_cuda(cudaMemset(p->coarse_ages.get(), 0xff, (size_t)cc * sizeof(uint32_t)), "ages");
     }
-    check_cuda(cudaStreamSynchronize(s), "history reset");
+    check_cuda(cudaStreamSynchronize(nullptr), "history reset");
     p->active_levels = p->L();
+    (void)s;
 }
 
 // Everything a frame does after its finest target is resident at `frame0`.

@@ -728,7 +728,9 @@ class ICGNWGPUFullPyramid:
 
     def reset_temporal_state(self) -> None:
         """Forget the temporal history (676-694); no-op before set_reference.
-        The adaptive policy starts again from the whole pyramid."""
+        The adaptive policy starts again from the whole pyramid.  Takes effect
+        at once: wait for register_device() frames in flight on a stream of
+        your own first."""
         self._adaptive_next_levels = self.pyramid_levels
         if self._handle is not None:
             self._check(self._lib.gbdic_pyramid_reset_temporal(self._handle))
