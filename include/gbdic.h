@@ -444,9 +444,7 @@ int gbdic_pyramid_set_partial_support(gbdic_pyramid *pyramid, int32_t level, int
  * GPU-prepared reference (B-spline interpolation, uniform weighting) and is
  * solved from a zero seed exactly like gbdic_register, followed by its own
  * outlier pass.  A step is one CUDA graph: prefilter of every target, the
- * IC-GN launches of the step mode over a device work queue (by default one
- * persistent launch over every job, heavy subsets first), then the outlier
- * passes. */
+ * IC-GN launches of the step mode, then the outlier passes. */
 typedef struct gbdic_batch gbdic_batch;
 
 typedef struct {
@@ -459,10 +457,11 @@ typedef struct {
 
 /* Step modes: PERSISTENT, one persistent launch per shape-function class
  * (affine + translation, quadratic) on two graph branches; PER_JOB, one
- * grid launch per job; SINGLE, one persistent launch over every job, or, with
- * ctas_per_sm 0 and 16 or 32 lanes where windows over 16 x 16, or of the banded
- * loop, hold a quarter or more of the pixels, every job as a branch of its own (upload to readback), the
- * solves concurrent launches.  A job's result is the same in every mode. */
+ * grid launch per job; SINGLE, one persistent launch over every job (heavy
+ * subsets first), or, for two or more jobs with ctas_per_sm 0 and 16 or 32 lanes
+ * where windows over 16 x 16, or of the banded loop, hold a quarter or more of the
+ * pixels, every job as a branch of its own (upload to readback), the solves
+ * concurrent launches.  A job's result is the same in every mode. */
 enum { GBDIC_BATCH_PERSISTENT = 0, GBDIC_BATCH_PER_JOB = 1, GBDIC_BATCH_SINGLE = 2 };
 
 int gbdic_batch_create(int32_t device, gbdic_batch **out);

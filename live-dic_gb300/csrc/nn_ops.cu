@@ -386,9 +386,6 @@ __global__ void __launch_bounds__(256) im2col_t_kernel(NnConvShape s, const __nv
     }
 }
 
-// out[n][k] = sum_s partial[s][k][n] (s ascending) for k < Kp, n < N.
-// Consecutive threads take consecutive n (contiguous partial reads); the
-// loads of four splits are issued before their ordered additions.
 // p[0] + p[stride] + ... in that order, 32 loads in flight.
 __device__ __forceinline__ float ordered_sum(const float *p, int count, size_t stride) {
     float acc = 0.0f;
@@ -405,6 +402,8 @@ __device__ __forceinline__ float ordered_sum(const float *p, int count, size_t s
     return acc;
 }
 
+// out[n][k] = sum_s partial[s][k][n] (s ascending) for k < Kp, n < N.
+// Consecutive threads take consecutive n (contiguous partial reads).
 __global__ void splitk_reduce_kernel(const float *partial, int splits, int Kp_rows, int N, int Kp, float *out) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= N * Kp) return;

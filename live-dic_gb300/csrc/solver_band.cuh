@@ -25,7 +25,7 @@
 // SMs with two subsets a warp start out that way, one subset to a warp.  What
 // a subset needs only between the pixel loops (its row of the metadata, the
 // inverse Hessian, stop counters) lives in shared memory, which keeps the
-// loops free of spills.
+// loops free of spills (quadratic with 16 lanes: 8 bytes).
 //
 // What bounds it.  The direct loop (solver_impl.cuh) gathers 16 taps and a
 // 16-byte plane entry for every pixel: 32 L1 wavefronts per warp and pixel,
@@ -41,7 +41,8 @@
 // UHD S 41 / s 10 quadratic 3,877 -> 3,229; 1280 x 720 S 21 / s 7 affine
 // 250 -> 219; 512 x 512 S 21 / s 10 80 -> 57; 2560 x 1440 S 31 / s 8
 // translation 666 -> 471; 400 x 300 S 41 / s 20 (234 subsets) quadratic
-// 149 -> 105.
+// 149 -> 105.  (Grids of few affine or translation windows take a block each,
+// solver_partial.cu.)
 //
 // Tried and not kept: smaller bands (more L1 left, but every band restarts the
 // rings: 1,826 us with 16-row bands); six CTAs per SM (80 registers, spills);

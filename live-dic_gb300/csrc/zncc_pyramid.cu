@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(128) final_zncc_kernel(ZnccArgs a) {
 // corner pixels; pixels between corners that lie inside by a margin lie
 // inside too (an affine map, rounded far below the margin), and a window
 // closer to the bound is checked pixel by pixel.
-// FMA-bound as the solver's sampling.  UHD S 31 / s 8 (127,359 subsets): 1,011
+// FMA-bound as the solver's sampling (96 registers, 44 bytes of spills).  UHD S 31 / s 8 (127,359 subsets): 1,011
 // us with sixteen clamped taps gathered and two integer divisions per pixel
 // (final_zncc_kernel), 517 us here.
 __global__ void __launch_bounds__(128, kBandBlocks) final_zncc_band_kernel(SolveArgs a, const float *f_plane, int f_pitch,

@@ -86,7 +86,7 @@ class _Conv:
     H: int            # input side
     OH: int           # output side
     kp: int           # forward reduction length (padded 9 cin)
-    kp_rows: int      # kp padded to 128 (rows of the weight-gradient GEMM)
+    kp_rows: int      # kp padded to 128 (the weight gradient's tiles of K)
     kt: int           # data-gradient reduction length (9 cout)
     M: int            # output rows (B OH^2)
     Min: int          # input rows (B H^2)
