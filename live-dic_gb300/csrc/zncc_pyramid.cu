@@ -512,6 +512,7 @@ static_assert(state_stride(kModelAffine) == 8 && status_slot(kModelAffine) == 6 
 }  // namespace
 
 cudaError_t launch_final_zncc(const ZnccArgs &a, cudaStream_t stream) {
+    if (a.count <= 0) return cudaSuccess;
     if (a.band.rows > 0) {
         SolveArgs b{};
         b.coef = a.coef;
@@ -522,7 +523,6 @@ cudaError_t launch_final_zncc(const ZnccArgs &a, cudaStream_t stream) {
             b, a.plane_f ? a.plane_f : reinterpret_cast<const float *>(a.plane), a.plane_f ? 1 : 4, a.out);
         return cudaGetLastError();
     }
-    if (a.count <= 0) return cudaSuccess;
     const int grid = (a.count + 1) / 2;
     switch (a.interp) {
     case kInterpLinear: final_zncc_kernel<kInterpLinear><<<grid, 128, 0, stream>>>(a); break;
